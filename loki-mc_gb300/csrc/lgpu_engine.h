@@ -1660,13 +1660,16 @@ class Engine {
     if (rate && n != P_) return fail(LGPU_ERR_BAD_ARG, "expected %d processes", P_);
     if (nc < 2 || !(max_e > 0))
       return fail(LGPU_ERR_BAD_ARG, "an EEDF needs at least 2 cells and a positive maximum energy");
-    const size_t nn = (size_t)nc + 1;
-    const size_t need = (size_t)n_eedf * ((size_t)nc + 5 * nn + (size_t)P_) + 16;
+    // [ticket | EEDFs | node shares and block sums (with the parameters) | rates | parameters]
+    const size_t nn = (size_t)nc + 1, n_f = (size_t)n_eedf * nc;
+    const size_t n_shares = rates_only ? 0 : 3 * (size_t)P_ * nn, n_sums = rates_only ? 0 : eedf_post_sums(nc);
+    const size_t need = 1 + n_f + n_shares + n_sums + (size_t)n_eedf * P_ + 16;
     if (need > post_cap_) {
       if (d_post_) cudaFree(d_post_);
       d_post_ = nullptr;
       post_cap_ = 0;
       LGPU_TRY(dalloc(&d_post_, need));
+      LGPU_CU(cudaMemsetAsync(d_post_, 0, sizeof(double), stream_));
       post_cap_ = need;
     }
     EedfPostArgs a{};
@@ -1678,13 +1681,17 @@ class Engine {
     a.gas_density = Ngas_;
     a.omega = omega_;
     a.omega_c = omega_c_;
-    a.eeh = eeh ? eeh : d_post_;  // unread when the EEDFs are given
+    a.ticket = reinterpret_cast<unsigned int*>(d_post_);
+    double* d_eedf = d_post_ + 1;
     if (eedf) {
-      LGPU_CU(cudaMemcpyAsync(d_post_, eedf, (size_t)n_eedf * nc * sizeof(double), cudaMemcpyHostToDevice, stream_));
-      a.eedf_in = d_post_;
+      LGPU_CU(cudaMemcpyAsync(d_eedf, eedf, n_f * sizeof(double), cudaMemcpyHostToDevice, stream_));
+      a.eedf_in = d_eedf;
     }
-    a.scratch = d_post_ + (size_t)n_eedf * nc;
-    a.rates = a.scratch + (size_t)n_eedf * 5 * nn;
+    a.eeh = eeh;
+    a.eedf_norm = d_eedf;
+    a.shares = d_eedf + n_f;
+    a.sums = a.shares + n_shares;
+    a.rates = a.sums + n_sums;
     a.params = a.rates + (size_t)n_eedf * P_;
     a.kind = d_tt_i_;
     a.ion = d_tt_i_ + P_;
@@ -1700,8 +1707,7 @@ class Engine {
     a.raw_iv = d_tt_raw_ + tt_int_total_;
     a.raw_me = d_tt_raw_ + 2 * tt_int_total_;
     a.raw_mv = d_tt_raw_ + 2 * tt_int_total_ + tt_mom_total_;
-    launch_eedf_post(a, stream_);
-    ++launches_;
+    launches_ += launch_eedf_post(a, sm_count_, stream_);
     LGPU_CU(cudaGetLastError());
     std::vector<double> res((size_t)n_eedf * P_ + 16);
     LGPU_CU(cudaMemcpyAsync(res.data(), a.rates, res.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_));

@@ -277,8 +277,8 @@ int launch_batch_post(const BatchArgs& b, int sm_count, int max_slots, unsigned 
 
 // End-of-job EEDF post-processing in FP64 (lgpu_post.cu): the EEDF-convolved
 // rate coefficient of every MC process (Collision.C:355-397) for each of
-// n_eedf EEDFs (one block each), and the two-term swarm parameters
-// (BoltzmannMC.C:2186-2266) of the first unless rates_only.
+// n_eedf EEDFs, and, unless rates_only, the two-term swarm parameters
+// (BoltzmannMC.C:2186-2266) of the one EEDF given.
 struct EedfPostArgs {
   int nc, P, n_eedf, rates_only;
   double max_energy, gas_density, omega, omega_c;
@@ -298,11 +298,16 @@ struct EedfPostArgs {
   const double* raw_iv;
   const double* raw_me;
   const double* raw_mv;
-  double* scratch;         // [n_eedf][5 x (nc + 1)]
+  double* eedf_norm;       // [n_eedf][nc]: the normalised EEDFs when eeh is given
+  double* shares;          // [3][P][nc + 1]: each process's share of the node totals (unless rates_only)
+  double* sums;            // [eedf_post_sums(nc)]: block sums of the parameters (unless rates_only)
+  unsigned int* ticket;    // zero before the first call, left zero by each
   double* rates;           // [n_eedf][P]
   double* params;          // [16], lgpu_eedf_params order
 };
-void launch_eedf_post(const EedfPostArgs& a, cudaStream_t s);
+size_t eedf_post_sums(int nc);
+// returns the kernels it launched
+int launch_eedf_post(const EedfPostArgs& a, int sm_count, cudaStream_t s);
 
 // Replay kernels for the parity tests: the production device functions
 // driven by given inputs and recorded uniforms.

@@ -6,8 +6,8 @@
 // Built with -fmad=false: every elementwise step rounds as the reference's
 // (whose build contracts nothing), so the per-node totals of the
 // momentum-transfer and energy-relaxation cross sections come out bit for
-// bit; the sums over cells run as a fixed-order block reduction, so they
-// agree with the reference's to rounding.
+// bit; the sums over cells run as fixed-order reductions, so they agree with
+// the reference's to rounding.
 #include "lgpu_kernels.cuh"
 
 namespace lgpu {
@@ -56,187 +56,310 @@ __device__ double raw_at(const double* e, const double* v, int n, double x) {
   return v[lo] + (x - e[lo]) / (e[lo + 1] - e[lo]) * (v[lo + 1] - v[lo]);
 }
 
-// sum over cells l = lmin .. nc-1 of (sig_l + sig_l+1) / 2 * cell_l * eedf_(l - shift)
-__device__ double conv_sum(const PostGrid& g, const double* sig, const double* eedf, int lmin, int shift,
-                           double* red) {
-  double s = 0.0;
-  for (int l = lmin + (int)threadIdx.x; l < g.nc; l += blockDim.x)
-    s += (sig[l] + sig[l + 1]) / 2.0 * g.cell(l) * eedf[l - shift];
-  return block_sum(s, red);
-}
+constexpr int kPostTile = 1024;       // cells whose cross sections a block holds at a time
+constexpr int kPostStage = 512;       // raw points of a table staged in shared memory (longer ones stay global)
+constexpr int kPostRows = 256;        // EEDFs of one block at most
+constexpr int kPostCells = 32;        // cells per block of the parameter sums
+constexpr int kPostSums = 13;
 
-// One block per EEDF (row blockIdx.x of eedf_in or eeh); the two-term swarm
-// parameters from row 0 unless rates_only.
-__global__ void __launch_bounds__(kPostThreads) k_eedf_post(EedfPostArgs a) {
-  __shared__ double red[kPostThreads / 32];
-  const int nc = a.nc, nn = nc + 1;
-  const int row = blockIdx.x;
-  if (a.eedf_in) a.eedf_in += (size_t)row * nc;
-  a.eeh += (size_t)row * nc;
-  a.scratch += (size_t)row * 5 * nn;
-  a.rates += (size_t)row * a.P;
+__device__ __forceinline__ PostGrid post_grid(const EedfPostArgs& a) {
   PostGrid g;
-  g.nc = nc;
+  g.nc = a.nc;
   g.max = a.max_energy;
-  g.step = a.max_energy / nc;
+  g.step = a.max_energy / a.nc;
   g.lo = g.step / 2.0;
   g.hi = a.max_energy - g.step / 2.0;
-  g.cstep = nc > 1 ? (g.hi - g.lo) / (nc - 1) : 0.0;
-  double* eedf = a.scratch;
-  double* mt = eedf + nn;
-  double* er = mt + nn;
-  double* erc = er + nn;
-  double* sig = erc + nn;  // the last forward collision's integral cross section on the nodes
-  // the EEDF: given, or normalised from the context's histogram sums
-  // (BoltzmannMC.C:1580: f = h / (sqrt(cell) sum(h) step))
-  if (a.eedf_in) {
-    for (int l = threadIdx.x; l < nc; l += blockDim.x) eedf[l] = a.eedf_in[l];
-  } else {
-    double s = 0.0;
-    for (int l = threadIdx.x; l < nc; l += blockDim.x) s += a.eeh[l];
-    const double norm = block_sum(s, red);
-    for (int l = threadIdx.x; l < nc; l += blockDim.x) eedf[l] = a.eeh[l] / (sqrt(g.cell(l)) * norm * g.step);
+  g.cstep = a.nc > 1 ? (g.hi - g.lo) / (a.nc - 1) : 0.0;
+  return g;
+}
+
+// The EEDFs normalised from histogram sums (BoltzmannMC.C:1580: f = h /
+// (sqrt(cell) sum(h) step)), one block per EEDF.
+__global__ void __launch_bounds__(kPostThreads) k_post_normalise(EedfPostArgs a, double* out) {
+  __shared__ double red[kPostThreads / 32];
+  const PostGrid g = post_grid(a);
+  const double* h = a.eeh + (size_t)blockIdx.x * a.nc;
+  double* f = out + (size_t)blockIdx.x * a.nc;
+  double s = 0.0;
+  for (int l = threadIdx.x; l < a.nc; l += blockDim.x) s += h[l];
+  const double norm = block_sum(s, red);
+  for (int l = threadIdx.x; l < a.nc; l += blockDim.x) f[l] = h[l] / (sqrt(g.cell(l)) * norm * g.step);
+}
+
+// a table in shared memory when it fits (the bisection's first touches are
+// then one round trip instead of one per step)
+__device__ __forceinline__ void stage_table(const double*& e, const double*& v, int n, double* se, double* sv) {
+  if (n > kPostStage) return;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    se[k] = e[k];
+    sv[k] = v[k];
   }
-  for (int i = threadIdx.x; i < nn; i += blockDim.x) mt[i] = er[i] = erc[i] = 0.0;
-  __syncthreads();
-  const double factor2 = sqrt(2.0 * kQeP / kMeP);
-  const double factor = factor2 / 3.0;
-  double k_ion = 0.0, k_att = 0.0;
-  for (int p = 0; p < a.P; ++p) {
-    const double thr = a.thr[p], dens = a.dens[p];
-    const double* ie = a.raw_ie + a.int_off[p];
-    const double* iv = a.raw_iv + a.int_off[p];
-    const double* me = a.raw_me + a.mom_off[p];
-    const double* mv = a.raw_mv + a.mom_off[p];
-    const int ni = a.int_len[p], nm = a.mom_len[p];
-    const int lmin = (int)floor(thr / g.step);
-    if (a.kind[p] == 2) {
-      // superelastic copy: Klein-Rosseland at the nodes (Collision.C:290-353),
-      // zero at the zero-energy node (BoltzmannMC.C:2205-2217)
-      for (int i = 1 + (int)threadIdx.x; i < nn; i += blockDim.x) {
-        const double u = g.node(i), x = u + thr, kr = 1.0 + thr / u;
-        const double s_int = kr * (raw_at(ie, iv, ni, x) * a.stat[p]);
-        const double s_mom = kr * (raw_at(me, mv, nm, x) * a.stat[p]);
-        const double w = s_int * dens;
-        mt[i] = mt[i] + s_mom * dens;
-        er[i] = er[i] + w * thr / u;
-        erc[i] = erc[i] + w;
-      }
-      double r = 0.0;
-      const int part = nc - lmin;
-      if (part > 0) {
-        // the forward collision's cross section, shifted EEDF (Collision.C:390)
-        double s = 0.0;
-        for (int k = threadIdx.x; k < part; k += blockDim.x) {
-          const int l = lmin + k;
-          s += (sig[l] + sig[l + 1]) / 2.0 * g.cell(l) * eedf[k];
-        }
-        r = factor2 * a.stat[p] * block_sum(s, red) * g.step;
-      }
-      if (threadIdx.x == 0) a.rates[p] = r;
-      __syncthreads();
-      continue;
-    }
-    // forward collision: cross sections on the nodes (Collision.C:221-228:
-    // every node for elastic collisions, from the first node above the
-    // threshold otherwise)
-    const bool elastic = a.kind[p] == 0;
-    for (int i = threadIdx.x; i < nn; i += blockDim.x) {
+  e = se;
+  v = sv;
+}
+
+// EEDF-convolved rate coefficients: one block per group of EEDFs
+// (blockIdx.x) and process (blockIdx.y). The process's cross section on a tile of the
+// grid's nodes goes to shared memory once and every EEDF of the group is summed
+// against it by a team of warps. With the parameters (one EEDF) the block also
+// writes the process's share of the momentum-transfer and energy-relaxation
+// totals at every node, which k_post_params adds up in process order.
+//
+// Bound by FP64 issue (a few operations per SM and clock on this device), so
+// the work is spread over the SMs. Whole calls, before (one block for all
+// processes of an EEDF, one after the other) -> now: one EEDF of 1000 cells
+// with the parameters, 40 processes, 1201 -> 89 us; the rates of 100 EEDFs, 65
+// processes, 1763 -> 104 us.
+__global__ void __launch_bounds__(kPostThreads) k_post_rates(EedfPostArgs a, const double* eedf, int rows_per_block) {
+  constexpr int kWarps = kPostThreads / 32;
+  __shared__ double s_e[kPostStage], s_v[kPostStage];
+  __shared__ double s_me[kPostStage], s_mv[kPostStage];
+  __shared__ double s_sig[kPostTile + 1];
+  __shared__ double s_acc[kPostRows > kWarps ? kPostRows : kWarps];
+  const PostGrid g = post_grid(a);
+  const int nc = a.nc, nn = nc + 1, p = blockIdx.y;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int row0 = blockIdx.x * rows_per_block, rows = min(rows_per_block, a.n_eedf - row0);
+  if (rows <= 0) return;
+  const bool super = a.kind[p] == 2;
+  // a superelastic copy convolves the forward collision's cross section with
+  // the EEDF shifted by the threshold (Collision.C:390)
+  const int f = super ? p - 1 : p;
+  const double thr = a.thr[p], fthr = a.thr[f], dens = a.dens[p];
+  const bool elastic = a.kind[f] == 0;
+  const int lmin = (int)floor(thr / g.step), shift = super ? lmin : 0;
+  const int ni = a.int_len[f];
+  const double *ie = a.raw_ie + a.int_off[f], *iv = a.raw_iv + a.int_off[f];
+  const bool shares = !a.rates_only;  // one EEDF
+  // a copy's own tables (its shares) are the forward collision's, given again
+  const int nm = a.mom_len[p], no = a.int_len[p];
+  const double *me = a.raw_me + a.mom_off[p], *mv = a.raw_mv + a.mom_off[p];
+  const double *oe = a.raw_ie + a.int_off[p], *ov = a.raw_iv + a.int_off[p];
+  stage_table(ie, iv, ni, s_e, s_v);
+  if (shares) stage_table(me, mv, nm, s_me, s_mv);
+  for (int k = threadIdx.x; k < rows; k += blockDim.x) s_acc[k] = 0.0;
+  // warps of a team share an EEDF's cells; with fewer than kWarps EEDFs a team
+  // has several, whose partial sums are added up in a fixed order
+  int team = 1;
+  while (2 * team * rows <= kWarps) team *= 2;
+  const int t = wid % team, r_first = wid / team, r_step = kWarps / team;
+  double part = 0.0;  // this warp's sum when its team has one EEDF at most (team > 1)
+  for (int c0 = 0; c0 < nc; c0 += kPostTile) {
+    const int cells = min(kPostTile, nc - c0);
+    __syncthreads();  // the tables are staged, the previous tile is done with
+    for (int j = threadIdx.x; j <= cells; j += blockDim.x) {
+      const int i = c0 + j;
       const double x = g.node(i);
-      const bool on = elastic || x > thr;
-      const double s_int = on ? raw_at(ie, iv, ni, x) : 0.0;
-      const double s_mom = on ? raw_at(me, mv, nm, x) : 0.0;
-      sig[i] = s_int;
-      mt[i] = mt[i] + s_mom * dens;
-      if (elastic) {
-        er[i] = er[i] + 2.0 * a.mass_ratio[p] * s_int * dens;
+      // on the nodes: every one for elastic collisions, from the first above the
+      // threshold otherwise (Collision.C:221-228)
+      const double s_int = (elastic || x > fthr) ? raw_at(ie, iv, ni, x) : 0.0;
+      s_sig[j] = s_int;
+      if (!shares || (j == cells && i != nc)) continue;  // the next tile's first node writes its share
+      double w_mt = 0.0, w_er = 0.0, w_erc = 0.0;
+      if (super) {
+        // Klein-Rosseland at the nodes (Collision.C:290-353), zero at the
+        // zero-energy node (BoltzmannMC.C:2205-2217)
+        if (i > 0) {
+          const double y = x + thr, kr = 1.0 + thr / x;
+          const double w = kr * (raw_at(oe, ov, no, y) * a.stat[p]) * dens;
+          w_mt = kr * (raw_at(me, mv, nm, y) * a.stat[p]) * dens;
+          w_er = w * thr / x;
+          w_erc = w;
+        }
       } else {
-        const double w = s_int * dens;
-        if (i > 0) er[i] = er[i] + w * thr / x;
-        erc[i] = erc[i] + w;
+        w_mt = ((elastic || x > thr) ? raw_at(me, mv, nm, x) : 0.0) * dens;
+        if (elastic) {
+          w_er = 2.0 * a.mass_ratio[p] * s_int * dens;
+        } else {
+          const double w = s_int * dens;
+          w_er = i > 0 ? w * thr / x : 0.0;
+          w_erc = w;
+        }
+      }
+      double* o = a.shares + (size_t)p * nn + i;
+      o[0] = w_mt;
+      o[(size_t)a.P * nn] = w_er;
+      o[2 * (size_t)a.P * nn] = w_erc;
+    }
+    __syncthreads();
+    // the tile's cells from lmin on, as weights (sig_l + sig_l+1) / 2 * cell_l in place
+    double keep[(kPostTile + kPostThreads - 1) / kPostThreads];
+    int m = 0;
+    for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m)
+      keep[m] = c0 + j >= lmin ? (s_sig[j] + s_sig[j + 1]) / 2.0 * g.cell(c0 + j) : 0.0;
+    __syncthreads();
+    m = 0;
+    for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m) s_sig[j] = keep[m];
+    __syncthreads();
+    const int j0 = max(0, lmin - c0);
+    for (int r = r_first; r < rows; r += r_step) {
+      const double* fr = eedf + (size_t)(row0 + r) * nc + c0 - shift;
+      double s = 0.0;
+      for (int j = j0 + 32 * t + lane; j < cells; j += 32 * team) s += s_sig[j] * fr[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (team > 1) part += s;
+      else if (lane == 0) s_acc[r] += s;
+    }
+  }
+  __syncthreads();
+  if (team > 1) {  // at most one EEDF per team: r_first
+    if (lane == 0) s_acc[wid] = part;
+    __syncthreads();
+  }
+  const double k = sqrt(2.0 * kQeP / kMeP) * (super ? a.stat[p] : 1.0);
+  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+    double s = 0.0;
+    for (int w = 0; w < team; ++w) s += s_acc[r * team + w];
+    a.rates[(size_t)(row0 + r) * a.P + p] = nc > lmin ? k * s * g.step : 0.0;
+  }
+}
+
+// The two-term swarm parameters (BoltzmannMC.C:2220-2266) from the processes'
+// shares: kPostCells cells per block, one node per lane and total per warp (the
+// sum over processes is in their order, as the reference's), then each block's
+// sums over its cells; the last block to finish adds those up in block order.
+__global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const double* eedf) {
+  __shared__ double s_tot[3][kPostCells + 1];
+  __shared__ double s_k[2];
+  __shared__ bool s_last;
+  const PostGrid g = post_grid(a);
+  const int nc = a.nc, nn = nc + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * kPostCells;
+  if (wid < 3) {
+    for (int j = lane; j <= kPostCells; j += 32) {
+      const int i = c0 + j;
+      if (i >= nn) break;
+      const double* q = a.shares + (size_t)wid * a.P * nn + i;
+      double s = 0.0;
+#pragma unroll 8
+      for (int p = 0; p < a.P; ++p) s = s + q[(size_t)p * nn];
+      s_tot[wid][j] = s;
+    }
+  } else if (lane < 2) {
+    // ionization and attachment rate coefficients of the forward collisions
+    double k = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < a.P; ++p)
+      if (a.kind[p] != 2 && a.ion[p] == lane + 1) k += a.dens[p] * a.rates[p];
+    s_k[lane] = k;
+  }
+  __syncthreads();
+  const double factor = sqrt(2.0 * kQeP / kMeP) / 3.0;
+  const double N = a.gas_density, w = a.omega, wc = a.omega_c;
+  const double k_ion = s_k[0], k_att = s_k[1], growth = k_ion - k_att;
+  auto mta = [&](int j) {  // momentum transfer plus the growth term (BoltzmannMC.C:2233-2234)
+    const int i = c0 + j;
+    return i == 0 ? s_tot[0][j] : s_tot[0][j] + 1.0 / (3.0 * factor * sqrt(g.node(i))) * growth;
+  };
+  // the warps share the sums: 0..6 and, of the mobility tensor, xx and xy on
+  // one warp, zz on another
+  double v[7] = {0, 0, 0, 0, 0, 0, 0};
+  const int l = c0 + lane;
+  if (l < nc) {
+    const double c = g.cell(l), f = eedf[l];
+    if (wid == 0) {
+      for (int q = 0; q < 3; ++q) v[q] = f * c * ((s_tot[q][lane + 1] + s_tot[q][lane]) * 0.5);
+      const double den = mta(lane) + mta(lane + 1);
+      v[3] = c * c * f / den;
+      v[4] = c * f / den;
+    }
+    if (wid > 0 && l >= 1) {
+      const double x = g.node(l), m = mta(lane), df = f - eedf[l - 1];
+      if (wid == 1) {
+        v[0] = x * x * df / m;
+        v[1] = x * df / m;
+      } else {
+        const double aux1 = -2.0 / 3.0 * kQeP / kMeP * pow(x, 1.5) * df;
+        const double fr = N * m * 3.0 * factor * sqrt(x);
+        const double f2 = fr * fr;
+        if (wid == 2) {
+          const double aux2 = (f2 + (w - wc) * (w - wc)) * (f2 + (w + wc) * (w + wc));
+          v[0] = fr * (f2 + w * w + wc * wc) / aux2 * aux1;
+          v[1] = w * (f2 + w * w - wc * wc) / aux2 * aux1;
+          v[2] = (f2 - w * w + wc * wc) / aux2 * aux1;
+          v[3] = fr / aux2 * aux1;
+        } else {
+          const double aux3 = f2 + w * w;
+          v[0] = fr / aux3 * aux1;
+          v[1] = w / aux3 * aux1;
+        }
       }
     }
-    __syncthreads();
-    double r = 0.0;
-    if (nc - lmin > 0) r = factor2 * conv_sum(g, sig, eedf, lmin, 0, red) * g.step;
-    if (threadIdx.x == 0) a.rates[p] = r;
-    if (a.ion[p] == 1) k_ion += dens * r;
-    if (a.ion[p] == 2) k_att += dens * r;
-    __syncthreads();
   }
-  if (a.rates_only) return;
-  // two-term swarm parameters (BoltzmannMC.C:2220-2266)
-  const double N = a.gas_density, w = a.omega, wc = a.omega_c;
-  const double growth = k_ion - k_att;
-  auto mta = [&](int i) {  // momentum transfer plus the growth term (BoltzmannMC.C:2233-2234)
-    return i == 0 ? mt[0] : mt[i] + 1.0 / (3.0 * factor * sqrt(g.node(i))) * growth;
-  };
-  double s_mt = 0, s_er = 0, s_erc = 0, s_de = 0, s_d = 0, s_me = 0, s_m = 0;
-  double s_xr = 0, s_xi = 0, s_yr = 0, s_yi = 0, s_zr = 0, s_zi = 0;
-  for (int l = threadIdx.x; l < nc; l += blockDim.x) {
-    const double c = g.cell(l), f = eedf[l];
-    s_mt += f * c * ((mt[l + 1] + mt[l]) * 0.5);
-    s_er += f * c * ((er[l + 1] + er[l]) * 0.5);
-    s_erc += f * c * ((erc[l + 1] + erc[l]) * 0.5);
-    const double den = mta(l) + mta(l + 1);
-    s_de += c * c * f / den;
-    s_d += c * f / den;
-    if (l >= 1) {
-      const double x = g.node(l), m = mta(l), df = f - eedf[l - 1];
-      s_me += x * x * df / m;
-      s_m += x * df / m;
-      const double aux1 = -2.0 / 3.0 * kQeP / kMeP * pow(x, 1.5) * df;
-      const double fr = N * m * 3.0 * factor * sqrt(x);
-      const double f2 = fr * fr;
-      const double aux2 = (f2 + (w - wc) * (w - wc)) * (f2 + (w + wc) * (w + wc));
-      const double aux3 = f2 + w * w;
-      s_xr += fr * (f2 + w * w + wc * wc) / aux2 * aux1;
-      s_xi += w * (f2 + w * w - wc * wc) / aux2 * aux1;
-      s_yr += (f2 - w * w + wc * wc) / aux2 * aux1;
-      s_yi += fr / aux2 * aux1;
-      s_zr += fr / aux3 * aux1;
-      s_zi += w / aux3 * aux1;
-    }
+  // warp -> first sum and count: 0: 0-4, 1: 5-6, 2: 7-10, 3: 11-12
+  const int first = wid == 0 ? 0 : wid == 1 ? 5 : wid == 2 ? 7 : 11, count = wid == 0 ? 5 : wid == 2 ? 4 : 2;
+  for (int q = 0; q < count; ++q) {
+    double s = v[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) a.sums[(size_t)blockIdx.x * kPostSums + first + q] = s;
   }
-  const double pre = N * 3.0 * factor * g.step;
-  const double v_mt = pre * block_sum(s_mt, red);
-  const double v_er = pre * block_sum(s_er, red);
-  const double v_erc = pre * block_sum(s_erc, red);
-  const double v_de = 2.0 * factor * g.step * block_sum(s_de, red);
-  const double v_me = -factor * block_sum(s_me, red);
-  const double v_d = 2.0 * factor * g.step * block_sum(s_d, red);
-  const double v_m = -factor * block_sum(s_m, red);
-  const double v_xr = N * block_sum(s_xr, red);
-  const double v_xi = -N * block_sum(s_xi, red);
-  const double v_yr = -N * wc * block_sum(s_yr, red);
-  const double v_yi = N * 2.0 * w * wc * block_sum(s_yi, red);
-  const double v_zr = N * block_sum(s_zr, red);
-  const double v_zi = -N * block_sum(s_zi, red);
+  __threadfence();
+  __syncthreads();
   if (threadIdx.x == 0) {
+    s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    if (s_last) *a.ticket = 0u;  // for the next call
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  __shared__ double s_sum[kPostSums];
+  if (threadIdx.x < kPostSums) {
+    double s = 0.0;
+#pragma unroll 8
+    for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(&a.sums[(size_t)b * kPostSums + threadIdx.x]);
+    s_sum[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double* s = s_sum;
+    const double pre = N * 3.0 * factor * g.step;
+    const double v_d = 2.0 * factor * g.step * s[4], v_m = -factor * s[6];
     double* o = a.params;
     o[0] = k_ion;
     o[1] = k_att;
-    o[2] = v_mt;
-    o[3] = v_er;
-    o[4] = v_erc;
-    o[5] = v_de;
-    o[6] = v_me;
+    o[2] = pre * s[0];
+    o[3] = pre * s[1];
+    o[4] = pre * s[2];
+    o[5] = 2.0 * factor * g.step * s[3];
+    o[6] = -factor * s[5];
     o[7] = v_d;
     o[8] = v_m;
     o[9] = v_d / v_m;
-    o[10] = v_xr;
-    o[11] = v_xi;
-    o[12] = v_yr;
-    o[13] = v_yi;
-    o[14] = v_zr;
-    o[15] = v_zi;
+    o[10] = N * s[7];
+    o[11] = -N * s[8];
+    o[12] = -N * wc * s[9];
+    o[13] = N * 2.0 * w * wc * s[10];
+    o[14] = N * s[11];
+    o[15] = -N * s[12];
   }
 }
 
 }  // namespace
 
-void launch_eedf_post(const EedfPostArgs& a, cudaStream_t s) {
-  k_eedf_post<<<a.n_eedf, kPostThreads, 0, s>>>(a);
+size_t eedf_post_sums(int nc) { return (size_t)((nc + kPostCells - 1) / kPostCells) * kPostSums; }
+
+int launch_eedf_post(const EedfPostArgs& a, int sm_count, cudaStream_t s) {
+  int n = 1;
+  const double* eedf = a.eedf_in;
+  if (!eedf) {
+    k_post_normalise<<<a.n_eedf, kPostThreads, 0, s>>>(a, a.eedf_norm);
+    eedf = a.eedf_norm;
+    ++n;
+  }
+  // groups of EEDFs so that the blocks about fill the device once: a block
+  // interpolates its process's cross section itself, so more groups than that
+  // only repeat it
+  const int fill = max(1, sm_count / max(a.P, 1));
+  const int groups = max((a.n_eedf + kPostRows - 1) / kPostRows, min(a.n_eedf, fill));
+  const int rows = (a.n_eedf + groups - 1) / groups;
+  k_post_rates<<<dim3((a.n_eedf + rows - 1) / rows, a.P), kPostThreads, 0, s>>>(a, eedf, rows);
+  if (!a.rates_only) {
+    k_post_params<<<(a.nc + kPostCells - 1) / kPostCells, 128, 0, s>>>(a, eedf);
+    ++n;
+  }
+  return n;
 }
 
 }  // namespace lgpu
