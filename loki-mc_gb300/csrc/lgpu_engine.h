@@ -116,6 +116,12 @@ class Engine {
     return reinterpret_cast<T*>(base + off);
   }
 
+  // What the host sends before an interval of a context on its own.
+  struct PlainCtl {
+    IntervalCtl ctl;
+    DistCtl dist;
+  };
+
   // The secondary, spill and population-control buffers for `cap` records
   // in one allocation.
   struct SecondarySet {
@@ -164,7 +170,7 @@ class Engine {
     if (cfg_.device < 0 || cfg_.device >= ndev) return fail(LGPU_ERR_BAD_ARG, "device %d out of range", cfg_.device);
     if (cfg_.n_electrons < 1 || cfg_.n_electrons > 2.0e9) return fail(LGPU_ERR_BAD_ARG, "nElectrons out of range");
     if (cfg_.n_interp < 2 || cfg_.n_interp > (1 << 24)) return fail(LGPU_ERR_BAD_ARG, "nInterpPoints out of range");
-    if (cfg_.n_energy_cells < 1 || cfg_.n_energy_cells > 4096) return fail(LGPU_ERR_BAD_ARG, "nEnergyCells must be 1..4096");
+    if (cfg_.n_energy_cells < 1 || cfg_.n_energy_cells > kMaxEnergyCells) return fail(LGPU_ERR_BAD_ARG, "nEnergyCells must be 1..4096");
     if (cfg_.sync_oversampling < 1) return fail(LGPU_ERR_BAD_ARG, "synchronizationOverSampling must be >= 1");
     if (cfg_.advance_real_batch < 0 || cfg_.advance_real_batch > 32)
       return fail(LGPU_ERR_BAD_ARG, "advance_real_batch must be 0..32");
@@ -186,7 +192,7 @@ class Engine {
     // the fixed device buffers: ensemble, scalars, tables, tallies, constants
     Carve cv;
     const size_t o_state = cv.take<float4>(2 * (size_t)N_), o_att = cv.take<int>(N_);
-    const size_t o_sc = cv.take<DevScalars>(1), o_ctl = cv.take<IntervalCtl>(1);
+    const size_t o_sc = cv.take<DevScalars>(1), o_ctl = cv.take<PlainCtl>(1);
     const size_t o_nup = cv.take<float2>(M_), o_nut = cv.take<double>(M_), o_num = cv.take<double>(M_);
     const size_t o_nuc = cv.take<float>(kMaxCoarse);
     const size_t o_eedf = cv.take<double>(nEC);
@@ -200,7 +206,8 @@ class Engine {
     if (reinterpret_cast<uintptr_t>(d_state_) % 32 != 0) return fail(LGPU_ERR_CUDA, "ensemble not 32-byte aligned");
     d_att_ = at<int>(d_core_, o_att);
     d_sc_ = at<DevScalars>(d_core_, o_sc);
-    d_ctl_ = at<IntervalCtl>(d_core_, o_ctl);
+    d_plain_ = at<PlainCtl>(d_core_, o_ctl);
+    d_ctl_ = &d_plain_->ctl;
     d_nu_pair_ = at<float2>(d_core_, o_nup);
     d_nu_tot_ = at<double>(d_core_, o_nut);
     d_nu_max_ = at<double>(d_core_, o_num);
@@ -216,12 +223,13 @@ class Engine {
     use_secondaries(q);
     // pinned host: the scalar read-back, the control block, the running maximum
     Carve ch;
-    const size_t o_hsc = ch.take<DevScalars>(1), o_hctl = ch.take<IntervalCtl>(1), o_hnum = ch.take<double>(M_);
+    const size_t o_hsc = ch.take<DevScalars>(1), o_hctl = ch.take<PlainCtl>(1), o_hnum = ch.take<double>(M_);
     LGPU_CU(cudaMallocHost((void**)&h_pinned_, ch.bytes));
     h_sc_ = at<DevScalars>(h_pinned_, o_hsc);
-    h_ctl_ = at<IntervalCtl>(h_pinned_, o_hctl);
+    h_plain_ = at<PlainCtl>(h_pinned_, o_hctl);
+    h_ctl_ = &h_plain_->ctl;
     h_nu_max_ = at<double>(h_pinned_, o_hnum);
-    std::memset(h_ctl_, 0, sizeof(IntervalCtl));
+    std::memset(h_plain_, 0, sizeof(PlainCtl));
     std::memset(h_nu_max_, 0, (size_t)M_ * sizeof(double));
     LGPU_CU(cudaMemsetAsync(d_claim_, 0, claim_words_ * sizeof(unsigned int), stream_));
     LGPU_CU(cudaMemsetAsync(d_sc_, 0, sizeof(DevScalars), stream_));
@@ -240,6 +248,7 @@ class Engine {
     if (h_pinned_) cudaFreeHost(h_pinned_);
     h_pinned_ = nullptr;
     h_sc_ = nullptr;
+    h_plain_ = nullptr;
     h_ctl_ = nullptr;
     h_nu_max_ = nullptr;
     if (tables_ev_) cudaEventDestroy(tables_ev_);
@@ -725,7 +734,7 @@ class Engine {
   // population control (when the mixture ionizes or attaches), the ensemble
   // sample and the scalar read-back. Captured once as a CUDA graph.
   void enqueue_interval(bool sample) {
-    copy(d_ctl_, h_ctl_, sizeof(IntervalCtl), cudaMemcpyHostToDevice);
+    copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice);
     cudaMemsetAsync(d_sc_, 0, offsetof(DevScalars, null_count), stream_);
     AdvanceArgs a = advance_args();
     cudaEventRecordWithFlags(ev0_, stream_, cudaEventRecordExternal);
@@ -740,19 +749,21 @@ class Engine {
       launch_pop_control(pop_args(), stream_);
       launches_ += 1 + kPopLaunches;
     }
-    if (sample) enqueue_sample();
+    if (sample) enqueue_sample(true);
     copy(h_sc_, d_sc_, sizeof(DevScalars), cudaMemcpyDeviceToHost);
   }
 
-  void enqueue_sample() {
+  // dist: with the distributions the interval's control block asks for
+  void enqueue_sample(bool dist = false) {
     cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_);
     cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_);
-    SampleArgs s{};
-    s.state = d_state_;
-    s.n = N_;
-    s.half_me_over_e = (float)(0.5 * kMeD / kQeD);
-    s.moments = d_sc_->moments;
-    s.max_energy_bits = &d_sc_->sample_max_bits;
+    SampleArgs s = sample_args();
+    if (dist) {
+      s.dist = &d_plain_->dist;
+      s.advance_max_bits = &d_sc_->max_energy_bits;
+      s.dist_e_cells = cfg_.n_energy_cells;
+      s.dist_v_cells = cylindrical_ ? cfg_.n_radial_cells * cfg_.n_axial_cells : 0;
+    }
     launch_sample(s, sm_count_, stream_);
     ++launches_;
   }
@@ -769,7 +780,7 @@ class Engine {
       cudaGraphDestroy(g);
       graph_launches_[sample ? 1 : 0] = launches_ - l0;
       launches_ = l0;
-      h2d_bytes_ -= sizeof(IntervalCtl);
+      h2d_bytes_ -= sizeof(PlainCtl);
       d2h_bytes_ -= sizeof(DevScalars);
     }
     *out = ge;
@@ -814,7 +825,22 @@ class Engine {
     // in a batch the sample of this interval counts its EVDF in the moment
     // pass when it will record distributions (grid fixed since the steady state)
     evdf_fused_ = batch_ && sampling_ && ss_time_ != kNonDef && cylindrical_;
+    // alone, the sample counts all of them in one read while the energy grid holds
+    DistCtl& d = h_plain_->dist;
+    d.on = !batch_ && sampling_ && ss_time_ != kNonDef && N_ <= kDistInSample;
+    if (d.on) {
+      d.h = hist_args(time_ + pending_dt_);
+      d.e_bound = (float)max_eedf_;
+      if ((double)d.e_bound > max_eedf_) d.e_bound = std::nextafter(d.e_bound, 0.0f);
+    }
     return LGPU_OK;
+  }
+
+  // whether the last interval's sample counted its distributions (k_sample's test)
+  bool sample_counted() const {
+    float adv_max;
+    std::memcpy(&adv_max, &h_sc_->max_energy_bits, 4);
+    return h_plain_->dist.on && adv_max <= h_plain_->dist.e_bound;
   }
 
   // The second half, once the interval's device work is done and its scalars
@@ -889,7 +915,7 @@ class Engine {
     LGPU_TRY(graph_for(sample, &ge));
     LGPU_CU(cudaGraphLaunch(ge, stream_));
     launches_ += graph_launches_[sample ? 1 : 0];
-    h2d_bytes_ += sizeof(IntervalCtl);
+    h2d_bytes_ += sizeof(PlainCtl);
     d2h_bytes_ += sizeof(DevScalars);
     LGPU_TRY(sync("interval"));
     {
@@ -1039,9 +1065,8 @@ class Engine {
     return sync("rebin write");
   }
 
-  // getTimeDependDistributions (BoltzmannMC.C:1492-1572)
-  int sample_distributions() {
-    if (max_elec_energy_ > max_eedf_) LGPU_TRY(rebin_distributions());
+  // the tallies of a sample taken at `time` on the current grids
+  HistArgs hist_args(double time) const {
     HistArgs h{};
     h.state = d_state_;
     h.n = N_;
@@ -1052,7 +1077,7 @@ class Engine {
     h.eedf_periodic_row = nullptr;
     if (omega_ != 0) {
       const int nPh = cfg_.n_phases;
-      const double ph = std::fmod(omega_ * time_, 2.0 * kPi);
+      const double ph = std::fmod(omega_ * time, 2.0 * kPi);
       const int pi = (int)std::fmin(std::floor(ph / (2.0 * kPi / nPh)), nPh - 1);
       h.eedf_periodic_row = d_eedf_per_ + (size_t)pi * cfg_.n_energy_cells;
     }
@@ -1065,6 +1090,14 @@ class Engine {
     h.inv_ax_step = (float)(1.0 / ax_step_);
     h.max_speed = (float)max_speed_;
     h.evdf = d_evdf_;
+    return h;
+  }
+
+  // getTimeDependDistributions (BoltzmannMC.C:1492-1572)
+  int sample_distributions() {
+    if (sample_counted()) return LGPU_OK;
+    if (max_elec_energy_ > max_eedf_) LGPU_TRY(rebin_distributions());
+    HistArgs h = hist_args(time_);
     h.evdf_done = evdf_fused_ ? 1 : 0;
     evdf_fused_ = false;
     if (batch_) {
@@ -1532,6 +1565,7 @@ class Engine {
   // lgpu_advance: n intervals with a sample after each
   int advance(int n, lgpu_step_report* rep) {
     if (!initialized_) return fail(LGPU_ERR_STATE, "init_ensemble comes first");
+    sampling_ = false;  // no distributions: only lgpu_solve tallies them
     for (int i = 0; i < n; ++i) {
       LGPU_TRY(step_interval(true));
       ++n_samp_;
@@ -1901,7 +1935,8 @@ class Engine {
   int *d_removed_ = nullptr, *d_pair_slot_ = nullptr, *d_pair_sec_ = nullptr;
   DevScalars* d_sc_ = nullptr;
   DevScalars* h_sc_ = nullptr;
-  IntervalCtl* d_ctl_ = nullptr;
+  PlainCtl *d_plain_ = nullptr, *h_plain_ = nullptr;
+  IntervalCtl* d_ctl_ = nullptr;  // the control blocks' interval part
   IntervalCtl* h_ctl_ = nullptr;
   cudaGraphExec_t graph_[2] = {nullptr, nullptr};
   long long graph_launches_[2] = {0, 0};

@@ -216,7 +216,8 @@ __global__ void k_coarse_max(const float2* nu_pair, int M, int shift, float* coa
 }
 
 // ---------------------------------------------------------------- sample
-constexpr int kSampleThreads = 256;
+constexpr int kSampleThreads = 512;
+constexpr int kSampleSmem = 100 * 1024;  // EEDF and EVDF counts, two blocks per SM
 
 // Moment sums of electrons begin, begin+step, ... < end into a.moments: per
 // thread in FP32 (a handful of electrons each), FP64 from the warp reduction on.
@@ -280,11 +281,6 @@ __device__ __forceinline__ void sample_range(const SampleArgs& a, int begin, int
   }
 }
 
-__global__ void __launch_bounds__(kSampleThreads) k_sample(SampleArgs a) {
-  __shared__ double s_m[kSampleThreads / 32][kMoments];
-  sample_range(a, blockIdx.x * blockDim.x + threadIdx.x, a.n, gridDim.x * blockDim.x, s_m);
-}
-
 // ------------------------------------------------------------- histograms
 // The tallies of one sample in two passes over the electrons' velocities,
 // each in blocks of up to kHistChunk electrons that count in shared memory and
@@ -317,6 +313,60 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
     cy = (int)((cosang + 1.0f) * (0.5f * (float)a.n_cos));
     rx = (int)(radial_speed(v2xy) * a.inv_rad_step);
     ry = (int)((B.z + a.max_speed) * a.inv_ax_step);
+  }
+}
+
+// The sample of one condition: the moments and, when the interval's DistCtl says
+// so, the distributions in the same read: EEDF counts in shared memory (one FP64
+// atomic per occupied cell and block), EADF and (V_SHARED false) EVDF counts
+// straight to the FP64 tallies, whose cells are too many for the electrons of a
+// block to share. V_SHARED counts the EVDF in shared memory (16-bit, two per
+// word: a block sees fewer than 2^16 electrons).
+//
+// Bound by the FP64 additions at L2 (about 1.1e11/s measured, faster than 32-bit
+// ones to the same cells). Separate passes over the electrons in 65535-electron
+// chunks, which this replaces up to kDistInSample electrons, left most SMs idle:
+// moments + EEDF/EADF + EVDF of 1e6 electrons 16 + 49 + 91 -> 35 us, of 4e6
+// 28 + 54 + 93 -> 83 us, of 10,000 5 + 12 + 14.5 -> 7 us.
+template <bool V_SHARED>
+__global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sample(SampleArgs a) {
+  __shared__ double s_m[kSampleThreads / 32][kMoments];
+  extern __shared__ unsigned int sm_dist[];
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (!a.dist || !a.dist->on || !(__uint_as_float(*a.advance_max_bits) <= a.dist->e_bound)) {
+    sample_range(a, first, a.n, step, s_m);
+    return;
+  }
+  const HistArgs h = a.dist->h;
+  const int nE = h.n_e_cells, nV = h.cylindrical ? h.n_rad * h.n_ax : 0, nVw = V_SHARED ? (nV + 1) >> 1 : 0;
+  unsigned int* hE = sm_dist;
+  unsigned int* hV = sm_dist + nE;
+  for (int c = threadIdx.x; c < nE + nVw; c += blockDim.x) sm_dist[c] = 0u;
+  __syncthreads();
+  auto count = [&](float4 B) {
+    int c, cy, rx, ry;
+    hist_cells(h, B, c, cy, rx, ry);
+    if (c >= 0 && c < nE) {
+      atomicAdd(&hE[c], 1u);
+      if (cy >= 0 && cy < h.n_cos) atomicAdd(&h.eadf[c * h.n_cos + cy], 1.0);
+    }
+    if (rx >= 0 && rx < h.n_rad && ry >= 0 && ry < h.n_ax) {
+      const int idx = rx * h.n_ax + ry;
+      if (V_SHARED) atomicAdd(&hV[idx >> 1], 1u << ((idx & 1) << 4));
+      else atomicAdd(&h.evdf[idx], 1.0);
+    }
+  };
+  sample_range(a, first, a.n, step, s_m, count);  // ends behind a block barrier
+  for (int c = threadIdx.x; c < nE; c += blockDim.x) {
+    const unsigned int k = hE[c];
+    if (!k) continue;
+    atomicAdd(&h.eedf[c], (double)k);
+    if (h.eedf_periodic_row) atomicAdd(&h.eedf_periodic_row[c], (double)k);
+  }
+  for (int w = threadIdx.x; w < nVw; w += blockDim.x) {
+    const unsigned int k = hV[w];
+    if (k & 0xFFFFu) atomicAdd(&h.evdf[2 * w], (double)(k & 0xFFFFu));
+    if (k >> 16) atomicAdd(&h.evdf[2 * w + 1], (double)(k >> 16));
   }
 }
 
@@ -935,10 +985,25 @@ void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
   if (a.nu_coarse) k_coarse_max<<<1, kMaxCoarse, 0, s>>>(a.nu_pair, a.M, a.coarse_shift, a.nu_coarse, a.n_coarse);
 }
 
+// Blocks of the single-condition sample: half-size ones while the ensemble does
+// not fill the device with full ones (they clear and add up their EEDF counts
+// side by side; 10,000 electrons with distributions 9.1 -> 7.1 us), full ones
+// from there (fewer EEDF additions per electron: 200,000 electrons under AC
+// 21.9 -> 15.9 us). EVDF counts go to shared memory from 1e6 electrons on: 4e6
+// electrons 112 -> 83 us, 1e6 37 -> 35 us, 200,000 15.9 -> 21.8 us.
+constexpr int kSampleSharedV = 1000000;
+
 void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   if (a.n <= 0) return;
-  const int grid = min(blocks_for(a.n, kSampleThreads), max(1, sm_count) * 4);
-  k_sample<<<grid, kSampleThreads, 0, s>>>(a);
+  const int sms = max(1, sm_count), full = sms * (1024 / kSampleThreads);
+  const int threads = a.n < full * kSampleThreads / 2 ? kSampleThreads / 2 : kSampleThreads;
+  const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
+  const int eedf = a.dist ? a.dist_e_cells * (int)sizeof(unsigned int) : 0;
+  const long long v_words = ((long long)a.dist_v_cells + 1) / 2;
+  const bool v_shared = a.dist && a.n >= kSampleSharedV && eedf + 4 * v_words <= kSampleSmem &&
+                        blocks_for(a.n, grid * threads) * (long long)threads < 65536;
+  if (v_shared) k_sample<true><<<grid, threads, eedf + 4 * (int)v_words, s>>>(a);
+  else k_sample<false><<<grid, threads, eedf, s>>>(a);
 }
 
 void launch_hist(const HistArgs& a, cudaStream_t s) {
@@ -963,6 +1028,7 @@ cudaError_t prepare_kernels() {
     e = cudaFuncSetAttribute(k_hist_b_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistBSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sample_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleBatchSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sample<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
   if (e == cudaSuccess) e = prepare_advance_stash();
   return e;
 }

@@ -12,6 +12,7 @@ namespace lgpu {
 
 constexpr int kMaxProcesses = 512;
 constexpr int kMaxGases = 16;
+constexpr int kMaxEnergyCells = 4096;
 constexpr int kMoments = 22;  // sum e, r(3), v(3), r r^T (6 unique), r v^T (9)
 
 // Device scalars of one condition, read back after every interval.
@@ -123,17 +124,6 @@ struct TableBuildArgs {
 };
 void launch_build_tables(const TableBuildArgs& a, cudaStream_t s);
 
-// Ensemble sample: moment sums (FP64) and the largest energy.
-struct SampleArgs {
-  const float4* state;
-  int n;
-  float half_me_over_e;
-  double* moments;                 // [kMoments], accumulated (zeroed by the caller)
-  unsigned int* max_energy_bits;
-};
-// grid: at most four blocks per SM (sm_count = the device's multiprocessors)
-void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s);
-
 // Distribution tallies of one sample (BoltzmannMC.C:1550-1571).
 struct HistArgs {
   const float4* state;
@@ -152,6 +142,40 @@ struct HistArgs {
   int evdf_done;                   // the EVDF of this sample was counted with its moments (batches)
   int pad;
 };
+// What the sample of an interval counts beside its moments, written by the host
+// with the interval's control block: the distributions (BoltzmannMC.C:1550-1571)
+// when their energy grid holds every electron. Whether it does is known before
+// the sample: no electron at the end of the interval is above the largest energy
+// the advance saw (population control only drops and copies electrons), so the
+// sample counts when that energy is at most `e_bound`, the largest float on the
+// grid, and otherwise leaves the tallies to the host, which re-bins first.
+struct DistCtl {
+  int on;
+  float e_bound;
+  HistArgs h;
+};
+
+// Ensembles up to this size count their distributions with the sample: above it
+// the passes over 65535-electron chunks fill the device, and their shared-memory
+// counts cost less than two FP64 additions at L2 per electron (from the figures at
+// k_sample: 21 against 17 us per 1e6 electrons at 2e7).
+constexpr int kDistInSample = 16000000;
+
+// Ensemble sample: moment sums (FP64) and the largest energy, and, with `dist`,
+// the distributions in the same read of the ensemble.
+struct SampleArgs {
+  const float4* state;
+  int n;
+  float half_me_over_e;
+  double* moments;                 // [kMoments], accumulated (zeroed by the caller)
+  unsigned int* max_energy_bits;
+  const DistCtl* dist;             // null: moments only
+  const unsigned int* advance_max_bits;  // largest energy of the interval's advance (with dist)
+  int dist_e_cells, dist_v_cells;        // EEDF and EVDF cells (with dist)
+};
+// grid: at most four blocks per SM (sm_count = the device's multiprocessors)
+void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s);
+
 void launch_hist(const HistArgs& a, cudaStream_t s);
 
 // Population control (BoltzmannMC.C:1282-1408) at the end of an interval,
