@@ -476,62 +476,71 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
 constexpr bool kPrefetchChunk = true;  // a claimed chunk's states, at the claim
 constexpr bool kPrefetchRows = true;   // a parked collision's cumulative row (stash shapes)
 
+// A warp's place in the ensemble (warp-uniform): the electrons [next, end) it
+// holds, and where it takes more: chunks of `chunk` electrons from `base` on, by
+// the work counter. A context on its own starts each warp on a share of its own
+// (no counter, no wait) and leaves the rest, if any, to the counter.
+struct WarpCursor {
+  int next, end, base, chunk;
+  bool exhausted;
+};
+
+__device__ __forceinline__ void prefetch_states(const AdvanceArgs& a, int first, int end) {
+  prefetch_l2(a.state + 2 * first, (uint32_t)(end - first) * 2u * sizeof(float4));
+}
+
 // The index of the ensemble electron a lane claims (-1: none): the `n_want`
 // claiming lanes (this one `wants` it, rank r among them) take the next
 // electrons of the warp's chunk, and of a new chunk from the work counter
-// when it runs out; `next`, `end` and `exhausted` are the warp-uniform cursors.
-template <int CHUNK>
+// when it runs out.
 __device__ __forceinline__ int lane_claim(const AdvanceArgs& a, int n_want, int r, bool wants, int lane, int n_el,
-                                          int& next, int& end, bool& exhausted) {
+                                          WarpCursor& w) {
   int idx = -1;
-  const int take = min(n_want, end - next);
-  if (wants && r < take) idx = next + r;
-  next += take;
+  const int take = min(n_want, w.end - w.next);
+  if (wants && r < take) idx = w.next + r;
+  w.next += take;
   if (n_want > take) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(a.work_counter, CHUNK);
-    base = __shfl_sync(0xffffffffu, base, 0);
+    int base = n_el;
+    if (w.base < n_el) {
+      if (lane == 0) base = w.base + atomicAdd(a.work_counter, w.chunk);
+      base = __shfl_sync(0xffffffffu, base, 0);
+    }
     if (base >= n_el) {
-      exhausted = true;
+      w.exhausted = true;
     } else {
-      next = base;
-      end = min(base + CHUNK, n_el);
-      if (kPrefetchChunk && lane == 0) prefetch_l2(a.state + 2 * base, (uint32_t)(end - base) * 2u * sizeof(float4));
+      w.next = base;
+      w.end = min(base + w.chunk, n_el);
+      if (kPrefetchChunk && lane == 0) prefetch_states(a, base, w.end);
       const int r2 = r - take;
-      const int take2 = min(n_want - take, end - next);
-      if (wants && r2 >= 0 && r2 < take2) idx = next + r2;
-      next += take2;
+      const int take2 = min(n_want - take, w.end - w.next);
+      if (wants && r2 >= 0 && r2 < take2) idx = w.next + r2;
+      w.next += take2;
     }
   }
   return idx;
 }
 
 // Lanes without an electron (`need`) take the next ones of the warp's chunk.
-template <int CHUNK>
 __device__ __forceinline__ void lane_take_chunk(const AdvanceArgs& a, const IntervalView& iv, Lane& L,
-                                                unsigned need, int lane, unsigned lt_mask, int n_el, int& next,
-                                                int& end, bool& exhausted) {
-  const int idx = lane_claim<CHUNK>(a, __popc(need), __popc(need & lt_mask), !L.have, lane, n_el, next, end,
-                                    exhausted);
+                                                unsigned need, int lane, unsigned lt_mask, int n_el, WarpCursor& w) {
+  const int idx = lane_claim(a, __popc(need), __popc(need & lt_mask), !L.have, lane, n_el, w);
   if (idx >= 0) lane_take_electron(a, iv, L, idx);
 }
 
-// The warps' work on one condition: the ensemble in 128-electron warp chunks
-// from the condition's work counter, then each warp's queued secondaries (or,
-// drain, only the spilled secondaries). Returns when the condition's counter
+// The warps' work on one condition: the ensemble in warp chunks from `cur` on,
+// then each warp's queued secondaries (or, drain, only the spilled secondaries). Returns when the condition's counter
 // and the warp's queue are exhausted; the caller flushes the lane sums.
 template <int MODE, class Sh>
 __device__ __forceinline__ void warp_loop(const AdvanceArgs& a, Sh& sh, const IntervalView& iv,
-                                          LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag) {
+                                          LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag, WarpCursor cur) {
   const bool drain = a.queue_only != 0;
   const int n_el = drain ? 0 : a.n;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
   Lane L;
   reset_lane(L);
-  // warp-uniform cursors: ensemble chunk, spill buffer (drain only)
-  int next = 0, end = 0, sp_next = 0;
-  bool exhausted = drain;
+  int sp_next = 0;  // warp-uniform place in the spill buffer (drain only)
+  if (drain) cur.exhausted = true;
 
   for (;;) {
     __syncwarp();
@@ -542,8 +551,8 @@ __device__ __forceinline__ void warp_loop(const AdvanceArgs& a, Sh& sh, const In
     int qn = min(sh.qn[wid], a.local_q);
     if (qn > 0) qn = lane_take_queued(a, iv, sh, wid, lane, lt_mask, L, tl, sec_id, warp_tag);
     const unsigned need = __ballot_sync(0xffffffffu, !L.have);
-    if (need && !exhausted) lane_take_chunk<Sh::kChunk>(a, iv, L, need, lane, lt_mask, n_el, next, end, exhausted);
-    if (exhausted) {
+    if (need && !cur.exhausted) lane_take_chunk(a, iv, L, need, lane, lt_mask, n_el, cur);
+    if (cur.exhausted) {
       if (drain) {
         const unsigned idle2 = __ballot_sync(0xffffffffu, !L.have);
         const int cnt = min(*(volatile int*)a.spill_count, a.spill_cap);
@@ -560,7 +569,7 @@ __device__ __forceinline__ void warp_loop(const AdvanceArgs& a, Sh& sh, const In
     const unsigned live = __ballot_sync(0xffffffffu, L.have);
     if (!live) {
       const bool spill_left = drain && sp_next < min(*(volatile int*)a.spill_count, a.spill_cap);
-      if (exhausted && qn == 0 && !spill_left) break;
+      if (cur.exhausted && qn == 0 && !spill_left) break;
       continue;
     }
     warp_turn<MODE>(a, sh, wid, iv, L, tl, live);
@@ -646,7 +655,8 @@ __device__ __forceinline__ void stash_swap(float4* wst, int e, Lane& L) {
 // is ready, take the rest. So np + nr <= 63 throughout.
 template <int MODE, class Sh>
 __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, float4* wst, const IntervalView& iv,
-                                                LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag) {
+                                                LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag,
+                                                WarpCursor cur) {
   constexpr int NS = Sh::kStash;
   static_assert(NS >= 64, "the stash holds up to 63 records");
   const int n_el = a.n;
@@ -654,8 +664,7 @@ __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, fl
   const unsigned lt_mask = (1u << lane) - 1u;
   Lane L;
   reset_lane(L);
-  int next = 0, end = 0, np = 0, nr = 0;
-  bool exhausted = false;
+  int np = 0, nr = 0;
 
   for (;;) {
     __syncwarp();
@@ -674,7 +683,7 @@ __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, fl
       qn = lane_take_queued(a, iv, sh, wid, lane, lt_mask, L, tl, sec_id, warp_tag);
       need = __ballot_sync(0xffffffffu, !L.have);
     }
-    if (need && !exhausted) lane_take_chunk<Sh::kChunk>(a, iv, L, need, lane, lt_mask, n_el, next, end, exhausted);
+    if (need && !cur.exhausted) lane_take_chunk(a, iv, L, need, lane, lt_mask, n_el, cur);
     const unsigned live = __ballot_sync(0xffffffffu, L.have);
 
     // ---- collision turn on the top min(np, 32) pending records
@@ -693,7 +702,7 @@ __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, fl
     }
     if (!live) {
       // np == 0 and nr == 0 here: idle lanes take every ready record first
-      if (exhausted && qn == 0) break;
+      if (cur.exhausted && qn == 0) break;
       continue;
     }
 
@@ -726,19 +735,28 @@ __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, fl
   }
 }
 
-// One condition per launch (or, drain, its spilled secondaries).
+// One condition per launch (or, drain, its spilled secondaries): every warp
+// starts on its own a.share electrons.
 template <int MODE, class Sh>
 __device__ __forceinline__ void advance_body(const AdvanceArgs& a, Sh& sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int warps = (int)(blockDim.x >> 5);
+  // drain launches: one block, whose warp tag stays below the spill's 0xFFFFFFFF
+  const uint32_t warp_tag = (uint32_t)(blockIdx.x * warps + wid);
+  WarpCursor cur;
+  cur.next = min((int)warp_tag * a.share, a.n);
+  cur.end = min(cur.next + a.share, a.n);
+  cur.base = (int)gridDim.x * warps * a.share;
+  cur.chunk = a.chunk;
+  cur.exhausted = false;
+  if (kPrefetchChunk && lane == 0 && cur.end > cur.next) prefetch_states(a, cur.next, cur.end);
   load_block_consts(a, sh);
   __syncthreads();
   const IntervalView iv = interval_view<MODE>(a);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  // drain launches: one block, whose warp tag stays below the spill's 0xFFFFFFFF
-  const uint32_t warp_tag = (uint32_t)(blockIdx.x * Sh::kWarps + wid);
   LaneTally tl;
   reset_tally(tl);
   uint32_t sec_id = 0;
-  warp_loop<MODE>(a, sh, iv, tl, sec_id, warp_tag);
+  warp_loop<MODE>(a, sh, iv, tl, sec_id, warp_tag, cur);
   block_flush(a, sh, tl, lane, wid);
 }
 
@@ -789,10 +807,11 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
     if (threadIdx.x == 0) s_iv = interval_view<-1>(s_a);
     __syncthreads();
     reset_tally(tl);
+    const WarpCursor cur{0, 0, 0, Sh::kChunk, false};
     if constexpr (Sh::kStash > 0)
-      warp_loop_stash<MODE>(s_a, sh, adv_stash + wid * 4 * Sh::kStash, s_iv, tl, sec_id, warp_tag);
+      warp_loop_stash<MODE>(s_a, sh, adv_stash + wid * 4 * Sh::kStash, s_iv, tl, sec_id, warp_tag, cur);
     else
-      warp_loop<MODE>(s_a, sh, s_iv, tl, sec_id, warp_tag);
+      warp_loop<MODE>(s_a, sh, s_iv, tl, sec_id, warp_tag, cur);
     __syncthreads();  // every warp is done with the slot
     block_flush(s_a, sh, tl, lane, wid);
     __syncthreads();  // the flush has read the shared tallies and arguments

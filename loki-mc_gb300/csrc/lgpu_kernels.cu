@@ -953,23 +953,40 @@ inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; 
 
 }  // namespace
 
-void launch_advance(const AdvanceArgs& a, cudaStream_t s) {
-#define LGPU_ADVANCE(K, G, B)                                  \
-  switch (a.field.mode) {                                      \
-    case kFieldDC: K<kFieldDC><<<G, B, 0, s>>>(a); break;      \
-    case kFieldAC: K<kFieldAC><<<G, B, 0, s>>>(a); break;      \
-    case kFieldB: K<kFieldB><<<G, B, 0, s>>>(a); break;        \
-    case kFieldECR: K<kFieldECR><<<G, B, 0, s>>>(a); break;    \
-    default: K<kFieldACB><<<G, B, 0, s>>>(a); break;           \
+// The main pass over one condition's ensemble. The electrons are spread over all
+// warps the device holds: one per lane while they last (an electron's events follow
+// one another, so a second electron of the lane only adds to the longest chain),
+// else each warp starts on four fifths of an even share and takes the rest 32 at a
+// time. Every warp taking 128 at a time from a counter instead kept one SM in 15
+// busy with 10,000 electrons, and left the last chunks to a few warps at 1e6:
+// 10,000 electrons (atomic gas, DC) 38 -> 23 us, 33,333 (Reid) 34 -> 17, 100,000
+// (mixture, crossed B, thermal) 58 -> 38, 1e6 (N2-like) 85 -> 74, 4e6 unchanged
+// at 194. The collision stash of the batched shapes waits for 32 collisions at the
+// end of every condition and is no faster here (79 us at 1e6, 194 at 4e6).
+void launch_advance(const AdvanceArgs& args, cudaStream_t s) {
+  AdvanceArgs a = args;
+  int grid = 1, threads = 32;
+  if (!a.queue_only) {
+    // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
+    threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
+    const int warps = threads / 32, per_sm = kAdvanceBlocksPerSM * kAdvanceThreads / threads;
+    grid = max(1, min(a.sm_count * per_sm, (a.n + threads - 1) / threads));
+    const int all = grid * warps;
+    a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
+    a.chunk = 32;
+  }
+#define LGPU_ADVANCE(K)                                               \
+  switch (a.field.mode) {                                             \
+    case kFieldDC: K<kFieldDC><<<grid, threads, 0, s>>>(a); break;    \
+    case kFieldAC: K<kFieldAC><<<grid, threads, 0, s>>>(a); break;    \
+    case kFieldB: K<kFieldB><<<grid, threads, 0, s>>>(a); break;      \
+    case kFieldECR: K<kFieldECR><<<grid, threads, 0, s>>>(a); break;  \
+    default: K<kFieldACB><<<grid, threads, 0, s>>>(a); break;         \
   }
   if (a.queue_only) {
-    LGPU_ADVANCE(k_advance_drain, 1, 32)
+    LGPU_ADVANCE(k_advance_drain)
   } else {
-    // persistent grid: at most kAdvanceBlocksPerSM blocks per SM, fewer when
-    // the electrons do not fill them (one chunk per warp)
-    const int warps_needed = (a.n + AdvShape<0>::kChunk - 1) / AdvShape<0>::kChunk;
-    const int grid = max(1, min(a.sm_count * kAdvanceBlocksPerSM, (warps_needed + 7) / 8));
-    LGPU_ADVANCE(k_advance, grid, kAdvanceThreads)
+    LGPU_ADVANCE(k_advance)
   }
 #undef LGPU_ADVANCE
 }

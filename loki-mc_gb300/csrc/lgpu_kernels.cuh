@@ -80,6 +80,9 @@ struct AdvanceArgs {
   int real_batch;                  // pending real collisions that start a warp's collision turn (1..32)
   int coarse;                      // 1: null test against the block bounds first (t.nu_coarse)
   int local_q;                     // secondaries a warp queues before it spills (1..kLocalQ)
+  // one condition per launch: the electrons each warp starts on, and the ones it
+  // takes at a time from the work counter after them (set by launch_advance)
+  int share, chunk;
 };
 constexpr int kDefaultRealBatch = 20;
 

@@ -46,3 +46,23 @@ def test_sample_counts_what_the_separate_passes_count(n, cells, freq, thermal):
     batch.close()
     alone.close()
     batched.close()
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 65, 19455, 19457, 155647, 155649, 155681, 700001])
+def test_every_electron_is_advanced_once_alone(n):
+    """The solve alone spreads the ensemble over its warps by size (blocks of two
+    warps, one electron per lane, shares and chunks of 32): collision counts equal
+    the batched solve's, whose warps take chunks from a counter."""
+    from lokigpu import capi
+    alone = _context(n, DEFAULT, 0.0, 0)
+    a = alone.solve()
+    batched = _context(n, DEFAULT, 0.0, 0)
+    batch = capi.Batch(0, 1)
+    batch.add(batched)
+    res, status, _ = batch.run()
+    assert status == [0]
+    assert (a.real_collisions, a.null_collisions) == (res[0].real_collisions, res[0].null_collisions)
+    np.testing.assert_array_equal(alone.process_results()[0], batched.process_results()[0])
+    batch.close()
+    alone.close()
+    batched.close()
