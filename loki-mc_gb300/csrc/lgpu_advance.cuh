@@ -95,7 +95,7 @@ constexpr int kAdvanceWarps = kAdvanceThreads / 32;
 // warp's own queue (shared memory) and an idle lane of the same warp pushes it
 // from its creation time to the end of the interval: the creating lane keeps
 // the warp alive, so no warp ever waits on another. A warp whose queue is full
-// spills to a global buffer that the one-warp drain launch works off after.
+// spills to a global buffer that is worked off after the launch (drain_body).
 constexpr int kLocalQ = 32;
 
 // Shared memory of an advance block: constants and per-process tallies of the
@@ -477,12 +477,15 @@ constexpr bool kPrefetchChunk = true;  // a claimed chunk's states, at the claim
 constexpr bool kPrefetchRows = true;   // a parked collision's cumulative row (stash shapes)
 
 // A warp's place in the ensemble (warp-uniform): the electrons [next, end) it
-// holds, and where it takes more: chunks of `chunk` electrons from `base` on, by
-// the work counter. A context on its own starts each warp on a share of its own
-// (no counter, no wait) and leaves the rest, if any, to the counter.
+// holds, and where it takes more: CHUNK electrons at a time from `base` on, by the
+// work counter. OWN: a context on its own starts each warp on a share of its own
+// (no counter, no wait) and leaves the rest, if any, to the counter; else all
+// electrons go by the counter.
+template <int CHUNK, bool OWN>
 struct WarpCursor {
-  int next, end, base, chunk;
-  bool exhausted;
+  int next = 0, end = 0;
+  bool exhausted = false;
+  int base = 0;  // OWN only
 };
 
 __device__ __forceinline__ void prefetch_states(const AdvanceArgs& a, int first, int end) {
@@ -493,23 +496,25 @@ __device__ __forceinline__ void prefetch_states(const AdvanceArgs& a, int first,
 // claiming lanes (this one `wants` it, rank r among them) take the next
 // electrons of the warp's chunk, and of a new chunk from the work counter
 // when it runs out.
+template <int CHUNK, bool OWN>
 __device__ __forceinline__ int lane_claim(const AdvanceArgs& a, int n_want, int r, bool wants, int lane, int n_el,
-                                          WarpCursor& w) {
+                                          WarpCursor<CHUNK, OWN>& w) {
   int idx = -1;
   const int take = min(n_want, w.end - w.next);
   if (wants && r < take) idx = w.next + r;
   w.next += take;
   if (n_want > take) {
-    int base = n_el;
-    if (w.base < n_el) {
-      if (lane == 0) base = w.base + atomicAdd(a.work_counter, w.chunk);
+    int base = 0;
+    if (!OWN || w.base < n_el) {
+      if (lane == 0) base = atomicAdd(a.work_counter, CHUNK);
       base = __shfl_sync(0xffffffffu, base, 0);
     }
+    if (OWN) base += w.base;
     if (base >= n_el) {
       w.exhausted = true;
     } else {
       w.next = base;
-      w.end = min(base + w.chunk, n_el);
+      w.end = min(base + CHUNK, n_el);
       if (kPrefetchChunk && lane == 0) prefetch_states(a, base, w.end);
       const int r2 = r - take;
       const int take2 = min(n_want - take, w.end - w.next);
@@ -521,30 +526,30 @@ __device__ __forceinline__ int lane_claim(const AdvanceArgs& a, int n_want, int 
 }
 
 // Lanes without an electron (`need`) take the next ones of the warp's chunk.
+template <class Cursor>
 __device__ __forceinline__ void lane_take_chunk(const AdvanceArgs& a, const IntervalView& iv, Lane& L,
-                                                unsigned need, int lane, unsigned lt_mask, int n_el, WarpCursor& w) {
+                                                unsigned need, int lane, unsigned lt_mask, int n_el, Cursor& w) {
   const int idx = lane_claim(a, __popc(need), __popc(need & lt_mask), !L.have, lane, n_el, w);
   if (idx >= 0) lane_take_electron(a, iv, L, idx);
 }
 
 // The warps' work on one condition: the ensemble in warp chunks from `cur` on,
-// then each warp's queued secondaries (or, drain, only the spilled secondaries). Returns when the condition's counter
-// and the warp's queue are exhausted; the caller flushes the lane sums.
-template <int MODE, class Sh>
+// then each warp's queued secondaries (DRAIN: only the spilled secondaries). Returns
+// when the condition's counter and the warp's queue are exhausted; the caller
+// flushes the lane sums.
+template <int MODE, bool DRAIN, class Sh, class Cursor>
 __device__ __forceinline__ void warp_loop(const AdvanceArgs& a, Sh& sh, const IntervalView& iv,
-                                          LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag, WarpCursor cur) {
-  const bool drain = a.queue_only != 0;
-  const int n_el = drain ? 0 : a.n;
+                                          LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag, Cursor cur) {
+  const int n_el = DRAIN ? 0 : a.n;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
   Lane L;
   reset_lane(L);
   int sp_next = 0;  // warp-uniform place in the spill buffer (drain only)
-  if (drain) cur.exhausted = true;
 
   for (;;) {
     __syncwarp();
-    if (drain) __threadfence();
+    if (DRAIN) __threadfence();
     // ---- refill lanes without an electron: the warp's own queued secondaries
     // first (the queue stays short, so it rarely spills), then the ensemble
     // chunk, then (drain) the spilled secondaries
@@ -552,23 +557,21 @@ __device__ __forceinline__ void warp_loop(const AdvanceArgs& a, Sh& sh, const In
     if (qn > 0) qn = lane_take_queued(a, iv, sh, wid, lane, lt_mask, L, tl, sec_id, warp_tag);
     const unsigned need = __ballot_sync(0xffffffffu, !L.have);
     if (need && !cur.exhausted) lane_take_chunk(a, iv, L, need, lane, lt_mask, n_el, cur);
-    if (cur.exhausted) {
-      if (drain) {
-        const unsigned idle2 = __ballot_sync(0xffffffffu, !L.have);
-        const int cnt = min(*(volatile int*)a.spill_count, a.spill_cap);
-        const int r2 = __popc(idle2 & lt_mask);
-        const int take2 = min(__popc(idle2), cnt - sp_next);
-        if (((idle2 >> lane) & 1u) && r2 < take2) {
-          const int k = sp_next + r2;
-          lane_take_secondary(a, iv, L, tl, __ldcg(&a.spill[2 * k]), __ldcg(&a.spill[2 * k + 1]),
-                              0xFFFFFFFFu, (uint32_t)k);
-        }
-        sp_next += max(take2, 0);
+    if (DRAIN) {
+      const unsigned idle2 = __ballot_sync(0xffffffffu, !L.have);
+      const int cnt = min(*(volatile int*)a.spill_count, a.spill_cap);
+      const int r2 = __popc(idle2 & lt_mask);
+      const int take2 = min(__popc(idle2), cnt - sp_next);
+      if (((idle2 >> lane) & 1u) && r2 < take2) {
+        const int k = sp_next + r2;
+        lane_take_secondary(a, iv, L, tl, __ldcg(&a.spill[2 * k]), __ldcg(&a.spill[2 * k + 1]),
+                            0xFFFFFFFFu, (uint32_t)k);
       }
+      sp_next += max(take2, 0);
     }
     const unsigned live = __ballot_sync(0xffffffffu, L.have);
     if (!live) {
-      const bool spill_left = drain && sp_next < min(*(volatile int*)a.spill_count, a.spill_cap);
+      const bool spill_left = DRAIN && sp_next < min(*(volatile int*)a.spill_count, a.spill_cap);
       if (cur.exhausted && qn == 0 && !spill_left) break;
       continue;
     }
@@ -653,10 +656,10 @@ __device__ __forceinline__ void stash_swap(float4* wst, int e, Lane& L) {
 // flying an electron take the lowest of them and leave their electron in its
 // place, on top of the ready ones; empty lanes, which exist only once nothing
 // is ready, take the rest. So np + nr <= 63 throughout.
-template <int MODE, class Sh>
+template <int MODE, class Sh, class Cursor>
 __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, float4* wst, const IntervalView& iv,
                                                 LaneTally& tl, uint32_t& sec_id, uint32_t warp_tag,
-                                                WarpCursor cur) {
+                                                Cursor cur) {
   constexpr int NS = Sh::kStash;
   static_assert(NS >= 64, "the stash holds up to 63 records");
   const int n_el = a.n;
@@ -735,20 +738,42 @@ __device__ __forceinline__ void warp_loop_stash(const AdvanceArgs& a, Sh& sh, fl
   }
 }
 
-// One condition per launch (or, drain, its spilled secondaries): every warp
-// starts on its own a.share electrons.
+// The secondaries of one condition that its warps could not queue, pushed to the
+// end of the interval by the first warp of a block (every thread of it calls this;
+// `a` lies in shared memory). Their streams carry the warp tag 0xFFFFFFFF, those of
+// the secondaries they create the salt 3 and the tag 0.
+template <class Sh>
+__device__ __forceinline__ void drain_body(AdvanceArgs& a, Sh& sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) a.salt = 2;
+  load_block_consts(a, sh);
+  __syncthreads();
+  LaneTally tl;
+  reset_tally(tl);
+  if (wid == 0) {
+    uint32_t sec_id = 0;
+    WarpCursor<32, false> none;
+    none.exhausted = true;
+    warp_loop<-1, true>(a, sh, interval_view<-1>(a), tl, sec_id, 0u, none);
+  }
+  __syncthreads();
+  block_flush(a, sh, tl, lane, wid);
+  __syncthreads();
+}
+
+// One condition per launch: every warp starts on its own a.share electrons and takes
+// kOwnChunk at a time after them.
+constexpr int kOwnChunk = 32;
+
 template <int MODE, class Sh>
 __device__ __forceinline__ void advance_body(const AdvanceArgs& a, Sh& sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int warps = (int)(blockDim.x >> 5);
-  // drain launches: one block, whose warp tag stays below the spill's 0xFFFFFFFF
   const uint32_t warp_tag = (uint32_t)(blockIdx.x * warps + wid);
-  WarpCursor cur;
+  WarpCursor<kOwnChunk, true> cur;
   cur.next = min((int)warp_tag * a.share, a.n);
   cur.end = min(cur.next + a.share, a.n);
   cur.base = (int)gridDim.x * warps * a.share;
-  cur.chunk = a.chunk;
-  cur.exhausted = false;
   if (kPrefetchChunk && lane == 0 && cur.end > cur.next) prefetch_states(a, cur.next, cur.end);
   load_block_consts(a, sh);
   __syncthreads();
@@ -756,7 +781,7 @@ __device__ __forceinline__ void advance_body(const AdvanceArgs& a, Sh& sh) {
   LaneTally tl;
   reset_tally(tl);
   uint32_t sec_id = 0;
-  warp_loop<MODE>(a, sh, iv, tl, sec_id, warp_tag, cur);
+  warp_loop<MODE, false>(a, sh, iv, tl, sec_id, warp_tag, cur);
   block_flush(a, sh, tl, lane, wid);
 }
 
@@ -807,11 +832,11 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
     if (threadIdx.x == 0) s_iv = interval_view<-1>(s_a);
     __syncthreads();
     reset_tally(tl);
-    const WarpCursor cur{0, 0, 0, Sh::kChunk, false};
+    const WarpCursor<Sh::kChunk, false> cur;
     if constexpr (Sh::kStash > 0)
       warp_loop_stash<MODE>(s_a, sh, adv_stash + wid * 4 * Sh::kStash, s_iv, tl, sec_id, warp_tag, cur);
     else
-      warp_loop<MODE>(s_a, sh, s_iv, tl, sec_id, warp_tag, cur);
+      warp_loop<MODE, false>(s_a, sh, s_iv, tl, sec_id, warp_tag, cur);
     __syncthreads();  // every warp is done with the slot
     block_flush(s_a, sh, tl, lane, wid);
     __syncthreads();  // the flush has read the shared tallies and arguments

@@ -7,9 +7,9 @@
 // graph launches: first the previous samples' distribution tallies (launched
 // before the host works through the conditions, so that its work runs beside
 // them), then slot control blocks and scalars (prep), one persistent advance
-// launch per field branch over all slots' electrons, the drain of spilled
-// secondaries, population control over all slots' items, the moment sums and
-// a gather of every slot's scalars into mapped host memory. Per interval the
+// launch per field branch over all slots' electrons, spilled secondaries and
+// population control over all slots' items, the moment sums and a gather of every
+// slot's scalars into mapped host memory. Per interval the
 // host stages one BatchSlot per running condition (the argument blocks the
 // single-condition launches take, plus the interval's control block) into
 // pinned memory and copies it over once. A condition whose energy grid is

@@ -126,7 +126,7 @@ class Engine {
   // in one allocation.
   struct SecondarySet {
     char* base = nullptr;
-    int *alive = nullptr, *removed = nullptr, *pair_slot = nullptr, *pair_sec = nullptr;
+    int *removed = nullptr, *pair_slot = nullptr, *pair_sec = nullptr;
     float4 *spill = nullptr, *sec = nullptr;
     unsigned int* claim = nullptr;
     size_t claim_words = 0;
@@ -134,7 +134,7 @@ class Engine {
   cudaError_t alloc_secondaries(int cap, SecondarySet* o) const {
     Carve cv;
     const size_t words = ((size_t)N_ + cap + 31) / 32;
-    const size_t a = cv.take<int>(cap), sp = cv.take<float4>(2 * (size_t)cap), se = cv.take<float4>(2 * (size_t)cap);
+    const size_t sp = cv.take<float4>(2 * (size_t)cap), se = cv.take<float4>(2 * (size_t)cap);
     const size_t cl = cv.take<unsigned int>(words), rm = cv.take<int>(cap), ps = cv.take<int>(cap);
     const size_t pc = cv.take<int>(cap);
     const cudaError_t e = cudaMalloc((void**)&o->base, cv.bytes);
@@ -142,7 +142,6 @@ class Engine {
       o->base = nullptr;
       return e;
     }
-    o->alive = at<int>(o->base, a);
     o->spill = at<float4>(o->base, sp);
     o->sec = at<float4>(o->base, se);
     o->claim = at<unsigned int>(o->base, cl);
@@ -154,7 +153,6 @@ class Engine {
   }
   void use_secondaries(const SecondarySet& q) {
     d_secbuf_ = q.base;
-    d_alive_ = q.alive;
     d_spill_ = q.spill;
     d_sec_ = q.sec;
     d_claim_ = q.claim;
@@ -712,12 +710,12 @@ class Engine {
     p.n_electrons = N_;
     p.sec = d_sec_;
     p.sec_count = &d_sc_->sec_count;
+    p.spill_count = &d_sc_->spill_count;
     p.sec_cap = sec_cap_;
     p.counts = d_sc_->pop_counts;
     p.att_list = d_att_;
     p.att_count = &d_sc_->att_count;
     p.claim = d_claim_;
-    p.alive = d_alive_;
     p.removed = d_removed_;
     p.pair_slot = d_pair_slot_;
     p.pair_sec = d_pair_sec_;
@@ -730,9 +728,9 @@ class Engine {
   }
 
   // The device work of one interval: the advance of every electron and of the
-  // secondaries they create, the drain of any secondary left in the queue,
-  // population control (when the mixture ionizes or attaches), the ensemble
-  // sample and the scalar read-back. Captured once as a CUDA graph.
+  // secondaries they create, any secondary its warps could not queue and population
+  // control (when the mixture ionizes or attaches), the ensemble sample and the
+  // scalar read-back. Captured once as a CUDA graph.
   void enqueue_interval(bool sample) {
     copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice);
     cudaMemsetAsync(d_sc_, 0, offsetof(DevScalars, null_count), stream_);
@@ -742,12 +740,8 @@ class Engine {
     cudaEventRecordWithFlags(ev1_, stream_, cudaEventRecordExternal);
     ++launches_;
     if (have_ion_att_) {
-      AdvanceArgs d = a;
-      d.queue_only = 1;
-      d.salt = 2;
-      launch_advance(d, stream_);
-      launch_pop_control(pop_args(), stream_);
-      launches_ += 1 + kPopLaunches;
+      launch_pop_control(a, pop_args(), stream_);
+      launches_ += kPopLaunches;
     }
     if (sample) enqueue_sample(true);
     copy(h_sc_, d_sc_, sizeof(DevScalars), cudaMemcpyDeviceToHost);
@@ -1402,7 +1396,7 @@ class Engine {
     const double N = c.n_electrons, cap = initial_sec_cap(c), M = c.n_interp;
     const double stride = (double)((P + 1) & ~1);
     double b = N * 2 * sizeof(float4);                      // state
-    b += cap * (sizeof(int) * 4 + 4 * sizeof(float4));      // alive, removed, pair_slot/sec; spill, sec
+    b += cap * (sizeof(int) * 3 + 4 * sizeof(float4));      // removed, pair_slot/sec; spill, sec
     b += N * sizeof(int) + (N + cap) / 8.0;                 // attached list, claim bitmap
     b += M * (sizeof(float2) + 2 * sizeof(double));         // nu pairs, nu_tot, nu_max
     b += 2.0 * M * stride * sizeof(float2);                 // cumulative and sigma row pairs
@@ -1927,7 +1921,6 @@ class Engine {
   // device buffers (carved from d_core_, d_secbuf_ and d_procbuf_) and the pinned host block
   char *d_core_ = nullptr, *d_secbuf_ = nullptr, *d_procbuf_ = nullptr, *h_pinned_ = nullptr;
   float4* d_state_ = nullptr;
-  int* d_alive_ = nullptr;
   float4* d_spill_ = nullptr;
   float4* d_sec_ = nullptr;
   int* d_att_ = nullptr;

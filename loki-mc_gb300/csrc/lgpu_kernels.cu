@@ -21,41 +21,12 @@ namespace lgpu {
 
 namespace {
 
-// the main pass over the ensemble and the drain of left-over secondaries
-// carry different names so that profiles can tell them apart
+// the main pass over the ensemble
 template <int MODE>
-__global__ void __launch_bounds__(kAdvanceThreads, kAdvanceBlocksPerSM) k_advance(AdvanceArgs a) {
+__global__ void __launch_bounds__(kAdvanceThreads, kAdvanceBlocksPerSM) k_advance(const __grid_constant__ AdvanceArgs a) {
   __shared__ AdvShared sh;
   advance_body<MODE>(a, sh);
 }
-template <int MODE>
-__global__ void __launch_bounds__(32) k_advance_drain(AdvanceArgs a) {
-  __shared__ AdvShared sh;
-  // the warps took their own queues during the advance: only spilled
-  // secondaries are left (the count is final: the advance launch came first)
-  if (*(volatile const int*)a.spill_count == 0) return;
-  advance_body<MODE>(a, sh);
-}
-
-// the drain of every slot's spilled secondaries: one warp per slot
-__global__ void __launch_bounds__(32) k_advance_drain_batch(BatchArgs b) {
-  __shared__ AdvShared sh;
-  __shared__ AdvanceArgs s_a;
-  const int slot = blockIdx.x;
-  if (slot >= b.hdr->n_slots || !(b.slots[slot].flags & kSlotIonAtt)) return;
-  // the warps took their own queues during the advance: only spilled
-  // secondaries are left (the count is final: the advance launches came first)
-  if (*(volatile const int*)b.slots[slot].adv.spill_count == 0) return;
-  load_slot_args(&b.slots[slot].adv, &s_a);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_a.queue_only = 1;
-    s_a.salt = 2;
-  }
-  __syncthreads();
-  advance_body<-1>(s_a, sh);
-}
-
 // ------------------------------------------------------------------ init
 __global__ void k_init(InitArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -516,22 +487,31 @@ __device__ __forceinline__ void add_growth(double* growth, double e) {
 __device__ __forceinline__ float energy4(float4 B, float hme) { return energy_of(make_float3(B.x, B.y, B.z), hme); }
 
 // Population control (BoltzmannMC.C:1282-1408), when all electrons and
-// secondaries are at the synchronisation time. Five launches, each a grid of
-// blocks over one or many slots (blockIdx.y) whose threads stride over the
-// slot's items:
-//  (0) the secondaries that did not attach are listed (alive);
-//  (1) attached slots take secondaries, one per slot (:1344-1359); the slots
-//      that stay attached are marked in the claim bitmap, so that no clone is
-//      made from another clone;
-//  (2) the slots still attached clone a random non-attached electron, whose
-//      energy enters the growth term (:1360-1376); or, when secondaries are
-//      left over, a uniformly random subset of size m is drawn from the pool of
-//      N slots + m unplaced secondaries - the outcome of the reference's
-//      sequential uniform removal (:1379-1407) - by claiming pool bits;
-//  (3) clone marks are cleared; the removed ensemble slots and the unremoved
-//      secondaries are listed, removed energies leave the growth term;
-//  (4) the listed secondaries move into the removed slots; removal marks are
-//      cleared, so the bitmap is zero again.
+// secondaries are at the synchronisation time (every listed secondary is alive:
+// one that attached was not listed). The secondaries that a condition's warps could
+// not queue come first: there seldom are any, and then one block pushes them and
+// does the condition's first phase. Three launches, each a grid over the items
+// of one or many slots. With n_att attached slots and n_sec secondaries:
+//  (a) the first min(n_att, n_sec) attached slots take the last secondaries
+//      (:1344-1359); slots left attached are marked in the claim bitmap, so that no
+//      clone is made from another clone; or, when secondaries are left over, a
+//      uniformly random subset of their number m is drawn from the pool of N slots
+//      + m unplaced secondaries - the outcome of the reference's sequential uniform
+//      removal (:1379-1407) - by claiming pool bits. No item depends on another:
+//      marks and draws never meet in one interval, and a slot drawn while it takes
+//      its secondary is read in the next phase;
+//  (b) the slots left attached clone a random non-attached electron, whose energy
+//      enters the growth term (:1360-1376); or the removed ensemble slots and the
+//      unremoved secondaries are listed, removed energies leave the growth term;
+//  (c) the listed secondaries move into the removed slots; all marks are cleared,
+//      so the bitmap is zero again.
+//
+// Bound by latency: a handful of dependent loads per launch on few items. Listing,
+// filling, drawing, sorting and placing in a launch each, after another for the
+// spilled secondaries, took 25 us per interval for 1e6 electrons alone and 39 for
+// 32 conditions of 10,000-30,000; these three take 15 and 24. One launch of a
+// cluster per condition with a barrier between the phases took 14 and 26, but 7 %
+// more of the whole sweep: its largest conditions need more than a cluster's threads.
 constexpr int kPopThreads = 256;
 constexpr int kPopBlocks = 64;           // blocks, single condition
 constexpr int kPopBlocksPerSM = 2;       // blocks per SM, batches
@@ -539,7 +519,9 @@ constexpr int kPopBlocksPerSM = 2;       // blocks per SM, batches
 // one condition, arguments by value
 struct PopOne {
   PopArgs a;
+  AdvanceArgs adv;
   __device__ int count() const { return 1; }
+  __device__ const AdvanceArgs* advance(int) const { return &adv; }
   __device__ const PopArgs* get(int s) const { return s == 0 ? &a : nullptr; }
 };
 // the slots of a batch that ionize or attach
@@ -547,6 +529,7 @@ struct PopBatch {
   const BatchHeader* hdr;
   const BatchSlot* slots;
   __device__ int count() const { return hdr->n_slots; }
+  __device__ const AdvanceArgs* advance(int s) const { return &slots[s].adv; }
   __device__ const PopArgs* get(int s) const {
     return (s < hdr->n_slots && (slots[s].flags & kSlotIonAtt)) ? &slots[s].pop : nullptr;
   }
@@ -616,8 +599,7 @@ __device__ __forceinline__ int pop_plan(const Src& src, int n, Items items, PopP
 
 // body(a, i) for every item i of every slot
 template <class Src, class Items, class Body>
-__device__ __forceinline__ void pop_phase(const Src& src, Items items, Body body) {
-  __shared__ PopPlan pl;
+__device__ __forceinline__ void pop_phase(const Src& src, PopPlan& pl, Items items, Body body) {
   const int n = src.count();
   const int total = pop_plan(src, n, items, pl);
   const int lane = threadIdx.x & 31;
@@ -634,136 +616,131 @@ __device__ __forceinline__ void pop_phase(const Src& src, Items items, Body body
   }
 }
 
-template <class Src>
-__global__ void __launch_bounds__(kPopThreads) k_pop_list(Src src) {
-  pop_phase(
-      src, [](const PopArgs& a) { return pop_sec_total(a); },
-      [](const PopArgs& a, int j) {
-        if (a.sec[2 * j + 1].w == 0.0f) a.alive[append_slot(&a.counts[0])] = j;
-      });
+__device__ __forceinline__ int pop_attached(const PopArgs& a) { return *a.att_count; }
+// attached slots and left-over secondaries (items of the first phase), and how many
+// more there are of one than of the other (items of the others)
+__device__ __forceinline__ int pop_left(const PopArgs& a) { return abs(pop_attached(a) - pop_sec_total(a)); }
+
+// items of the first phase: the attached slots and the removal draws
+__device__ __forceinline__ int pop_fill_items(const PopArgs& a) { return max(pop_attached(a), pop_sec_total(a)); }
+
+__device__ __forceinline__ void pop_fill_item(const PopArgs& a, int i) {
+  const int n_att = pop_attached(a), n_sec = pop_sec_total(a);
+  if (i < n_att) {
+    const int slot = a.att_list[i];
+    if (i < n_sec) {
+      const int k = n_sec - 1 - i;
+      a.state[2 * slot] = a.sec[2 * k];
+      a.state[2 * slot + 1] = a.sec[2 * k + 1];
+    } else {
+      atomicOr(&a.claim[slot >> 5], 1u << (slot & 31));
+    }
+    return;
+  }
+  const int j = i - n_att, pool = a.n_electrons + (n_sec - n_att);
+  const uint64_t interval = a.ctl->interval;
+  int got = -1;
+  for (uint32_t d = 0; d < 4096u; ++d) {
+    const int r = uniform_index(pop_word((uint32_t)j, interval, a.seed, 2u, d), pool);
+    const unsigned int bit = 1u << (r & 31);
+    const unsigned int old = atomicOr(&a.claim[r >> 5], bit);
+    if (!(old & bit)) {
+      got = r;
+      break;
+    }
+  }
+  a.removed[j] = got;
+  if (got < 0) atomicExch(a.error_flag, 5);
 }
 
-// items: every attached slot; the first min(n_att, n_sec) take secondaries,
-// the rest are marked for clones
+// the drain's shared memory: the process constants stay in global memory
+using DrainShared = AdvSharedT<kPopThreads / 32, 32, 1>;
+
 template <class Src>
-__global__ void __launch_bounds__(kPopThreads) k_pop_fill(Src src) {
+__global__ void __launch_bounds__(kPopThreads) k_pop_fill(const __grid_constant__ Src src) {
+  __shared__ DrainShared sh;
+  __shared__ AdvanceArgs s_a;
+  __shared__ PopPlan pl;
+  // (a slot's spill count is final here except for its own drain, which only raises it)
+  auto spilled = [](const AdvanceArgs& a) { return *(volatile const int*)a.spill_count != 0; };
+  for (int s = blockIdx.x; s < src.count(); s += gridDim.x) {
+    const PopArgs* a = src.get(s);
+    if (!a || !spilled(*src.advance(s))) continue;
+    __syncthreads();
+    load_slot_args(src.advance(s), &s_a);
+    __syncthreads();
+    drain_body(s_a, sh);
+    for (int i = threadIdx.x; i < pop_fill_items(*a); i += blockDim.x) pop_fill_item(*a, i);
+  }
   pop_phase(
-      src, [](const PopArgs& a) { return *a.att_count; },
-      [](const PopArgs& a, int j) {
-        const int n_att = *a.att_count, n_sec = a.counts[0];
-        const int k = min(n_att, n_sec);
-        if (j < k) {
-          const int slot = a.att_list[j];
-          const int sidx = a.alive[n_sec - 1 - j];
-          a.state[2 * slot] = a.sec[2 * sidx];
-          a.state[2 * slot + 1] = a.sec[2 * sidx + 1];
-        } else {
-          const int dest = a.att_list[j];
-          atomicOr(&a.claim[dest >> 5], 1u << (dest & 31));
-        }
-      });
+      src, pl,
+      [&](const PopArgs& a) { return *(volatile const int*)a.spill_count != 0 ? 0 : pop_fill_items(a); },
+      [](const PopArgs& a, int i) { pop_fill_item(a, i); });
 }
 
-// items: the clones (n_att > n_sec) or the removal draws (n_sec > n_att)
 template <class Src>
-__global__ void __launch_bounds__(kPopThreads) k_pop_draw(Src src) {
-  pop_phase(
-      src, [](const PopArgs& a) { return abs(*a.att_count - a.counts[0]); },
-      [](const PopArgs& a, int item) {
-        const int n_att = *a.att_count, n_sec = a.counts[0];
-        const uint64_t interval = a.ctl->interval;
-        if (n_att > n_sec) {
-          const int j = n_sec + item;
-          const int dest = a.att_list[j];
-          int src_slot = -1;
-          for (uint32_t d = 0; d < 4096u; ++d) {
-            const int r = uniform_index(pop_word((uint32_t)j, interval, a.seed, 1u, d), a.n_electrons);
-            if (!claimed(a.claim, r) && a.state[2 * r + 1].w == 0.0f) {
-              src_slot = r;
-              break;
-            }
-          }
-          if (src_slot < 0) {
-            atomicExch(a.error_flag, 4);
-            return;
-          }
-          const float4 A = a.state[2 * src_slot], B = a.state[2 * src_slot + 1];
-          a.state[2 * dest] = A;
-          a.state[2 * dest + 1] = B;
-          add_growth(a.growth, (double)energy4(B, a.half_me_over_e));
-        } else {
-          const int j = item;
-          const int pool = a.n_electrons + (n_sec - n_att);
-          int got = -1;
-          for (uint32_t d = 0; d < 4096u; ++d) {
-            const int r = uniform_index(pop_word((uint32_t)j, interval, a.seed, 2u, d), pool);
-            const unsigned int bit = 1u << (r & 31);
-            const unsigned int old = atomicOr(&a.claim[r >> 5], bit);
-            if (!(old & bit)) {
-              got = r;
-              break;
-            }
-          }
-          a.removed[j] = got;
-          if (got < 0) atomicExch(a.error_flag, 5);
+__global__ void __launch_bounds__(kPopThreads) k_pop_clone(Src src) {
+  __shared__ PopPlan pl;
+  pop_phase(src, pl, pop_left, [](const PopArgs& a, int item) {
+    const int n_att = pop_attached(a), n_sec = pop_sec_total(a);
+    if (n_att > n_sec) {
+      const int j = n_sec + item;
+      const int dest = a.att_list[j];
+      const uint64_t interval = a.ctl->interval;
+      int src_slot = -1;
+      for (uint32_t d = 0; d < 4096u; ++d) {
+        const int r = uniform_index(pop_word((uint32_t)j, interval, a.seed, 1u, d), a.n_electrons);
+        if (!claimed(a.claim, r) && a.state[2 * r + 1].w == 0.0f) {
+          src_slot = r;
+          break;
         }
-      });
+      }
+      if (src_slot < 0) {
+        atomicExch(a.error_flag, 4);
+        return;
+      }
+      const float4 A = a.state[2 * src_slot], B = a.state[2 * src_slot + 1];
+      a.state[2 * dest] = A;
+      a.state[2 * dest + 1] = B;
+      add_growth(a.growth, (double)energy4(B, a.half_me_over_e));
+      return;
+    }
+    const int r = a.removed[item];
+    if (r >= 0 && r < a.n_electrons) {
+      a.pair_slot[append_slot(&a.counts[0])] = r;
+      add_growth(a.growth, -(double)energy4(a.state[2 * r + 1], a.half_me_over_e));
+    } else if (r >= a.n_electrons) {
+      add_growth(a.growth, -(double)energy4(a.sec[2 * (r - a.n_electrons) + 1], a.half_me_over_e));
+    }
+    if (!claimed(a.claim, a.n_electrons + item)) a.pair_sec[append_slot(&a.counts[1])] = item;
+  });
 }
 
-// items: the clone marks to clear (n_att > n_sec) or the removal outcomes to
-// list (n_sec > n_att)
-template <class Src>
-__global__ void __launch_bounds__(kPopThreads) k_pop_sort(Src src) {
-  pop_phase(
-      src, [](const PopArgs& a) { return abs(*a.att_count - a.counts[0]); },
-      [](const PopArgs& a, int item) {
-        const int n_att = *a.att_count, n_sec = a.counts[0];
-        if (n_att > n_sec) {
-          const int dest = a.att_list[n_sec + item];
-          atomicAnd(&a.claim[dest >> 5], ~(1u << (dest & 31)));
-          return;
-        }
-        const int j = item;
-        const int r = a.removed[j];
-        if (r >= 0 && r < a.n_electrons) {
-          a.pair_slot[append_slot(&a.counts[1])] = r;
-          add_growth(a.growth, -(double)energy4(a.state[2 * r + 1], a.half_me_over_e));
-        } else if (r >= a.n_electrons) {
-          add_growth(a.growth, -(double)energy4(a.sec[2 * a.alive[r - a.n_electrons] + 1], a.half_me_over_e));
-        }
-        if (!claimed(a.claim, a.n_electrons + j)) a.pair_sec[append_slot(&a.counts[2])] = a.alive[j];
-      });
-}
-
-// items: the (removed slot, surviving secondary) pairs, then the removal
-// marks to clear
 template <class Src>
 __global__ void __launch_bounds__(kPopThreads) k_pop_place(Src src) {
-  pop_phase(
-      src,
-      [](const PopArgs& a) {
-        return min(a.counts[1], a.counts[2]) + max(a.counts[0] - *a.att_count, 0);
-      },
-      [](const PopArgs& a, int item) {
-        const int np = min(a.counts[1], a.counts[2]);
-        if (item < np) {
-          const int slot = a.pair_slot[item];
-          const int sidx = a.pair_sec[item];
-          a.state[2 * slot] = a.sec[2 * sidx];
-          a.state[2 * slot + 1] = a.sec[2 * sidx + 1];
-        } else {
-          const int r = a.removed[item - np];
-          if (r >= 0) atomicAnd(&a.claim[r >> 5], ~(1u << (r & 31)));
-        }
-      });
+  __shared__ PopPlan pl;
+  pop_phase(src, pl, pop_left, [](const PopArgs& a, int item) {
+    const int n_att = pop_attached(a), n_sec = pop_sec_total(a);
+    if (n_att > n_sec) {
+      const int dest = a.att_list[n_sec + item];
+      atomicAnd(&a.claim[dest >> 5], ~(1u << (dest & 31)));
+      return;
+    }
+    // as many secondaries survive as slots were removed, unless a draw gave up
+    if (item < min(a.counts[0], a.counts[1])) {
+      const int slot = a.pair_slot[item], k = a.pair_sec[item];
+      a.state[2 * slot] = a.sec[2 * k];
+      a.state[2 * slot + 1] = a.sec[2 * k + 1];
+    }
+    const int r = a.removed[item];
+    if (r >= 0) atomicAnd(&a.claim[r >> 5], ~(1u << (r & 31)));
+  });
 }
 
 template <class Src>
 void launch_pop_phases(const Src& src, int grid, cudaStream_t s) {
-  k_pop_list<<<grid, kPopThreads, 0, s>>>(src);
   k_pop_fill<<<grid, kPopThreads, 0, s>>>(src);
-  k_pop_draw<<<grid, kPopThreads, 0, s>>>(src);
-  k_pop_sort<<<grid, kPopThreads, 0, s>>>(src);
+  k_pop_clone<<<grid, kPopThreads, 0, s>>>(src);
   k_pop_place<<<grid, kPopThreads, 0, s>>>(src);
 }
 
@@ -786,7 +763,7 @@ __global__ void k_batch_prep(BatchArgs b) {
     sc->error_flag = 0;
     sc->max_energy_bits = 0u;
     sc->work_counter = 0;
-    sc->pop_counts[0] = sc->pop_counts[1] = sc->pop_counts[2] = 0;
+    sc->pop_counts[0] = sc->pop_counts[1] = 0;
   }
   if (sl.flags & kSlotSample) {
     if (lane < kMoments) sc->moments[lane] = 0.0;
@@ -965,30 +942,19 @@ inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; 
 // end of every condition and is no faster here (79 us at 1e6, 194 at 4e6).
 void launch_advance(const AdvanceArgs& args, cudaStream_t s) {
   AdvanceArgs a = args;
-  int grid = 1, threads = 32;
-  if (!a.queue_only) {
-    // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
-    threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
-    const int warps = threads / 32, per_sm = kAdvanceBlocksPerSM * kAdvanceThreads / threads;
-    grid = max(1, min(a.sm_count * per_sm, (a.n + threads - 1) / threads));
-    const int all = grid * warps;
-    a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
-    a.chunk = 32;
+  // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
+  const int threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
+  const int warps = threads / 32, per_sm = kAdvanceBlocksPerSM * kAdvanceThreads / threads;
+  const int grid = max(1, min(a.sm_count * per_sm, (a.n + threads - 1) / threads));
+  const int all = grid * warps;
+  a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
+  switch (a.field.mode) {
+    case kFieldDC: k_advance<kFieldDC><<<grid, threads, 0, s>>>(a); break;
+    case kFieldAC: k_advance<kFieldAC><<<grid, threads, 0, s>>>(a); break;
+    case kFieldB: k_advance<kFieldB><<<grid, threads, 0, s>>>(a); break;
+    case kFieldECR: k_advance<kFieldECR><<<grid, threads, 0, s>>>(a); break;
+    default: k_advance<kFieldACB><<<grid, threads, 0, s>>>(a); break;
   }
-#define LGPU_ADVANCE(K)                                               \
-  switch (a.field.mode) {                                             \
-    case kFieldDC: K<kFieldDC><<<grid, threads, 0, s>>>(a); break;    \
-    case kFieldAC: K<kFieldAC><<<grid, threads, 0, s>>>(a); break;    \
-    case kFieldB: K<kFieldB><<<grid, threads, 0, s>>>(a); break;      \
-    case kFieldECR: K<kFieldECR><<<grid, threads, 0, s>>>(a); break;  \
-    default: K<kFieldACB><<<grid, threads, 0, s>>>(a); break;         \
-  }
-  if (a.queue_only) {
-    LGPU_ADVANCE(k_advance_drain)
-  } else {
-    LGPU_ADVANCE(k_advance)
-  }
-#undef LGPU_ADVANCE
 }
 
 void launch_init(const InitArgs& a, cudaStream_t s) {
@@ -1030,9 +996,10 @@ void launch_hist(const HistArgs& a, cudaStream_t s) {
   if (a.cylindrical && !a.evdf_done) k_hist_b<<<chunks, kHistBThreads, kHistBSmem, s>>>(a);
 }
 
-void launch_pop_control(const PopArgs& a, cudaStream_t s) {
+void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s) {
   PopOne one;
   one.a = a;
+  one.adv = adv;
   launch_pop_phases(one, kPopBlocks, s);
 }
 
@@ -1078,12 +1045,11 @@ int launch_batch_post(const BatchArgs& b, int sm_count, int max_slots, unsigned 
   const int slots = max(1, min(max_slots, kBatchMaxSlots));
   int n = 1;
   if (parts & kPartIonAtt) {
-    k_advance_drain_batch<<<slots, 32, 0, s>>>(b);
     PopBatch pb;
     pb.hdr = b.hdr;
     pb.slots = b.slots;
     launch_pop_phases(pb, sm_count * kPopBlocksPerSM, s);
-    n += 1 + kPopLaunches;
+    n += kPopLaunches;
   }
   if (parts & kPartSample) {
     k_sample_batch<<<sm_count * 2, kSampleBatchThreads, kSampleBatchSmem, s>>>(b);

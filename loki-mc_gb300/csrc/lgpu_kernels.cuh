@@ -21,8 +21,7 @@ struct DevScalars {
   int sec_count, att_count, spill_count, error_flag;
   unsigned int max_energy_bits;
   int work_counter;
-  int pop_counts[3];    // population control: alive secondaries, removed slots, surviving secondaries
-  int pad1;
+  int pop_counts[2];    // population control: removed slots, surviving secondaries
   unsigned long long null_count;
   unsigned long long real_count;
   double field_gain;
@@ -76,13 +75,10 @@ struct AdvanceArgs {
   int* work_counter;               // chunk counter of the persistent grid (zero before the launch)
   int sm_count;
   const IntervalCtl* ctl;          // when set: per-interval values are read from here
-  int queue_only;                  // 1: only drain the spilled secondaries (one warp)
   int real_batch;                  // pending real collisions that start a warp's collision turn (1..32)
   int coarse;                      // 1: null test against the block bounds first (t.nu_coarse)
   int local_q;                     // secondaries a warp queues before it spills (1..kLocalQ)
-  // one condition per launch: the electrons each warp starts on, and the ones it
-  // takes at a time from the work counter after them (set by launch_advance)
-  int share, chunk;
+  int share;                       // one condition per launch: the electrons each warp starts on (set by launch_advance)
 };
 constexpr int kDefaultRealBatch = 20;
 
@@ -188,12 +184,12 @@ struct PopArgs {
   int n_electrons;
   const float4* sec;               // advanced secondaries (x, y, z, s), (vx, vy, vz, dead flag)
   const int* sec_count;            // may exceed sec_cap after an overflow (reported by the host)
+  const int* spill_count;          // secondaries that the warps could not queue
   int sec_cap;
-  int* counts;                     // [3] zero on entry: alive secondaries, removed slots, surviving secondaries
+  int* counts;                     // [2] zero on entry: removed slots, surviving secondaries
   const int* att_list;
   const int* att_count;
   unsigned int* claim;             // bitmap over n_electrons + sec_cap, all zero on entry and on exit
-  int* alive;                      // [sec_cap] scratch: indices of secondaries that did not attach
   int* removed;                    // [sec_cap] scratch
   int* pair_slot;                  // [sec_cap] scratch
   int* pair_sec;                   // [sec_cap] scratch
@@ -203,10 +199,11 @@ struct PopArgs {
   const IntervalCtl* ctl;
   int* error_flag;                 // set when a bounded retry loop gives up
 };
-// Five launches (compaction, filling of attached slots, clones or removal
-// draws, listing, pairing), each spread over many blocks.
-void launch_pop_control(const PopArgs& a, cudaStream_t s);
-constexpr int kPopLaunches = 5;
+// The secondaries the warps could not queue (adv: the advance's arguments), then
+// three launches (filling of attached slots and removal draws, clones or listing,
+// pairing), each spread over many blocks.
+void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s);
+constexpr int kPopLaunches = 3;
 
 // ------------------------------------------------------------------ batches
 // Many swarm conditions (slots) advanced by one launch sequence per interval.
@@ -273,7 +270,7 @@ size_t batch_slots_offset();    // bytes from the staging start to slots[0]
 // One batched interval is three launch groups on one stream:
 //   pre:     slot control blocks and per-interval scalars
 //   advance: one persistent launch per field mode
-//   post:    drain of spilled secondaries, population control, moments, gather
+//   post:    spilled secondaries and population control, moments, gather
 // ahead of them, from a second staging area of the same layout, the
 // distribution passes of the previous interval's samples (`hist` of each
 // slot), launched before the host prepares the interval so that its work
@@ -285,7 +282,7 @@ enum BatchParts : unsigned {
   kPartHistA = 1u << 8,   // a slot records its energy distributions
   kPartHistB = 1u << 9,   // a slot records its velocity distribution in a separate pass
   kPartSample = 1u << 10, // a slot samples its moments
-  kPartIonAtt = 1u << 11, // a slot has ionization or attachment (drain, population control)
+  kPartIonAtt = 1u << 11, // a slot has ionization or attachment (spilled secondaries, population control)
 };
 int launch_batch_pre(const BatchArgs& b, int sm_count, int max_slots, unsigned parts, cudaStream_t s);
 int launch_batch_hist(const BatchArgs& b, int sm_count, unsigned parts, cudaStream_t s);
