@@ -143,8 +143,8 @@ typedef struct lgpu_step_report {
   long long sync_steps;       /* cumulative */
 } lgpu_step_report;
 
-/* Device-time accounting of the main advance kernel (CUDA events on the
- * context's stream). */
+/* Device-time accounting of the main advance kernel (by the device's clock,
+ * from its first block's start to its last one's end). */
 typedef struct lgpu_timing {
   double advance_ms;          /* summed duration of the main advance launches */
   long long advance_launches;

@@ -761,12 +761,21 @@ __device__ __forceinline__ void drain_body(AdvanceArgs& a, Sh& sh) {
   __syncthreads();
 }
 
+// the device's clock in nanoseconds
+__device__ __forceinline__ unsigned long long device_clock() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
 // One condition per launch: every warp starts on its own a.share electrons and takes
 // kOwnChunk at a time after them.
 constexpr int kOwnChunk = 32;
 
 template <int MODE, class Sh>
 __device__ __forceinline__ void advance_body(const AdvanceArgs& a, Sh& sh) {
+  if (!a.ctl->go) return;  // the chain of intervals has stopped
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.advance_begin = device_clock();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int warps = (int)(blockDim.x >> 5);
   const uint32_t warp_tag = (uint32_t)(blockIdx.x * warps + wid);
@@ -783,6 +792,7 @@ __device__ __forceinline__ void advance_body(const AdvanceArgs& a, Sh& sh) {
   uint32_t sec_id = 0;
   warp_loop<MODE, false>(a, sh, iv, tl, sec_id, warp_tag, cur);
   block_flush(a, sh, tl, lane, wid);
+  if (threadIdx.x == 0) atomicMax(a.advance_end, device_clock());
 }
 
 // ------------------------------------------------------------ batched advance

@@ -68,7 +68,6 @@ class Engine {
   std::string err_;
   lgpu_config cfg_;
   cudaStream_t stream_ = nullptr;
-  cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
 
   // ---------------------------------------------------------------- errors
   int fail(int code, const char* fmt, ...) {
@@ -115,12 +114,6 @@ class Engine {
   static T* at(char* base, size_t off) {
     return reinterpret_cast<T*>(base + off);
   }
-
-  // What the host sends before an interval of a context on its own.
-  struct PlainCtl {
-    IntervalCtl ctl;
-    DistCtl dist;
-  };
 
   // The secondary, spill and population-control buffers for `cap` records
   // in one allocation.
@@ -177,8 +170,6 @@ class Engine {
     LGPU_CU(prepare_kernels());
     LGPU_CU(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, cfg_.device));
     LGPU_CU(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    LGPU_CU(cudaEventCreate(&ev0_));
-    LGPU_CU(cudaEventCreate(&ev1_));
     LGPU_CU(cudaEventCreateWithFlags(&tables_ev_, cudaEventDisableTiming));
     N_ = (int)cfg_.n_electrons;
     M_ = cfg_.n_interp;
@@ -206,6 +197,7 @@ class Engine {
     d_sc_ = at<DevScalars>(d_core_, o_sc);
     d_plain_ = at<PlainCtl>(d_core_, o_ctl);
     d_ctl_ = &d_plain_->ctl;
+    LGPU_CU(cudaMemsetAsync(d_plain_, 0, sizeof(PlainCtl), stream_));
     d_nu_pair_ = at<float2>(d_core_, o_nup);
     d_nu_tot_ = at<double>(d_core_, o_nut);
     d_nu_max_ = at<double>(d_core_, o_num);
@@ -222,7 +214,11 @@ class Engine {
     // pinned host: the scalar read-back, the control block, the running maximum
     Carve ch;
     const size_t o_hsc = ch.take<DevScalars>(1), o_hctl = ch.take<PlainCtl>(1), o_hnum = ch.take<double>(M_);
-    LGPU_CU(cudaMallocHost((void**)&h_pinned_, ch.bytes));
+    const size_t o_out = ch.take<ChainOut>(1);
+    // (the device writes the chains' scalars there)
+    LGPU_CU(cudaHostAlloc((void**)&h_pinned_, ch.bytes, cudaHostAllocMapped));
+    h_out_ = at<ChainOut>(h_pinned_, o_out);
+    LGPU_CU(cudaHostGetDevicePointer((void**)&d_out_, h_out_, 0));
     h_sc_ = at<DevScalars>(h_pinned_, o_hsc);
     h_plain_ = at<PlainCtl>(h_pinned_, o_hctl);
     h_ctl_ = &h_plain_->ctl;
@@ -238,7 +234,6 @@ class Engine {
     if (batch_ && stream_) cudaStreamSynchronize(stream_);
     leave_batch();  // the batch's stream is not this context's to destroy
     if (stream_) cudaStreamSynchronize(stream_);
-    drop_graphs();
     void* ptrs[] = {d_core_, d_secbuf_, d_procbuf_, d_rp_in_, d_rp_out_, d_tt_i_, d_tt_d_, d_tt_raw_, d_post_};
     for (void* p : ptrs)
       if (p) cudaFree(p);
@@ -247,11 +242,10 @@ class Engine {
     h_pinned_ = nullptr;
     h_sc_ = nullptr;
     h_plain_ = nullptr;
+    h_out_ = nullptr;
     h_ctl_ = nullptr;
     h_nu_max_ = nullptr;
     if (tables_ev_) cudaEventDestroy(tables_ev_);
-    if (ev0_) cudaEventDestroy(ev0_);
-    if (ev1_) cudaEventDestroy(ev1_);
     if (stream_) cudaStreamDestroy(stream_);
     stream_ = nullptr;
   }
@@ -443,6 +437,7 @@ class Engine {
     else if (std::abs(omega_ - omega_c_) / omega_ < 1E-6) f.mode = kFieldECR;
     else f.mode = kFieldACB;
     field_ = f;
+    chain_nu_ = 0;  // the chains' energy limits follow the field
     return LGPU_OK;
   }
 
@@ -588,11 +583,46 @@ class Engine {
     return fail(LGPU_ERR_OVERFLOW, "trial frequency search did not converge");
   }
 
+  // whether check_max_frequency would leave tables and trial frequency alone
+  bool frequency_holds(double max_energy) const {
+    const double thermal = (cfg_.gas_temperature_effect == 1 || cfg_.gas_temperature_effect == 2) ? 10.0 * gas_energy_ : 0.0;
+    const double maxE = max_accel_energy(max_energy, 10.0 / nu_trial_) + thermal;
+    if (maxE > max_interp_ || 2.5 * maxE < max_interp_) {
+      const double target = 2.0 * maxE < emax_elastic_ ? 2.0 * maxE : emax_elastic_;
+      if (target != max_interp_) return false;
+    }
+    return !(nu_trial_ < h_nu_max_[(int)std::fmin(std::ceil(maxE / step_), M_ - 1)]);
+  }
+
+  // The largest energies [e_lo_, e_hi_] of a sample after which the next interval
+  // starts without a look by the host: the trial frequency and the tables hold
+  // (both ends found by bisection: what is checked grows with the energy) and no
+  // electron left the elastic tables. Kept a little inside, so that the device's
+  // comparison never says yes where the host's check would not.
+  void chain_energies() {
+    if (chain_nu_ == nu_trial_ && chain_interp_ == max_interp_) return;
+    chain_nu_ = nu_trial_;
+    chain_interp_ = max_interp_;
+    auto edge = [&](double in, double out) {
+      if (frequency_holds(out)) return out;
+      for (int k = 0; k < 40; ++k) {
+        const double mid = 0.5 * (in + out);
+        (frequency_holds(mid) ? in : out) = mid;
+      }
+      return in;
+    };
+    e_lo_ = (float)(edge(cur_max_energy_, 0.0) * (1.0 + 1e-6));
+    e_hi_ = (float)(std::fmin(edge(cur_max_energy_, std::fmax(max_interp_, cur_max_energy_)), emax_elastic_) * (1.0 - 1e-6));
+  }
+
   // ------------------------------------------------------------ ensemble
   int init_ensemble() {
     if (!have_procs_ || !have_cond_) return fail(LGPU_ERR_STATE, "set_processes and set_conditions come first");
-    drop_graphs();  // kernel arguments (field, constants, sizes) may have changed
     hist_pending_ = false;
+    scalars_clear_ = false;
+    chain_built_ = false;  // kernel arguments (field, constants, sizes) may have changed
+    chain_nu_ = 0;
+    chain_len_ = 2;
     LGPU_TRY(upload_proc_consts());
     time_ = 0;
     ss_time_ = kNonDef;
@@ -696,6 +726,8 @@ class Engine {
     a.max_energy_bits = &d_sc_->max_energy_bits;
     a.error_flag = &d_sc_->error_flag;
     a.work_counter = &d_sc_->work_counter;
+    a.advance_begin = &d_sc_->advance_begin;
+    a.advance_end = &d_sc_->advance_end;
     a.sm_count = sm_count_;
     a.ctl = d_ctl_;
     a.real_batch = cfg_.advance_real_batch > 0 ? std::min(cfg_.advance_real_batch, 32) : kDefaultRealBatch;
@@ -729,64 +761,32 @@ class Engine {
 
   // The device work of one interval: the advance of every electron and of the
   // secondaries they create, any secondary its warps could not queue and population
-  // control (when the mixture ionizes or attaches), the ensemble sample and the
-  // scalar read-back. Captured once as a CUDA graph.
+  // control (when the mixture ionizes or attaches), the ensemble sample and the end
+  // of the interval (k_sample, or k_interval_end without a sample).
   void enqueue_interval(bool sample) {
-    copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice);
-    cudaMemsetAsync(d_sc_, 0, offsetof(DevScalars, null_count), stream_);
-    AdvanceArgs a = advance_args();
-    cudaEventRecordWithFlags(ev0_, stream_, cudaEventRecordExternal);
-    launch_advance(a, stream_);
-    cudaEventRecordWithFlags(ev1_, stream_, cudaEventRecordExternal);
-    ++launches_;
-    if (have_ion_att_) {
-      launch_pop_control(a, pop_args(), stream_);
-      launches_ += kPopLaunches;
-    }
-    if (sample) enqueue_sample(true);
-    copy(h_sc_, d_sc_, sizeof(DevScalars), cudaMemcpyDeviceToHost);
+    launch_advance(chain_adv_, stream_);
+    if (have_ion_att_) launch_pop_control(chain_adv_, chain_pop_, stream_);
+    if (sample) launch_sample(chain_smp_, sm_count_, stream_);
+    else launch_interval_end(chain_smp_, stream_);
+    launches_ += 2 + (have_ion_att_ ? kPopLaunches : 0);
   }
 
-  // dist: with the distributions the interval's control block asks for
-  void enqueue_sample(bool dist = false) {
-    cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_);
-    cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_);
-    SampleArgs s = sample_args();
-    if (dist) {
-      s.dist = &d_plain_->dist;
-      s.advance_max_bits = &d_sc_->max_energy_bits;
-      s.dist_e_cells = cfg_.n_energy_cells;
-      s.dist_v_cells = cylindrical_ ? cfg_.n_radial_cells * cfg_.n_axial_cells : 0;
-    }
-    launch_sample(s, sm_count_, stream_);
-    ++launches_;
-  }
-
-  int graph_for(bool sample, cudaGraphExec_t* out) {
-    cudaGraphExec_t& ge = graph_[sample ? 1 : 0];
-    if (!ge) {
-      cudaGraph_t g;
-      const long long l0 = launches_;
-      LGPU_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-      enqueue_interval(sample);
-      LGPU_CU(cudaStreamEndCapture(stream_, &g));
-      LGPU_CU(cudaGraphInstantiate(&ge, g, 0));
-      cudaGraphDestroy(g);
-      graph_launches_[sample ? 1 : 0] = launches_ - l0;
-      launches_ = l0;
-      h2d_bytes_ -= sizeof(PlainCtl);
-      d2h_bytes_ -= sizeof(DevScalars);
-    }
-    *out = ge;
+  // the scalars of one interval, zero before its launches
+  int clear_interval_scalars() {
+    LGPU_CU(cudaMemsetAsync(d_sc_, 0, offsetof(DevScalars, null_count), stream_));
+    LGPU_CU(cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_));
+    LGPU_CU(cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_));
     return LGPU_OK;
   }
 
-  void drop_graphs() {
-    for (auto& g : graph_)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
+  // the field's phase rate and its phase at a time, reduced in FP64
+  double phase_rate() const {
+    if (field_.mode == kFieldAC || field_.mode == kFieldACB) return omega_;
+    return field_.mode == kFieldECR ? omega_c_ : 0.0;
+  }
+  double phase_at(double t) const {
+    const double rate = phase_rate();
+    return rate != 0.0 ? std::fmod(rate * t, 2.0 * kPi) : 0.0;
   }
 
   // The first half of a synchronisation interval (BoltzmannMC.C:617-688):
@@ -798,24 +798,17 @@ class Engine {
     LGPU_TRY(check_max_frequency(cur_max_energy_, ready));
     if (ready && !*ready) return LGPU_OK;
     pending_dt_ = cfg_.sync_x / nu_trial_;
-    double phi0 = 0.0, rate = 0.0;
-    if (field_.mode == kFieldAC || field_.mode == kFieldACB) {
-      phi0 = std::fmod(omega_ * time_, 2.0 * kPi);
-      rate = omega_;
-    } else if (field_.mode == kFieldECR) {
-      phi0 = std::fmod(omega_c_ * time_, 2.0 * kPi);
-      rate = omega_c_;
-    }
     IntervalCtl& c = *h_ctl_;
     c.dt_sync = (float)pending_dt_;
-    c.phi0 = (float)phi0;
-    c.phase_rate = (float)rate;
+    c.phi0 = (float)phase_at(time_);
+    c.phase_rate = (float)phase_rate();
     c.nu = (float)nu_trial_;
     c.inv_step = (float)(1.0 / step_);
     c.shift_x = (float)shift_[0];
     c.shift_y = (float)shift_[1];
     c.shift_z = (float)shift_[2];
     c.interval = interval_;
+    c.go = 1;
     // in a batch the sample of this interval counts its EVDF in the moment
     // pass when it will record distributions (grid fixed since the steady state)
     evdf_fused_ = batch_ && sampling_ && ss_time_ != kNonDef && cylindrical_;
@@ -879,7 +872,7 @@ class Engine {
   // leaves every claim bit clear). The new buffers are allocated before the
   // old ones go, so a failed allocation keeps the old capacity (an interval
   // that then overflows fails cleanly). Launch arguments built from the old
-  // pointers (the interval graphs, a batch slot) are rebuilt.
+  // pointers (a chain's, a batch slot's) are rebuilt.
   int grow_secondaries(long long cap) {
     const long long max_cap = std::min<long long>(INT32_MAX / 2, (long long)INT32_MAX - N_ - 32);
     if (sec_cap_ >= max_cap) return LGPU_OK;
@@ -894,32 +887,115 @@ class Engine {
     use_secondaries(q);
     sec_cap_ = new_cap;
     LGPU_CU(cudaMemsetAsync(d_claim_, 0, claim_words_ * sizeof(unsigned int), stream_));
-    drop_graphs();
+    chain_built_ = false;
     slot_built_ = -1;
     ++sec_grown_;
     return LGPU_OK;
   }
 
-  // one synchronisation interval on this context's own stream; when `sample`,
-  // the ensemble moments at its end are in h_sc_ afterwards
-  int step_interval(bool sample) {
+  // How many intervals may follow one another before the host has to look: up to a
+  // steady-state or error check (solve_post), a stop criterion (solve_next) or the
+  // caps on steps and wall time. A chain is short at first and after one that
+  // stopped early, whose launches left were for nothing, and holds the host for a
+  // few milliseconds at most.
+  int chain_limit(int want, bool solving) const {
+    int n = std::min({want, kChain, chain_len_});
+    if (interval_ms_ > 0) n = std::min(n, std::max(1, (int)(5.0 / interval_ms_)));
+    if (!solving) return n;
+    if (cfg_.sync_oversampling != 1) return 1;
+    const bool ss = ss_time_ != kNonDef;
+    // a stop criterion on the count of collisions may hold after any interval
+    if (ss && cfg_.max_coll_after_ss * N_ < 1e18) return 1;
+    if (cfg_.max_sync_steps > 0) n = (int)std::min<long long>(n, std::max<long long>(1, cfg_.max_sync_steps - solve_steps_));
+    double t = time_;
+    for (int i = 1; i < n; ++i) {
+      t += pending_dt_;
+      if (!ss) {
+        if (steady_state_check_at(n_samp_ + i)) return i;
+      } else if (error_check_at(n_int_ + i) || !wants_more(n_int_ + i, t - ss_time_)) {
+        return i;
+      }
+    }
+    return n;
+  }
+
+  // Up to `want` synchronisation intervals on this context's own stream, without
+  // a look by the host in between (PlainCtl), each followed by its part of the
+  // solve loop (solving) or a sample. *ran: the intervals run, at least one.
+  //
+  // A look per interval (graph launch, copies of control block and scalars, wait)
+  // cost 11-17 us of each: 10,000 atomic-gas electrons 53 -> 37 us per interval,
+  // 200,000 under AC 84 -> 66, 1e6 N2-like 135 -> 124.
+  int run_chain(int want, bool solving, int* ran) {
     if (batch_) return fail(LGPU_ERR_STATE, "the context is solved by a batch");
+    const auto t0 = std::chrono::steady_clock::now();
     LGPU_TRY(interval_pre());
-    cudaGraphExec_t ge;
-    LGPU_TRY(graph_for(sample, &ge));
-    LGPU_CU(cudaGraphLaunch(ge, stream_));
-    launches_ += graph_launches_[sample ? 1 : 0];
-    h2d_bytes_ += sizeof(PlainCtl);
-    d2h_bytes_ += sizeof(DevScalars);
+    const bool sample = !solving || sampling_;
+    chain_energies();
+    const int n = sample ? chain_limit(want, solving) : 1;
+    PlainCtl& pl = *h_plain_;
+    pl.n = n;
+    pl.pos = 0;
+    pl.ticket = 0;
+    pl.e_lo = e_lo_;
+    pl.e_hi = e_hi_;
+    pl.sec_stop = sec_cap_ / 4;
+    double t = time_;
+    for (int k = 0; k < n; ++k) {
+      IntervalCtl c = pl.ctl;
+      c.interval = interval_ + k;
+      c.phi0 = (float)phase_at(t);
+      c.shift_x = c.shift_y = c.shift_z = 0.0f;
+      pl.next[k] = c;
+      t += pending_dt_;
+      pl.row[k] = pl.dist.on ? hist_args(t).eedf_periodic_row : nullptr;
+    }
+    LGPU_CU(copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice));
+    if (!scalars_clear_) LGPU_TRY(clear_interval_scalars());
+    h_out_->done = 0;
+    if (!chain_built_) {
+      // fixed from the job's first interval on: conditions set since then are the next job's
+      chain_adv_ = advance_args();
+      chain_pop_ = pop_args();
+      chain_smp_ = sample_args();
+      chain_smp_.plain = d_plain_;
+      chain_smp_.sc = d_sc_;
+      chain_smp_.out = d_out_;
+      chain_smp_.dist_e_cells = cfg_.n_energy_cells;
+      chain_smp_.dist_v_cells = cylindrical_ ? cfg_.n_radial_cells * cfg_.n_axial_cells : 0;
+      chain_built_ = true;
+    }
+    for (int k = 0; k < n; ++k) enqueue_interval(sample);
+    scalars_clear_ = true;
     LGPU_TRY(sync("interval"));
-    {
-      float ms = 0;
-      LGPU_CU(cudaEventElapsedTime(&ms, ev0_, ev1_));
-      adv_ms_ += ms;
+    const int done = *(volatile int*)&h_out_->done;
+    if (done < 1 || done > n) return fail(LGPU_ERR_STATE, "a chain of %d intervals ran %d", n, done);
+    interval_ms_ = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() / done;
+    chain_len_ = done == n ? std::min(2 * std::max(n, chain_len_ / 2), kChain) : 2;
+    for (int k = 0; k < done; ++k) {
+      if (k > 0) {
+        // what the device went on without: the host's own checks agree
+        bool end = false;
+        if (solving) LGPU_TRY(solve_next(&end, true));
+        if (end || !frequency_holds(cur_max_energy_))
+          return fail(LGPU_ERR_STATE, "an interval ran that the host would not have started");
+        LGPU_TRY(interval_pre());
+      }
+      *h_sc_ = h_out_->sc[k];
+      d2h_bytes_ += sizeof(DevScalars);
+      adv_ms_ += 1e-6 * (double)(h_sc_->advance_end - h_sc_->advance_begin);
       ++adv_launches_;
       adv_electron_steps_ += N_;
+      LGPU_TRY(interval_post());
+      if (solving) {
+        LGPU_TRY(solve_post());
+      } else {
+        ++n_samp_;
+        LGPU_TRY(process_sample());
+      }
     }
-    return interval_post();
+    *ran = done;
+    return LGPU_OK;
   }
 
   int check_device_errors() {
@@ -940,9 +1016,12 @@ class Engine {
     return LGPU_OK;
   }
 
-  // ensemble moments at t = 0 (BoltzmannMC.C:306-310), outside the interval graph
+  // ensemble moments at t = 0 (BoltzmannMC.C:306-310), outside the intervals
   int sample_moments() {
-    enqueue_sample();
+    LGPU_CU(cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_));
+    LGPU_CU(cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_));
+    launch_sample(sample_args(), sm_count_, stream_);
+    ++launches_;
     LGPU_TRY(read_scalars());
     return process_sample();
   }
@@ -1245,10 +1324,26 @@ class Engine {
 
   // *done when a stop criterion holds (BoltzmannMC.C:311-316) or a cap is hit;
   // otherwise sampling_ says whether the next interval ends with a sample
-  int solve_next(bool* done) {
+  // (BoltzmannMC.C:311-316) with n_int integration points over int_time
+  bool wants_more(long long n_int, double int_time) const {
+    return (!solve_good_ && cfg_.errors_checked) || n_int < cfg_.req_integration_points ||
+           int_time / ss_time_ < cfg_.req_ss_times || int_time < cfg_.req_abs_time;
+  }
+  // the samples before the steady state and the integration points after which
+  // solve_post looks for it and checks the errors
+  static bool steady_state_check_at(long long n_samp) {
+    const int dec = (int)std::fmax(std::log((double)n_samp) / std::log(2.0) - 11, 6);
+    return n_samp >= 100 && n_samp % (long long)std::pow(2, dec) == 0;
+  }
+  bool error_check_at(long long n_int) const {
+    const int dec = (int)std::fmax(std::log((double)n_int) / std::log(2.0) - 9, 7);
+    return n_int > 200 && n_int % (long long)std::pow(2, dec) == 0 && cfg_.errors_checked;
+  }
+
+  // (within a chain of intervals the caps wait for its end)
+  int solve_next(bool* done, bool within = false) {
     *done = false;
-    if (!((!solve_good_ && cfg_.errors_checked) || n_int_ < cfg_.req_integration_points ||
-          total_int_time_ / ss_time_ < cfg_.req_ss_times || total_int_time_ < cfg_.req_abs_time)) {
+    if (!wants_more(n_int_, total_int_time_)) {
       *done = true;
       return LGPU_OK;
     }
@@ -1260,7 +1355,8 @@ class Engine {
       }
     }
     const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - solve_t0_).count();
-    if ((cfg_.max_seconds > 0 && el > cfg_.max_seconds) || (cfg_.max_sync_steps > 0 && solve_steps_ >= cfg_.max_sync_steps)) {
+    if (!within && ((cfg_.max_seconds > 0 && el > cfg_.max_seconds) ||
+                    (cfg_.max_sync_steps > 0 && solve_steps_ >= cfg_.max_sync_steps))) {
       solve_capped_ = 1;
       *done = true;
       return LGPU_OK;
@@ -1276,20 +1372,15 @@ class Engine {
     if (!sampling_) return LGPU_OK;
     ++n_samp_;
     LGPU_TRY(process_sample());
-    int dec = (int)std::fmax(std::log((double)n_samp_) / std::log(2.0) - 11, 6);
-    const long long between_ss = (long long)std::pow(2, dec);
     if (ss_time_ != kNonDef) {
       ++n_int_;
       total_int_time_ = time_ - ss_time_;
       LGPU_TRY(sample_distributions());
-    } else if (n_samp_ >= 100 && n_samp_ % between_ss == 0) {
+    } else if (steady_state_check_at(n_samp_)) {
       LGPU_TRY(read_counters());
       if ((double)total_real_dev_ > cfg_.min_coll_before_ss * N_) LGPU_TRY(check_steady_state());
     }
-    dec = (int)std::fmax(std::log((double)n_int_) / std::log(2.0) - 9, 7);
-    const long long between_err = (long long)std::pow(2, dec);
-    if (ss_time_ != kNonDef && n_int_ > 200 && n_int_ % between_err == 0 && cfg_.errors_checked)
-      solve_good_ = statistical_errors_ok();
+    if (ss_time_ != kNonDef && error_check_at(n_int_)) solve_good_ = statistical_errors_ok();
     return LGPU_OK;
   }
 
@@ -1313,8 +1404,8 @@ class Engine {
       bool done = false;
       LGPU_TRY(solve_next(&done));
       if (done) break;
-      LGPU_TRY(step_interval(sampling_));
-      LGPU_TRY(solve_post());
+      int ran = 0;
+      LGPU_TRY(run_chain(kChain, true, &ran));
     }
     return solve_end(r);
   }
@@ -1327,6 +1418,7 @@ class Engine {
     own_stream_ = stream_;
     stream_ = s;
     batch_ = true;
+    scalars_clear_ = false;
     hist_pending_ = false;
   }
   void leave_batch() {
@@ -1560,10 +1652,10 @@ class Engine {
   int advance(int n, lgpu_step_report* rep) {
     if (!initialized_) return fail(LGPU_ERR_STATE, "init_ensemble comes first");
     sampling_ = false;  // no distributions: only lgpu_solve tallies them
-    for (int i = 0; i < n; ++i) {
-      LGPU_TRY(step_interval(true));
-      ++n_samp_;
-      LGPU_TRY(process_sample());
+    for (int i = 0; i < n;) {
+      int ran = 0;
+      LGPU_TRY(run_chain(n - i, false, &ran));
+      i += ran;
     }
     if (rep) {
       LGPU_TRY(read_counters());
@@ -1931,8 +2023,15 @@ class Engine {
   PlainCtl *d_plain_ = nullptr, *h_plain_ = nullptr;
   IntervalCtl* d_ctl_ = nullptr;  // the control blocks' interval part
   IntervalCtl* h_ctl_ = nullptr;
-  cudaGraphExec_t graph_[2] = {nullptr, nullptr};
-  long long graph_launches_[2] = {0, 0};
+  ChainOut *d_out_ = nullptr, *h_out_ = nullptr;  // one block, as the device and the host see it
+  // chains of intervals (run_chain)
+  bool scalars_clear_ = false, chain_built_ = false;
+  AdvanceArgs chain_adv_{};
+  PopArgs chain_pop_{};
+  SampleArgs chain_smp_{};
+  int chain_len_ = 2;
+  double interval_ms_ = 0, chain_nu_ = 0, chain_interp_ = 0;
+  float e_lo_ = 0, e_hi_ = 0;
   float2 *d_nu_pair_ = nullptr, *d_cum_pair_ = nullptr, *d_sig_pair_ = nullptr;
   double *d_nu_tot_ = nullptr, *d_nu_max_ = nullptr;
   float* d_nu_coarse_ = nullptr;

@@ -13,6 +13,8 @@
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 
+#include <cstddef>
+
 #include "lgpu_advance.cuh"
 #include "lgpu_device.cuh"
 #include "lgpu_kernels.cuh"
@@ -287,6 +289,48 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
   }
 }
 
+// The end of an interval of one condition (every thread of one block calls this;
+// all other work of the interval is done): its scalars go to the host, the ones of
+// one interval are cleared, and the next interval of the chain is set up or the chain
+// stopped.
+__device__ __forceinline__ void end_interval(const SampleArgs& a, bool sampled) {
+  PlainCtl& pl = *a.plain;
+  const int pos = pl.pos;
+  constexpr int kWords = (int)(sizeof(DevScalars) / sizeof(int));
+  const int* src = reinterpret_cast<const int*>(a.sc);
+  int* dst = reinterpret_cast<int*>(&a.out->sc[pos]);
+  for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = __ldcg(&src[k]);
+  if (threadIdx.x == 0) {
+    const float e = __uint_as_float(__ldcg(&a.sc->sample_max_bits));
+    const bool counted = !pl.dist.on || __uint_as_float(__ldcg(&a.sc->max_energy_bits)) <= pl.dist.e_bound;
+    const bool go = sampled && pos + 1 < pl.n && counted && e >= pl.e_lo && e <= pl.e_hi &&
+                    __ldcg(&a.sc->error_flag) == 0 && __ldcg(&a.sc->sec_count) <= pl.sec_stop;
+    if (go) {
+      IntervalCtl c = pl.next[pos + 1];
+      // the host's arithmetic: the FP64 mean, rounded to FP32
+      const double n = (double)a.n;
+      c.shift_x = (float)(__ldcg(&a.moments[1]) / n);
+      c.shift_y = (float)(__ldcg(&a.moments[2]) / n);
+      c.shift_z = (float)(__ldcg(&a.moments[3]) / n);
+      pl.ctl = c;
+      pl.dist.h.eedf_periodic_row = pl.row[pos + 1];
+      pl.pos = pos + 1;
+    } else {
+      pl.ctl.go = 0;
+    }
+    a.out->done = pos + 1;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < (int)(offsetof(DevScalars, null_count) / sizeof(int)); k += blockDim.x)
+    reinterpret_cast<int*>(a.sc)[k] = 0;
+  if (threadIdx.x < kMoments) a.moments[threadIdx.x] = 0.0;
+  if (threadIdx.x == 0) a.sc->sample_max_bits = 0u;
+}
+
+__global__ void k_interval_end(SampleArgs a) {
+  if (a.plain->ctl.go) end_interval(a, false);
+}
+
 // The sample of one condition: the moments and, when the interval's DistCtl says
 // so, the distributions in the same read: EEDF counts in shared memory (one FP64
 // atomic per occupied cell and block), EADF and (V_SHARED false) EVDF counts
@@ -300,15 +344,9 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
 // moments + EEDF/EADF + EVDF of 1e6 electrons 16 + 49 + 91 -> 35 us, of 4e6
 // 28 + 54 + 93 -> 83 us, of 10,000 5 + 12 + 14.5 -> 7 us.
 template <bool V_SHARED>
-__global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sample(SampleArgs a) {
-  __shared__ double s_m[kSampleThreads / 32][kMoments];
-  extern __shared__ unsigned int sm_dist[];
-  const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-  if (!a.dist || !a.dist->on || !(__uint_as_float(*a.advance_max_bits) <= a.dist->e_bound)) {
-    sample_range(a, first, a.n, step, s_m);
-    return;
-  }
-  const HistArgs h = a.dist->h;
+__device__ __forceinline__ void sample_counting(const SampleArgs& a, int first, int step, double (*s_m)[kMoments],
+                                                unsigned int* sm_dist) {
+  const HistArgs h = a.plain->dist.h;
   const int nE = h.n_e_cells, nV = h.cylindrical ? h.n_rad * h.n_ax : 0, nVw = V_SHARED ? (nV + 1) >> 1 : 0;
   unsigned int* hE = sm_dist;
   unsigned int* hV = sm_dist + nE;
@@ -339,6 +377,30 @@ __global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sampl
     if (k & 0xFFFFu) atomicAdd(&h.evdf[2 * w], (double)(k & 0xFFFFu));
     if (k >> 16) atomicAdd(&h.evdf[2 * w + 1], (double)(k >> 16));
   }
+}
+
+template <bool V_SHARED>
+__global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sample(SampleArgs a) {
+  __shared__ double s_m[kSampleThreads / 32][kMoments];
+  __shared__ bool s_last;
+  extern __shared__ unsigned int sm_dist[];
+  if (a.plain && !a.plain->ctl.go) return;  // the chain of intervals has stopped
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  const bool counts = a.plain && a.plain->dist.on &&
+                      __uint_as_float(a.sc->max_energy_bits) <= a.plain->dist.e_bound;
+  if (counts) sample_counting<V_SHARED>(a, first, step, s_m, sm_dist);
+  else sample_range(a, first, a.n, step, s_m);
+  if (!a.plain) return;
+  // the last block ends the interval
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.plain->ticket, 1u) == gridDim.x - 1;
+    if (s_last) a.plain->ticket = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  if (s_last) end_interval(a, true);
 }
 
 // Below this many electrons a chunk counts EADF and EVDF with global atomics:
@@ -981,13 +1043,15 @@ void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   const int sms = max(1, sm_count), full = sms * (1024 / kSampleThreads);
   const int threads = a.n < full * kSampleThreads / 2 ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
-  const int eedf = a.dist ? a.dist_e_cells * (int)sizeof(unsigned int) : 0;
+  const int eedf = a.plain ? a.dist_e_cells * (int)sizeof(unsigned int) : 0;
   const long long v_words = ((long long)a.dist_v_cells + 1) / 2;
-  const bool v_shared = a.dist && a.n >= kSampleSharedV && eedf + 4 * v_words <= kSampleSmem &&
+  const bool v_shared = a.plain && a.n >= kSampleSharedV && eedf + 4 * v_words <= kSampleSmem &&
                         blocks_for(a.n, grid * threads) * (long long)threads < 65536;
   if (v_shared) k_sample<true><<<grid, threads, eedf + 4 * (int)v_words, s>>>(a);
   else k_sample<false><<<grid, threads, eedf, s>>>(a);
 }
+
+void launch_interval_end(const SampleArgs& a, cudaStream_t s) { k_interval_end<<<1, 128, 0, s>>>(a); }
 
 void launch_hist(const HistArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;

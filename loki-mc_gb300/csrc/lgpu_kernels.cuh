@@ -22,6 +22,9 @@ struct DevScalars {
   unsigned int max_energy_bits;
   int work_counter;
   int pop_counts[2];    // population control: removed slots, surviving secondaries
+  // device clock (ns) of the advance's first block's start and last block's end
+  // (one condition per launch)
+  unsigned long long advance_begin, advance_end;
   unsigned long long null_count;
   unsigned long long real_count;
   double field_gain;
@@ -78,7 +81,10 @@ struct AdvanceArgs {
   int real_batch;                  // pending real collisions that start a warp's collision turn (1..32)
   int coarse;                      // 1: null test against the block bounds first (t.nu_coarse)
   int local_q;                     // secondaries a warp queues before it spills (1..kLocalQ)
-  int share;                       // one condition per launch: the electrons each warp starts on (set by launch_advance)
+  // one condition per launch: the electrons each warp starts on (set by
+  // launch_advance) and the device clock of the launch
+  int share;
+  unsigned long long *advance_begin, *advance_end;
 };
 constexpr int kDefaultRealBatch = 20;
 
@@ -160,18 +166,49 @@ struct DistCtl {
 // k_sample: 21 against 17 us per 1e6 electrons at 2e7).
 constexpr int kDistInSample = 16000000;
 
-// Ensemble sample: moment sums (FP64) and the largest energy, and, with `dist`,
-// the distributions in the same read of the ensemble.
+// A chain of intervals of one condition: the host launches up to kChain of them
+// without a look in between. The last block of each interval's sample keeps the
+// interval's scalars for the host, clears them and writes the next interval's
+// control block (the origin shift is the new ensemble mean), or stops the chain,
+// whose launches left then do nothing, when the host has something to do first:
+// a look at the trial frequency or energy tables (the largest energy left
+// [e_lo, e_hi]), a re-binning, larger buffers, or an error to report.
+constexpr int kChain = 16;
+
+struct PlainCtl {
+  IntervalCtl ctl;            // the interval being run
+  DistCtl dist;
+  int n;                      // intervals of the chain
+  int pos;                    // index of the one being run
+  float e_lo, e_hi;
+  int sec_stop;               // more secondaries than this stop the chain
+  unsigned int ticket;        // blocks of the sample that are done (left zero)
+  IntervalCtl next[kChain];   // the control blocks of the chain, origin shifts left out
+  double* row[kChain];        // their samples' per-phase EEDF rows
+};
+
+// where a chain's scalars go: host memory the device can write
+struct ChainOut {
+  int done;                   // intervals run
+  int pad[3];
+  DevScalars sc[kChain];
+};
+
+// Ensemble sample: moment sums (FP64) and the largest energy, and, with `plain`,
+// the distributions in the same read of the ensemble and the end of the interval.
 struct SampleArgs {
   const float4* state;
   int n;
   float half_me_over_e;
-  double* moments;                 // [kMoments], accumulated (zeroed by the caller)
+  double* moments;                 // [kMoments], accumulated (zero on entry)
   unsigned int* max_energy_bits;
-  const DistCtl* dist;             // null: moments only
-  const unsigned int* advance_max_bits;  // largest energy of the interval's advance (with dist)
-  int dist_e_cells, dist_v_cells;        // EEDF and EVDF cells (with dist)
+  PlainCtl* plain;                 // null: moments only
+  DevScalars* sc;                  // the condition's scalars (with plain)
+  ChainOut* out;
+  int dist_e_cells, dist_v_cells;  // EEDF and EVDF cells (with plain)
 };
+// the end of an interval without a sample
+void launch_interval_end(const SampleArgs& a, cudaStream_t s);
 // grid: at most four blocks per SM (sm_count = the device's multiprocessors)
 void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s);
 

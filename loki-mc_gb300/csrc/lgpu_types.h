@@ -92,6 +92,8 @@ struct IntervalCtl {
   float inv_step;         // 1 / table energy step (1/eV)
   float shift_x, shift_y, shift_z;  // origin shift subtracted from every position on load
   unsigned long long interval;      // interval index (random-number counter)
+  int go;                 // 0: the chain of intervals has stopped (one condition per launch)
+  int pad;
 };
 
 // Per-block tallies written by the advance kernels (reduced on the device).
