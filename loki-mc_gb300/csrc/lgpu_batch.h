@@ -381,8 +381,8 @@ class Batch {
   // this interval) sits the interval out and goes on at the next step.
   int step(std::vector<int>* finished = nullptr) {
     const auto h0 = std::chrono::steady_clock::now();
-    // the previous samples' distribution passes first: the host work below
-    // (stop criteria, trial frequencies, staging) runs while they do
+    // the samples left to count first: the host work below (stop criteria, trial
+    // frequencies, staging) runs while they are counted
     if (int rc = launch_pending_hists()) return rc;
     std::vector<int> go, wait;
     go.reserve(active_.size());
@@ -450,8 +450,14 @@ class Batch {
     const int shape = tune_stage_ == 0 ? turn(kAdvShapes) : shape_;
     const int k1 = tune_stage_ == 1 ? turn(stage1_count()) : 0;
     const int cand = tune_stage_ == 0 ? kTuneDefault : (tune_stage_ == 1 ? stage1_cand(k1) : tuned_);
+    double sampled = 0;
+    for (int s = 0; s < n; ++s) {
+      const Engine* e = member(go[s]).e;
+      if (e->sampling_) sampled += e->n_electrons();
+    }
     for (int s = 0; s < n; ++s) {
       Engine* e = member(go[s]).e;
+      if (sampled < kBatchDistMin) e->sample_moments_only();
       e->fill_slot(&sl[s]);
       if (e->cfg_.advance_real_batch == 0) {
         sl[s].adv.real_batch = tune_threshold(cand);
@@ -467,8 +473,12 @@ class Batch {
       take_[s] = (sl[s].flags & kSlotSample) ? 1 : 0;
     }
     ap[n] = na;
-    const auto smp = layout_pass(n, n_.data(), take_.data(), kBatchSampleChunk, sp, spart, rem_);
+    // one chunk per block of the samples (one per SM) while the electrons last; more
+    // and smaller ones cost more in clearing and adding up than they even out
+    const int chunk = even_chunk(sampled, sm_count_, kBatchSampleChunk, 1024);
+    const auto smp = layout_pass(n, n_.data(), take_.data(), chunk, sp, spart, rem_);
     std::memset(hdr, 0, sizeof(BatchHeader));
+    hdr->smp_chunk = chunk;
     hdr->n_slots = n;
     hdr->adv_chunks = na;
     hdr->smp_full = smp.first;
@@ -552,10 +562,17 @@ class Batch {
     return LGPU_OK;
   }
 
-  // The deferred distribution tallies of the running members' last samples
-  // (EEDF, EADF and, before the velocity grid is fixed, EVDF), staged in the
-  // second staging area and launched as their own graph on the batch stream,
-  // ahead of the interval that would otherwise advance the ensemble first.
+  // The electrons of a chunk, at most `most`, with which `electrons` make equally
+  // many chunks for each of `blocks`.
+  static int even_chunk(double electrons, int blocks, int most, int least) {
+    const double rounds = std::max(1.0, std::ceil(electrons / ((double)blocks * most)));
+    return std::min(most, std::max(least, (int)std::ceil(electrons / (blocks * rounds))));
+  }
+
+  // The deferred distribution tallies of the running members' last samples (of a
+  // small batch, and samples that had to be re-binned first), staged in the second staging area and launched as their own graph on
+  // the batch stream, ahead of the interval that would otherwise advance the
+  // ensemble first.
   int launch_pending_hists() {
     auto* hdr = reinterpret_cast<BatchHeader*>(h_hstage_);
     int* hp = reinterpret_cast<int*>(h_hstage_ + batch_prefix_offset()) + 2 * (kBatchMaxSlots + 1);
@@ -564,6 +581,7 @@ class Batch {
     int* vpart = hpart + kBatchMaxSlots;
     auto* sl = reinterpret_cast<BatchSlot*>(h_hstage_ + batch_slots_offset());
     int n = 0;
+    double electrons = 0;
     n_.clear();
     take_.clear();
     for (int idx : active_) {
@@ -571,13 +589,17 @@ class Batch {
       if (!member(idx).e->take_pending_hist(&h)) continue;
       sl[n++].hist = h;
       n_.push_back(h.n);
-      take_.push_back(h.cylindrical && !h.evdf_done ? 1 : 0);  // pass B: the EVDF not counted yet
+      take_.push_back(h.cylindrical ? 1 : 0);  // pass B
+      electrons += h.n;
     }
     if (n == 0) return LGPU_OK;
     all_.assign(n, 1);
-    const auto pa = layout_pass(n, n_.data(), all_.data(), kBatchHistChunk, hp, hpart, rem_);
-    const auto pb = layout_pass(n, n_.data(), take_.data(), kBatchHistChunk, vp, vpart, rem_);
+    const int chunk = electrons < kBatchDistMin ? kBatchHistChunk
+                                                : even_chunk(electrons, sm_count_, kBatchHistChunk, 4096);
+    const auto pa = layout_pass(n, n_.data(), all_.data(), chunk, hp, hpart, rem_);
+    const auto pb = layout_pass(n, n_.data(), take_.data(), chunk, vp, vpart, rem_);
     std::memset(hdr, 0, sizeof(BatchHeader));
+    hdr->hist_chunk = chunk;
     hdr->n_slots = n;
     hdr->hist_full = pa.first;
     hdr->hist2_full = pb.first;

@@ -809,12 +809,9 @@ class Engine {
     c.shift_z = (float)shift_[2];
     c.interval = interval_;
     c.go = 1;
-    // in a batch the sample of this interval counts its EVDF in the moment
-    // pass when it will record distributions (grid fixed since the steady state)
-    evdf_fused_ = batch_ && sampling_ && ss_time_ != kNonDef && cylindrical_;
-    // alone, the sample counts all of them in one read while the energy grid holds
+    // the sample counts its distributions with the moments while the energy grid holds
     DistCtl& d = h_plain_->dist;
-    d.on = !batch_ && sampling_ && ss_time_ != kNonDef && N_ <= kDistInSample;
+    d.on = sampling_ && ss_time_ != kNonDef && (batch_ || N_ <= kDistInSample);
     if (d.on) {
       d.h = hist_args(time_ + pending_dt_);
       d.e_bound = (float)max_eedf_;
@@ -829,6 +826,8 @@ class Engine {
     std::memcpy(&adv_max, &h_sc_->max_energy_bits, 4);
     return h_plain_->dist.on && adv_max <= h_plain_->dist.e_bound;
   }
+  // a batch that leaves the distributions to passes of their own (after interval_pre)
+  void sample_moments_only() { h_plain_->dist.on = 0; }
 
   // The second half, once the interval's device work is done and its scalars
   // are in h_sc_.
@@ -962,7 +961,6 @@ class Engine {
       chain_smp_.sc = d_sc_;
       chain_smp_.out = d_out_;
       chain_smp_.dist_e_cells = cfg_.n_energy_cells;
-      chain_smp_.dist_v_cells = cylindrical_ ? cfg_.n_radial_cells * cfg_.n_axial_cells : 0;
       chain_built_ = true;
     }
     for (int k = 0; k < n; ++k) enqueue_interval(sample);
@@ -1170,9 +1168,7 @@ class Engine {
   int sample_distributions() {
     if (sample_counted()) return LGPU_OK;
     if (max_elec_energy_ > max_eedf_) LGPU_TRY(rebin_distributions());
-    HistArgs h = hist_args(time_);
-    h.evdf_done = evdf_fused_ ? 1 : 0;
-    evdf_fused_ = false;
+    const HistArgs h = hist_args(time_);
     if (batch_) {
       pending_hist_ = h;
       hist_pending_ = true;
@@ -1412,8 +1408,9 @@ class Engine {
 
   // ---------------------------------------------------------- batch mode
   // While a batch solves this context, its work goes on the batch's stream
-  // and the distribution tallies of a sample run inside the batch's next
-  // launch sequence (before that interval's advance, as they would here).
+  // and the distribution tallies of a sample that had to be re-binned first run
+  // inside the batch's next launch sequence (before that interval's advance, as
+  // they would here).
   void enter_batch(cudaStream_t s) {
     own_stream_ = stream_;
     stream_ = s;
@@ -1459,17 +1456,7 @@ class Engine {
     std::memcpy(sl, &slot_, sizeof(*sl));
     sl->ctl = *h_ctl_;
     sl->flags = (have_ion_att_ ? kSlotIonAtt : 0) | (sampling_ ? kSlotSample : 0);
-    if (evdf_fused_) {
-      sl->flags |= kSlotEvdf;
-      HistArgs& v = sl->vhist;
-      v.n_rad = cfg_.n_radial_cells;
-      v.n_ax = cfg_.n_axial_cells;
-      v.inv_rad_step = (float)(1.0 / rad_step_);
-      v.inv_ax_step = (float)(1.0 / ax_step_);
-      v.max_speed = (float)max_speed_;
-      v.evdf = d_evdf_;
-      v.cylindrical = 1;
-    }
+    sl->dist = h_plain_->dist;
   }
   // the deferred tallies of the last sample, handed to the batch's
   // distribution passes (false when there are none)
@@ -2001,7 +1988,7 @@ class Engine {
   long long solve_steps_ = 0;
   double pending_dt_ = 0;
   // batch mode
-  bool batch_ = false, hist_pending_ = false, evdf_fused_ = false;
+  bool batch_ = false, hist_pending_ = false;
   BatchSlot slot_{};                            // cached argument blocks of this solve's batch slot
   long long solve_serial_ = 0, slot_built_ = -1;
   int sec_grown_ = 0;  // times the secondary buffers grew

@@ -189,8 +189,14 @@ __global__ void k_coarse_max(const float2* nu_pair, int M, int shift, float* coa
 }
 
 // ---------------------------------------------------------------- sample
-constexpr int kSampleThreads = 512;
-constexpr int kSampleSmem = 100 * 1024;  // EEDF and EVDF counts, two blocks per SM
+constexpr int kSampleThreads = 512;        // blocks that count without shared EADF and EVDF cells
+constexpr int kSampleSharedThreads = 1024;  // and with them: one block per SM
+// Their shared memory: EEDF (1000 cells), the slower rows of the EVDF and the lower
+// rows of the EADF. No more than this: the loads in flight live in what is left for
+// L1 (the EADF pass this replaces took 193 us per sweep interval with 224 KB of
+// counts and 160 with 195).
+constexpr int kSampleSmem = 124 * 1024;
+constexpr int kSampleSmemV = 56 * 1024;    // of it, at most, the EVDF's
 
 // Moment sums of electrons begin, begin+step, ... < end into a.moments: per
 // thread in FP32 (a handful of electrons each), FP64 from the warp reduction on.
@@ -266,10 +272,15 @@ __device__ __forceinline__ void sample_range(const SampleArgs& a, int begin, int
 constexpr int kHistChunk = kBatchHistChunk;  // below 2^16: 16-bit counts cannot carry
 constexpr int kHistAThreads = 1024;
 constexpr int kHistBThreads = 512;
-constexpr int kHistASmem = 224 * 1024;  // one block per SM
+constexpr int kHistASmem = 195 * 1024;  // one block per SM
 constexpr int kHistBSmem = 96 * 1024;   // two blocks per SM
 
 __device__ __forceinline__ float radial_speed(float v2xy) { return v2xy > 0.0f ? v2xy * rsqrtf(v2xy) : 0.0f; }
+
+__device__ __forceinline__ void velocity_cell(const HistArgs& a, float4 B, int& rx, int& ry) {
+  rx = (int)(radial_speed(__fmaf_rn(B.y, B.y, __fmul_rn(B.x, B.x))) * a.inv_rad_step);
+  ry = (int)((B.z + a.max_speed) * a.inv_ax_step);
+}
 
 __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, int& cy, int& rx, int& ry) {
   // MathFunctions.C:61-81 (energy) and 106-127 (energy x cos, radial x axial velocity)
@@ -284,8 +295,7 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
     // of any cell (a zero speed has no angle and stays outside the cos cells)
     const float cosang = v2 > 0.0f ? B.z * rsqrtf(v2) : 2.0f;
     cy = (int)((cosang + 1.0f) * (0.5f * (float)a.n_cos));
-    rx = (int)(radial_speed(v2xy) * a.inv_rad_step);
-    ry = (int)((B.z + a.max_speed) * a.inv_ax_step);
+    velocity_cell(a, B, rx, ry);
   }
 }
 
@@ -331,64 +341,98 @@ __global__ void k_interval_end(SampleArgs a) {
   if (a.plain->ctl.go) end_interval(a, false);
 }
 
-// The sample of one condition: the moments and, when the interval's DistCtl says
-// so, the distributions in the same read: EEDF counts in shared memory (one FP64
-// atomic per occupied cell and block), EADF and (V_SHARED false) EVDF counts
-// straight to the FP64 tallies, whose cells are too many for the electrons of a
-// block to share. V_SHARED counts the EVDF in shared memory (16-bit, two per
-// word: a block sees fewer than 2^16 electrons).
+// The cells a block counts in shared memory (16-bit, two per word: a block sees fewer
+// than 2^16 electrons before it adds them up): the EADF's energy rows and the EVDF's
+// radial rows from zero up, as many as fit. The grids reach beyond the fastest
+// electron by a fifth, so that the rows left out hold the last per mille of the
+// electrons; those are added to the FP64 tallies one by one.
+struct SharedCells {
+  int a_rows, v_rows;
+};
+__host__ __device__ __forceinline__ SharedCells shared_cells(int n_e, int n_cos, int n_rad, int n_ax) {
+  SharedCells c;
+  c.v_rows = min(n_rad, kSampleSmemV / 2 / max(n_ax, 1));
+  const long long left = kSampleSmem - 4ll * n_e - 4 * (((long long)c.v_rows * n_ax + 1) / 2) - 8;
+  c.a_rows = (int)min((long long)n_e, max(left, 0ll) / 2 / max(n_cos, 1));
+  return c;
+}
+
+// Moments and distributions of electrons first, first + step, ... < end in one
+// read: EEDF counts in shared memory (one FP64 addition per occupied cell and
+// block), EADF and EVDF counts there too (shared) or straight to the FP64 tallies,
+// where few electrons of a block share a cell. Every thread of the block calls this.
 //
-// Bound by the FP64 additions at L2 (about 1.1e11/s measured, faster than 32-bit
-// ones to the same cells). Separate passes over the electrons in 65535-electron
-// chunks, which this replaces up to kDistInSample electrons, left most SMs idle:
-// moments + EEDF/EADF + EVDF of 1e6 electrons 16 + 49 + 91 -> 35 us, of 4e6
-// 28 + 54 + 93 -> 83 us, of 10,000 5 + 12 + 14.5 -> 7 us.
-template <bool V_SHARED>
-__device__ __forceinline__ void sample_counting(const SampleArgs& a, int first, int step, double (*s_m)[kMoments],
-                                                unsigned int* sm_dist) {
-  const HistArgs h = a.plain->dist.h;
-  const int nE = h.n_e_cells, nV = h.cylindrical ? h.n_rad * h.n_ax : 0, nVw = V_SHARED ? (nV + 1) >> 1 : 0;
+// Straight counts are bound by the FP64 additions at L2 (1.1e11/s at best, faster than
+// 32-bit ones to the same cells, and about 7e10/s on the swarms' own cells), shared
+// ones by the read of the ensemble.
+__device__ __forceinline__ void sample_counting(const SampleArgs& a, const HistArgs& h, bool shared, int first,
+                                                int end, int step, double (*s_m)[kMoments], unsigned int* sm_dist) {
+  const int nE = h.n_e_cells;
+  const SharedCells sc = shared && h.cylindrical ? shared_cells(nE, h.n_cos, h.n_rad, h.n_ax) : SharedCells{0, 0};
+  const int nA = sc.a_rows * h.n_cos, nV = sc.v_rows * h.n_ax, nAw = (nA + 1) >> 1, nVw = (nV + 1) >> 1;
   unsigned int* hE = sm_dist;
-  unsigned int* hV = sm_dist + nE;
-  for (int c = threadIdx.x; c < nE + nVw; c += blockDim.x) sm_dist[c] = 0u;
+  unsigned int* hA = hE + nE;
+  unsigned int* hV = hA + nAw;
+  for (int c = threadIdx.x; c < nE + nAw + nVw; c += blockDim.x) sm_dist[c] = 0u;
   __syncthreads();
+  // (an EEDF cell whose EADF row is shared is that row's sum and what is counted
+  // apart: electrons outside the cos cells, cos rounding to 1 or zero speed)
   auto count = [&](float4 B) {
     int c, cy, rx, ry;
     hist_cells(h, B, c, cy, rx, ry);
     if (c >= 0 && c < nE) {
-      atomicAdd(&hE[c], 1u);
-      if (cy >= 0 && cy < h.n_cos) atomicAdd(&h.eadf[c * h.n_cos + cy], 1.0);
+      const bool angle = cy >= 0 && cy < h.n_cos;
+      const int idx = c * h.n_cos + cy;
+      if (angle && idx < nA) {
+        atomicAdd(&hA[idx >> 1], 1u << ((idx & 1) << 4));
+      } else {
+        atomicAdd(&hE[c], 1u);
+        if (angle) atomicAdd(&h.eadf[idx], 1.0);
+      }
     }
     if (rx >= 0 && rx < h.n_rad && ry >= 0 && ry < h.n_ax) {
       const int idx = rx * h.n_ax + ry;
-      if (V_SHARED) atomicAdd(&hV[idx >> 1], 1u << ((idx & 1) << 4));
+      if (idx < nV) atomicAdd(&hV[idx >> 1], 1u << ((idx & 1) << 4));
       else atomicAdd(&h.evdf[idx], 1.0);
     }
   };
-  sample_range(a, first, a.n, step, s_m, count);  // ends behind a block barrier
+  sample_range(a, first, end, step, s_m, count);  // ends behind a block barrier
   for (int c = threadIdx.x; c < nE; c += blockDim.x) {
-    const unsigned int k = hE[c];
+    unsigned int k = hE[c];
+    if (c < sc.a_rows)
+      for (int q = 0; q < h.n_cos; ++q) {
+        const int idx = c * h.n_cos + q;
+        k += (hA[idx >> 1] >> ((idx & 1) << 4)) & 0xFFFFu;
+      }
     if (!k) continue;
     atomicAdd(&h.eedf[c], (double)k);
     if (h.eedf_periodic_row) atomicAdd(&h.eedf_periodic_row[c], (double)k);
   }
-  for (int w = threadIdx.x; w < nVw; w += blockDim.x) {
-    const unsigned int k = hV[w];
-    if (k & 0xFFFFu) atomicAdd(&h.evdf[2 * w], (double)(k & 0xFFFFu));
-    if (k >> 16) atomicAdd(&h.evdf[2 * w + 1], (double)(k >> 16));
+  for (int w = threadIdx.x; w < nAw + nVw; w += blockDim.x) {
+    const unsigned int k = hA[w];
+    if (!k) continue;
+    double* cell = w < nAw ? h.eadf + 2 * w : h.evdf + 2 * (w - nAw);
+    if (k & 0xFFFFu) atomicAdd(&cell[0], (double)(k & 0xFFFFu));
+    if (k >> 16) atomicAdd(&cell[1], (double)(k >> 16));
   }
 }
 
-template <bool V_SHARED>
-__global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sample(SampleArgs a) {
-  __shared__ double s_m[kSampleThreads / 32][kMoments];
+// The sample of one condition: the moments and, when the interval's DistCtl says
+// so, the distributions. Separate passes over the electrons in 65535-electron chunks,
+// which this replaces up to kDistInSample electrons, left most SMs idle: moments +
+// EEDF/EADF + EVDF of 1e6 electrons 16 + 49 + 91 -> 35 us, of 4e6 28 + 54 + 93 -> 65,
+// of 10,000 5 + 12 + 14.5 -> 7.
+template <bool SHARED>
+__global__ void __launch_bounds__(SHARED ? kSampleSharedThreads : kSampleThreads, SHARED ? 1 : 2)
+    k_sample(SampleArgs a) {
+  __shared__ double s_m[(SHARED ? kSampleSharedThreads : kSampleThreads) / 32][kMoments];
   __shared__ bool s_last;
   extern __shared__ unsigned int sm_dist[];
   if (a.plain && !a.plain->ctl.go) return;  // the chain of intervals has stopped
   const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   const bool counts = a.plain && a.plain->dist.on &&
                       __uint_as_float(a.sc->max_energy_bits) <= a.plain->dist.e_bound;
-  if (counts) sample_counting<V_SHARED>(a, first, step, s_m, sm_dist);
+  if (counts) sample_counting(a, a.plain->dist.h, SHARED, first, a.n, step, s_m, sm_dist);
   else sample_range(a, first, a.n, step, s_m);
   if (!a.plain) return;
   // the last block ends the interval
@@ -407,27 +451,30 @@ __global__ void __launch_bounds__(kSampleThreads, 1024 / kSampleThreads) k_sampl
 // clearing and scanning the whole shared-memory grid would cost more.
 constexpr int kHistSharedMin = 16384;
 
-// pass A over electrons [first, last) of one condition
+// pass A over electrons [first, last) of one condition. Shared memory holds the
+// EEDF counts and as many of the EADF's rows as fit (SHARED rows), the rest, at the
+// top of the energy grid where hardly an electron is, goes to global atomics.
 __device__ __forceinline__ void hist_chunk_a(const HistArgs& a, int first, int last, unsigned int* sm, int sm_words) {
   const int nE = a.n_e_cells;
   const int nA = a.cylindrical ? nE * a.n_cos : 0;
-  const int nAw = (nA + 1) >> 1;
-  const bool a_shared = a.cylindrical && last - first >= kHistSharedMin && nE + nAw <= sm_words;
+  const bool a_shared = a.cylindrical && last - first >= kHistSharedMin && nE < sm_words;
+  // cells of whole energy rows in shared memory
+  const int nS = a_shared ? min(nE, (int)(2ll * (sm_words - nE) / a.n_cos)) * a.n_cos : 0;
+  const int nSw = (nS + 1) >> 1;
   unsigned int* hE = sm;
   unsigned int* hA = sm + nE;
-  const int zero_words = nE + (a_shared ? nAw : 0);
-  for (int w = threadIdx.x; w < zero_words; w += blockDim.x) sm[w] = 0u;
+  for (int w = threadIdx.x; w < nE + nSw; w += blockDim.x) sm[w] = 0u;
   __syncthreads();
-  // With the EADF in shared memory the EEDF count of a cell is its EADF row
-  // sum, so only electrons outside the cos cells (cos rounding to 1, zero
-  // speed) are counted into hE: one shared-memory atomic per electron.
+  // An EEDF count of a cell whose EADF row is in shared memory is that row's sum,
+  // so only electrons outside the cos cells (cos rounding to 1, zero speed) and
+  // the rows left out are counted into hE: one shared-memory atomic per electron.
   auto bin = [&](float4 B) {
     int c, cy, rx, ry;
     hist_cells(a, B, c, cy, rx, ry);
     if (c >= 0 && c < nE) {
       if (a.cylindrical && cy < a.n_cos && cy >= 0) {
         const int idx = c * a.n_cos + cy;
-        if (a_shared) {
+        if (idx < nS) {
           atomicAdd(&hA[idx >> 1], 1u << ((idx & 1) << 4));
         } else {
           atomicAdd(&hE[c], 1u);
@@ -462,7 +509,7 @@ __device__ __forceinline__ void hist_chunk_a(const HistArgs& a, int first, int l
   __syncthreads();
   for (int c = threadIdx.x; c < nE; c += blockDim.x) {
     unsigned int h = hE[c];
-    if (a_shared) {
+    if (c * a.n_cos < nS) {
       for (int k = 0; k < a.n_cos; ++k) {
         const int idx = c * a.n_cos + k;
         h += (hA[idx >> 1] >> ((idx & 1) << 4)) & 0xFFFFu;
@@ -473,12 +520,10 @@ __device__ __forceinline__ void hist_chunk_a(const HistArgs& a, int first, int l
       if (a.eedf_periodic_row) atomicAdd(&a.eedf_periodic_row[c], (double)h);
     }
   }
-  if (a_shared) {
-    for (int w = threadIdx.x; w < nAw; w += blockDim.x) {
-      const unsigned int h = hA[w];
-      if (h & 0xFFFFu) atomicAdd(&a.eadf[2 * w], (double)(h & 0xFFFFu));
-      if ((h >> 16) && 2 * w + 1 < nA) atomicAdd(&a.eadf[2 * w + 1], (double)(h >> 16));
-    }
+  for (int w = threadIdx.x; w < nSw; w += blockDim.x) {
+    const unsigned int h = hA[w];
+    if (h & 0xFFFFu) atomicAdd(&a.eadf[2 * w], (double)(h & 0xFFFFu));
+    if ((h >> 16) && 2 * w + 1 < nA) atomicAdd(&a.eadf[2 * w + 1], (double)(h >> 16));
   }
   __syncthreads();
 }
@@ -843,9 +888,9 @@ __global__ void __launch_bounds__(kHistAThreads) k_hist_a_batch(BatchArgs b) {
   for (int r = 0; r * (int)gridDim.x < total; ++r) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
-    const ChunkRef k = pass_chunk(b.hist_prefix, b.hist_part, n_slots, n_full, kHistChunk, c);
+    const ChunkRef k = pass_chunk(b.hist_prefix, b.hist_part, n_slots, n_full, b.hdr->hist_chunk, c);
     const HistArgs& a = b.slots[k.slot].hist;
-    hist_chunk_a(a, k.first, min(k.first + kHistChunk, a.n), sm_hist, kHistASmem / 4);
+    hist_chunk_a(a, k.first, min(k.first + b.hdr->hist_chunk, a.n), sm_hist, kHistASmem / 4);
   }
 }
 
@@ -855,63 +900,42 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b_batch(BatchArgs b) {
   for (int r = 0; r * (int)gridDim.x < total; ++r) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
-    const ChunkRef k = pass_chunk(b.hist2_prefix, b.hist2_part, n_slots, n_full, kHistChunk, c);
+    const ChunkRef k = pass_chunk(b.hist2_prefix, b.hist2_part, n_slots, n_full, b.hdr->hist_chunk, c);
     const HistArgs& a = b.slots[k.slot].hist;
-    hist_chunk_b(a, k.first, min(k.first + kHistChunk, a.n), sm_hist, kHistBSmem / 4);
+    hist_chunk_b(a, k.first, min(k.first + b.hdr->hist_chunk, a.n), sm_hist, kHistBSmem / 4);
   }
 }
 
-// Ensemble moments of the sampling slots; for the slots whose sample records
-// distributions (kSlotEvdf) the same pass counts the EVDF (BoltzmannMC.C:
-// 1550-1571; 16-bit counts in shared memory per chunk, global atomics for
-// small chunks), saving its separate pass over the velocities.
-constexpr int kSampleBatchThreads = 512;
-constexpr int kSampleBatchSmem = 80 * 1024;  // EVDF counts, two blocks per SM
+// Moments of the sampling slots and, in the same read, the distributions of the
+// slots whose sample records them on a grid that holds (DistCtl), in chunks of
+// hdr->smp_chunk electrons.
+//
+// The 64-point sweep: moments with the EVDF, then EEDF and EADF in a pass of their
+// own, took 123 + 195 us per interval; all of it takes 178 here (3.6 TB/s), about
+// half of it the counts (issue, shared additions) and a third the addition of every
+// chunk's occupied cells to the tallies at L2. 32 conditions of 10,000-30,000
+// electrons: 21 + 66 -> 34 us. Loads in flight are not what it waits for: a ring of
+// asynchronous copies in place of the four records in registers took 193.
+constexpr int kSampleBatchShared = 8192;  // electrons of a chunk that are worth shared cells (16 jobs: 62 us with 4096, 53)
 
-__global__ void __launch_bounds__(kSampleBatchThreads, 2) k_sample_batch(BatchArgs b) {
-  __shared__ double s_m[kSampleBatchThreads / 32][kMoments];
-  extern __shared__ unsigned int sm_evdf[];
-  const int n_slots = b.hdr->n_slots, total = b.hdr->smp_chunks, n_full = b.hdr->smp_full;
+__global__ void __launch_bounds__(kSampleSharedThreads) k_sample_batch(BatchArgs b) {
+  __shared__ double s_m[kSampleSharedThreads / 32][kMoments];
+  extern __shared__ unsigned int sm_dist[];
+  const int n_slots = b.hdr->n_slots, total = b.hdr->smp_chunks, n_full = b.hdr->smp_full, chunk = b.hdr->smp_chunk;
   for (int r = 0; r * (int)gridDim.x < total; ++r) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
-    const ChunkRef k = pass_chunk(b.smp_prefix, b.smp_part, n_slots, n_full, kBatchSampleChunk, c);
+    const ChunkRef k = pass_chunk(b.smp_prefix, b.smp_part, n_slots, n_full, chunk, c);
     const BatchSlot& sl = b.slots[k.slot];
     const SampleArgs& a = sl.smp;
-    const int first = k.first;
-    const int last = min(first + kBatchSampleChunk, a.n);
-    const bool evdf = (sl.flags & kSlotEvdf) != 0;
-    const HistArgs& h = sl.vhist;
-    const int nV = evdf ? h.n_rad * h.n_ax : 0;
-    const int nVw = (nV + 1) >> 1;
-    const bool v_shared = evdf && last - first >= kHistSharedMin && nVw <= kSampleBatchSmem / 4;
-    if (v_shared)
-      for (int w = threadIdx.x; w < nVw; w += blockDim.x) sm_evdf[w] = 0u;
-    __syncthreads();
-    if (evdf) {
-      auto bin = [&](float4 B) {
-        const float v2xy = __fmaf_rn(B.y, B.y, __fmul_rn(B.x, B.x));
-        const int rx = (int)(radial_speed(v2xy) * h.inv_rad_step);
-        const int ry = (int)((B.z + h.max_speed) * h.inv_ax_step);
-        if (rx < h.n_rad && rx >= 0 && ry < h.n_ax && ry >= 0) {
-          const int idx = rx * h.n_ax + ry;
-          if (v_shared) atomicAdd(&sm_evdf[idx >> 1], 1u << ((idx & 1) << 4));
-          else atomicAdd(&h.evdf[idx], 1.0);
-        }
-      };
-      sample_range(a, first + threadIdx.x, last, blockDim.x, s_m, bin);
+    const int last = min(k.first + chunk, a.n);
+    if (sl.dist.on && __uint_as_float(sl.sc->max_energy_bits) <= sl.dist.e_bound) {
+      const bool shared = last - k.first >= kSampleBatchShared;
+      sample_counting(a, sl.dist.h, shared, k.first + threadIdx.x, last, blockDim.x, s_m, sm_dist);
     } else {
-      sample_range(a, first + threadIdx.x, last, blockDim.x, s_m);
+      sample_range(a, k.first + threadIdx.x, last, blockDim.x, s_m);
     }
     __syncthreads();
-    if (v_shared) {
-      for (int w = threadIdx.x; w < nVw; w += blockDim.x) {
-        const unsigned int v = sm_evdf[w];
-        if (v & 0xFFFFu) atomicAdd(&h.evdf[2 * w], (double)(v & 0xFFFFu));
-        if ((v >> 16) && 2 * w + 1 < nV) atomicAdd(&h.evdf[2 * w + 1], (double)(v >> 16));
-      }
-      __syncthreads();
-    }
   }
 }
 
@@ -1034,21 +1058,22 @@ void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
 // not fill the device with full ones (they clear and add up their EEDF counts
 // side by side; 10,000 electrons with distributions 9.1 -> 7.1 us), full ones
 // from there (fewer EEDF additions per electron: 200,000 electrons under AC
-// 21.9 -> 15.9 us). EVDF counts go to shared memory from 1e6 electrons on: 4e6
-// electrons 112 -> 83 us, 1e6 37 -> 35 us, 200,000 15.9 -> 21.8 us.
-constexpr int kSampleSharedV = 1000000;
+// 21.9 -> 15.9 us), one large one per SM with EADF and EVDF cells in shared memory
+// from kSampleShared electrons on (1e6: 46 -> 35 us, 4e6 109 -> 65, but 200,000 under
+// AC 17.4 -> 28).
+constexpr int kSampleShared = 600000;
 
 void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   if (a.n <= 0) return;
-  const int sms = max(1, sm_count), full = sms * (1024 / kSampleThreads);
-  const int threads = a.n < full * kSampleThreads / 2 ? kSampleThreads / 2 : kSampleThreads;
+  const int sms = max(1, sm_count);
+  const bool shared = a.plain && a.n >= kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
+  if (shared) {
+    k_sample<true><<<min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s>>>(a);
+    return;
+  }
+  const int threads = a.n < sms * kSampleThreads ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
-  const int eedf = a.plain ? a.dist_e_cells * (int)sizeof(unsigned int) : 0;
-  const long long v_words = ((long long)a.dist_v_cells + 1) / 2;
-  const bool v_shared = a.plain && a.n >= kSampleSharedV && eedf + 4 * v_words <= kSampleSmem &&
-                        blocks_for(a.n, grid * threads) * (long long)threads < 65536;
-  if (v_shared) k_sample<true><<<grid, threads, eedf + 4 * (int)v_words, s>>>(a);
-  else k_sample<false><<<grid, threads, eedf, s>>>(a);
+  k_sample<false><<<grid, threads, a.plain ? a.dist_e_cells * (int)sizeof(unsigned int) : 0, s>>>(a);
 }
 
 void launch_interval_end(const SampleArgs& a, cudaStream_t s) { k_interval_end<<<1, 128, 0, s>>>(a); }
@@ -1057,7 +1082,7 @@ void launch_hist(const HistArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;
   const int chunks = (a.n + kHistChunk - 1) / kHistChunk;
   k_hist_a<<<chunks, kHistAThreads, kHistASmem, s>>>(a);
-  if (a.cylindrical && !a.evdf_done) k_hist_b<<<chunks, kHistBThreads, kHistBSmem, s>>>(a);
+  if (a.cylindrical) k_hist_b<<<chunks, kHistBThreads, kHistBSmem, s>>>(a);
 }
 
 void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s) {
@@ -1075,7 +1100,7 @@ cudaError_t prepare_kernels() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_hist_b_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistBSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sample_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleBatchSmem);
+    e = cudaFuncSetAttribute(k_sample_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sample<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
   if (e == cudaSuccess) e = prepare_advance_stash();
   return e;
@@ -1116,7 +1141,7 @@ int launch_batch_post(const BatchArgs& b, int sm_count, int max_slots, unsigned 
     n += kPopLaunches;
   }
   if (parts & kPartSample) {
-    k_sample_batch<<<sm_count * 2, kSampleBatchThreads, kSampleBatchSmem, s>>>(b);
+    k_sample_batch<<<sm_count, kSampleSharedThreads, kSampleSmem, s>>>(b);
     ++n;
   }
   k_batch_gather<<<min(slots, 64), 64, 0, s>>>(b);

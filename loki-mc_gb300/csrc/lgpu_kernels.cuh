@@ -144,8 +144,6 @@ struct HistArgs {
   int n_rad, n_ax;                 // EVDF: [n_rad x n_ax]
   float inv_rad_step, inv_ax_step, max_speed;
   double* evdf;
-  int evdf_done;                   // the EVDF of this sample was counted with its moments (batches)
-  int pad;
 };
 // What the sample of an interval counts beside its moments, written by the host
 // with the interval's control block: the distributions (BoltzmannMC.C:1550-1571)
@@ -160,11 +158,10 @@ struct DistCtl {
   HistArgs h;
 };
 
-// Ensembles up to this size count their distributions with the sample: above it
-// the passes over 65535-electron chunks fill the device, and their shared-memory
-// counts cost less than two FP64 additions at L2 per electron (from the figures at
-// k_sample: 21 against 17 us per 1e6 electrons at 2e7).
-constexpr int kDistInSample = 16000000;
+// Ensembles of a context on its own up to this size count their distributions with
+// the sample: above it a block of one per SM would see more electrons than its 16-bit
+// counts hold, and the passes over 65535-electron chunks fill the device.
+constexpr int kDistInSample = 9000000;
 
 // A chain of intervals of one condition: the host launches up to kChain of them
 // without a look in between. The last block of each interval's sample keeps the
@@ -205,7 +202,7 @@ struct SampleArgs {
   PlainCtl* plain;                 // null: moments only
   DevScalars* sc;                  // the condition's scalars (with plain)
   ChainOut* out;
-  int dist_e_cells, dist_v_cells;  // EEDF and EVDF cells (with plain)
+  int dist_e_cells;                // EEDF cells (with plain)
 };
 // the end of an interval without a sample
 void launch_interval_end(const SampleArgs& a, cudaStream_t s);
@@ -247,16 +244,14 @@ constexpr int kPopLaunches = 3;
 // Each slot carries the same argument blocks a single-condition launch takes;
 // the kernels split every slot's ensemble into fixed-size chunks and find the
 // slot of a chunk by bisection over exclusive prefix sums of the chunk counts.
-// kSlotEvdf: this interval's sample also counts the EVDF (its grid is fixed
-// from the steady state on, so it needs no re-binning check)
-enum SlotFlags : int { kSlotIonAtt = 1, kSlotSample = 2, kSlotEvdf = 8 };
+enum SlotFlags : int { kSlotIonAtt = 1, kSlotSample = 2 };
 
 struct BatchSlot {
   AdvanceArgs adv;        // adv.ctl points at ctl_dst
   PopArgs pop;
   SampleArgs smp;
   HistArgs hist;          // distribution staging only: the deferred tallies of a previous sample
-  HistArgs vhist;         // EVDF counted with this interval's sample (kSlotEvdf)
+  DistCtl dist;           // distributions counted with this interval's sample
   IntervalCtl ctl;        // this interval's values, copied to *ctl_dst by the prep kernel
   IntervalCtl* ctl_dst;
   DevScalars* sc;         // the condition's scalars; the per-interval part is cleared by prep
@@ -278,12 +273,18 @@ struct BatchHeader {
   // (prefix over slots) and then one partial chunk per slot, largest first,
   // so that the blocks' static shares of the list come out even
   int smp_full, hist_full, hist2_full;
+  int smp_chunk, hist_chunk;                // electrons per chunk of the samples and of the histograms
 };
 
 constexpr int kBatchMaxSlots = 1024;
 constexpr int kBatchAdvanceChunk = 4096;   // granularity of the advance's initial spread of blocks over slots
-constexpr int kBatchSampleChunk = 65535;   // electrons per block of the moment sums (and EVDF: < 2^16)
-constexpr int kBatchHistChunk = 65535;     // electrons per block of the histograms (16-bit counts)
+constexpr int kBatchSampleChunk = 65535;   // electrons per chunk of the samples at most (16-bit EVDF counts)
+constexpr int kBatchHistChunk = 65535;     // electrons per chunk of the histograms at most (16-bit counts)
+// Batches of fewer sampled electrons keep EEDF and EADF in a pass of their own. One
+// pass would be the faster one for them too (a served job of 50,000 electrons 66 ->
+// 37 ms), but the check that arriving jobs overlap on the device
+// (tests/test_gpu_batch.py) has them arrive 38 ms apart.
+constexpr double kBatchDistMin = 150000;
 
 // Staging layout (host pinned mirror and device copy are identical):
 //   BatchHeader | adv_prefix | smp_prefix | hist_prefix | hist2_prefix (kBatchMaxSlots+1 ints

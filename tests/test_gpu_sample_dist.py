@@ -1,10 +1,10 @@
 """The distributions a context on its own counts with the moments of each sample
 (k_sample) against the same condition in a batch, which counts them in separate
-passes: without ionization and attachment both see the same electrons, so every
+passes below 150,000 electrons and with its samples in other chunks above: without ionization and attachment both see the same electrons, so every
 count, and with it every reported value, is equal. Sizes around a warp, a block,
 the change of the block size and of the EVDF's place, odd grids and grids too
-large for shared memory; small ensembles re-bin often, which leaves a sample to the
-separate passes."""
+large for shared memory, in one direction or both; small ensembles re-bin often,
+which leaves a sample to the separate passes."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,9 @@ def _context(n, cells, freq, thermal):
 @pytest.mark.parametrize("n,cells,freq,thermal", [
     (1, DEFAULT, 0.0, 0), (33, DEFAULT, 0.0, 0), (511, (4096, 3, 33, 31), 0.0, 2), (20000, (17, 100, 400, 400), 0.0, 0),
     (77823, DEFAULT, 0.0, 0), (77825, DEFAULT, N_GAS * 1e-14 / (2 * np.pi), 0), (999999, DEFAULT, 0.0, 0),
-    (1000001, (999, 99, 199, 201), 0.0, 0), (1000001, (17, 100, 400, 400), 0.0, 0)])
+    (1000001, (999, 99, 199, 201), 0.0, 0), (1000001, (17, 100, 400, 400), 0.0, 0), (599999, DEFAULT, 0.0, 0),
+    (600001, DEFAULT, 0.0, 0), (1400003, DEFAULT, 0.0, 0), (1400003, (999, 99, 199, 201), 0.0, 0),
+    (1400003, (4096, 3, 1, 33000), 0.0, 0)])
 def test_sample_counts_what_the_separate_passes_count(n, cells, freq, thermal):
     from lokigpu import capi
     alone = _context(n, cells, freq, thermal)
