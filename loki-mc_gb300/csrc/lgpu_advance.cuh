@@ -353,7 +353,7 @@ __device__ __forceinline__ const ProcF* procs_of(const AdvanceArgs& a, const Sh&
 // A process's nominal energy change per collision (eV): minus its threshold
 // (the gain of a superelastic process), none for attachment, whose loss is
 // the electron's whole energy.
-__device__ __forceinline__ float nominal_change(const ProcF& p) { return p.type == kAttachment ? 0.0f : -p.eloss; }
+__device__ __forceinline__ float nominal_change(int type, float eloss) { return type == kAttachment ? 0.0f : -eloss; }
 
 // The collision turn: process choice, kinematics, tallies, secondaries and
 // attachment (BoltzmannMC.C:907-1280).
@@ -370,8 +370,8 @@ __device__ __forceinline__ void lane_real(const AdvanceArgs& a, Sh& sh, int wid,
   } else {
     ++tl.real_n;
     atomicAdd(&sh.count[cr.chosen], 1u);
-    const int ptype = procs[cr.chosen].type;
-    const float rest = cr.dE - nominal_change(procs[cr.chosen]);
+    const int ptype = cr.type;
+    const float rest = cr.dE - nominal_change(ptype, cr.eloss);
     if (cr.dE >= 0.0f) {
       if (rest != 0.0f) atomicAdd(&sh.gain[cr.chosen], rest);
     } else {
@@ -461,7 +461,7 @@ __device__ __forceinline__ void block_flush(const AdvanceArgs& a, Sh& sh, const 
   for (int q = threadIdx.x; q < a.P; q += blockDim.x) {
     if (sh.count[q]) {
       atomicAdd(&a.proc_count[q], (unsigned long long)sh.count[q]);
-      const double off = (double)nominal_change(procs[q]);
+      const double off = (double)nominal_change(procs[q].type, procs[q].eloss);
       const unsigned int n_loss = sh.neg[q], n_gain = sh.count[q] - n_loss;
       if (n_gain) atomicAdd(&a.proc_gain[q], (double)n_gain * off + (double)sh.gain[q]);
       if (n_loss) atomicAdd(&a.proc_loss[q], (double)n_loss * off + (double)sh.loss[q]);
