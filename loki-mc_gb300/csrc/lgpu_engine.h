@@ -1094,46 +1094,21 @@ class Engine {
   }
 
   // EEDF grid update and remap of the accumulated tallies (BoltzmannMC.C:1495-1548)
-  int rebin_distributions() {
-    const int nEC = cfg_.n_energy_cells, nCos = cfg_.n_cos_cells, nPh = cfg_.n_phases;
-    std::vector<double> eeh(nEC), eah((size_t)nEC * nCos), per((size_t)nPh * nEC);
-    LGPU_CU(copy(eeh.data(), d_eedf_, eeh.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    if (cylindrical_)
-      LGPU_CU(copy(eah.data(), d_eadf_, eah.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    if (omega_ != 0)
-      LGPU_CU(copy(per.data(), d_eedf_per_, per.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    LGPU_TRY(sync("rebin read"));
-    const double old_step = eedf_step_, old_max = max_eedf_;
+  void rebin_distributions() {
+    RebinArgs a{};
+    a.n_e = cfg_.n_energy_cells;
+    a.n_cos = cylindrical_ ? std::max(cfg_.n_cos_cells, 0) : 0;
+    a.n_phases = omega_ != 0 ? std::max(cfg_.n_phases, 0) : 0;
+    a.old_step = eedf_step_;
+    a.old_max = max_eedf_;
     max_eedf_ = 1.2 * max_elec_energy_;
-    eedf_step_ = max_eedf_ / nEC;
-    std::vector<double> neeh(nEC, 0.0), neah((size_t)nEC * nCos, 0.0);
-    // the periodic sums are not cleared before the remap and each old column
-    // is added once per phase, as the reference does (BoltzmannMC.C:1523-1541)
-    std::vector<double> nper = per;
-    for (int o = 0; o < nEC; ++o) {
-      const double lo = o * old_step, hi = (o + 1 == nEC) ? old_max : (o + 1) * old_step;
-      const int nl = (int)(lo / eedf_step_), nr = (int)(hi / eedf_step_);
-      const double lf = (nl == nr) ? 1.0 : (nr * eedf_step_ - lo) / old_step;
-      neeh[nl] += lf * eeh[o];
-      if (nl != nr) neeh[nr] += (1.0 - lf) * eeh[o];
-      if (cylindrical_)
-        for (int c = 0; c < nCos; ++c) {
-          neah[(size_t)nl * nCos + c] += lf * eah[(size_t)o * nCos + c];
-          if (nl != nr) neah[(size_t)nr * nCos + c] += (1.0 - lf) * eah[(size_t)o * nCos + c];
-        }
-      if (omega_ != 0)
-        for (int rep = 0; rep < nPh; ++rep)
-          for (int q = 0; q < nPh; ++q) {
-            nper[(size_t)q * nEC + nl] += lf * per[(size_t)q * nEC + o];
-            if (nl != nr) nper[(size_t)q * nEC + nr] += (1.0 - lf) * per[(size_t)q * nEC + o];
-          }
-    }
-    LGPU_CU(copy(d_eedf_, neeh.data(), neeh.size() * sizeof(double), cudaMemcpyHostToDevice));
-    if (cylindrical_)
-      LGPU_CU(copy(d_eadf_, neah.data(), neah.size() * sizeof(double), cudaMemcpyHostToDevice));
-    if (omega_ != 0)
-      LGPU_CU(copy(d_eedf_per_, nper.data(), nper.size() * sizeof(double), cudaMemcpyHostToDevice));
-    return sync("rebin write");
+    eedf_step_ = max_eedf_ / cfg_.n_energy_cells;
+    a.step = eedf_step_;
+    a.eedf = d_eedf_;
+    a.eadf = d_eadf_;
+    a.eedf_per = d_eedf_per_;
+    launch_rebin(a, stream_);
+    ++launches_;
   }
 
   // the tallies of a sample taken at `time` on the current grids
@@ -1167,7 +1142,7 @@ class Engine {
   // getTimeDependDistributions (BoltzmannMC.C:1492-1572)
   int sample_distributions() {
     if (sample_counted()) return LGPU_OK;
-    if (max_elec_energy_ > max_eedf_) LGPU_TRY(rebin_distributions());
+    if (max_elec_energy_ > max_eedf_) rebin_distributions();
     const HistArgs h = hist_args(time_);
     if (batch_) {
       pending_hist_ = h;

@@ -570,6 +570,40 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b(HistArgs a) {
     hist_chunk_b(a, c * kHistChunk, min(a.n, (c + 1) * kHistChunk), sm_hist, kHistBSmem / 4);
 }
 
+// One block per column on the energy grid: the EEDF, each angle's EADF column, each
+// phase's EEDF. A cell of the new grid adds, in their order, the shares of the old
+// cells that reach into it (an old cell is narrower than a new one and reaches into
+// two at most). As in the reference, the per-phase sums are not cleared first and
+// take every old cell once per phase (BoltzmannMC.C:1523-1541).
+//
+// On the host, between two copies of all tallies and with every per-phase cell added
+// once per phase one by one, re-binning was most of the 311 us of host work per
+// interval of 32 conditions in crossed B and AC fields (64 phases); 28 are left.
+constexpr int kRebinThreads = 256;
+
+__global__ void __launch_bounds__(kRebinThreads) k_rebin(RebinArgs a) {
+  __shared__ double old[kMaxEnergyCells];
+  const int col = blockIdx.x, nE = a.n_e;
+  const bool phase = col > a.n_cos;
+  double* v = col == 0 ? a.eedf : phase ? a.eedf_per + (size_t)(col - 1 - a.n_cos) * nE : a.eadf + (col - 1);
+  const int stride = col == 0 || phase ? 1 : a.n_cos;
+  for (int o = threadIdx.x; o < nE; o += blockDim.x) old[o] = v[(size_t)o * stride];
+  __syncthreads();
+  const double ratio = a.step / a.old_step;
+  for (int c = threadIdx.x; c < nE; c += blockDim.x) {
+    double s = 0.0;
+    const int first = max(0, (int)fmin(c * ratio, (double)nE) - 2), last = min(nE - 1, (int)fmin((c + 1) * ratio, (double)nE) + 2);
+    for (int o = first; o <= last; ++o) {
+      const double lo = o * a.old_step, hi = o + 1 == nE ? a.old_max : (o + 1) * a.old_step;
+      const int nl = (int)(lo / a.step), nr = (int)(hi / a.step);
+      const double lf = nl == nr ? 1.0 : (nr * a.step - lo) / a.old_step;
+      if (nl == c) s += lf * old[o];
+      if (nr == c && nl != nr) s += (1.0 - lf) * old[o];
+    }
+    v[(size_t)c * stride] = phase ? old[c] + a.n_phases * s : s;
+  }
+}
+
 // ------------------------------------------------------- population control
 __device__ __forceinline__ uint32_t pop_word(uint32_t idx, uint64_t interval, uint64_t seed, uint32_t salt,
                                              uint32_t draw) {
@@ -1074,6 +1108,10 @@ void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   const int threads = a.n < sms * kSampleThreads ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
   k_sample<false><<<grid, threads, a.plain ? a.dist_e_cells * (int)sizeof(unsigned int) : 0, s>>>(a);
+}
+
+void launch_rebin(const RebinArgs& a, cudaStream_t s) {
+  k_rebin<<<1 + a.n_cos + a.n_phases, kRebinThreads, 0, s>>>(a);
 }
 
 void launch_interval_end(const SampleArgs& a, cudaStream_t s) { k_interval_end<<<1, 128, 0, s>>>(a); }

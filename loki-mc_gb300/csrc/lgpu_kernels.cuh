@@ -145,6 +145,16 @@ struct HistArgs {
   float inv_rad_step, inv_ax_step, max_speed;
   double* evdf;
 };
+// The tallies on the energy grid moved to a wider one (BoltzmannMC.C:1495-1548).
+struct RebinArgs {
+  int n_e, n_cos, n_phases;        // n_cos 0: no EADF; n_phases 0: no per-phase EEDFs
+  double old_step, old_max, step;  // the grids' cell widths, the old one's maximum
+  double* eedf;                    // [n_e]
+  double* eadf;                    // [n_e x n_cos]
+  double* eedf_per;                // [n_phases x n_e]
+};
+void launch_rebin(const RebinArgs& a, cudaStream_t s);
+
 // What the sample of an interval counts beside its moments, written by the host
 // with the interval's control block: the distributions (BoltzmannMC.C:1550-1571)
 // when their energy grid holds every electron. Whether it does is known before
