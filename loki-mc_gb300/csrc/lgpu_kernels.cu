@@ -338,6 +338,8 @@ __device__ __forceinline__ void end_interval(const SampleArgs& a, bool sampled) 
 }
 
 __global__ void k_interval_end(SampleArgs a) {
+  next_may_start();
+  wait_for_previous();
   if (a.plain->ctl.go) end_interval(a, false);
 }
 
@@ -428,6 +430,8 @@ __global__ void __launch_bounds__(SHARED ? kSampleSharedThreads : kSampleThreads
   __shared__ double s_m[(SHARED ? kSampleSharedThreads : kSampleThreads) / 32][kMoments];
   __shared__ bool s_last;
   extern __shared__ unsigned int sm_dist[];
+  next_may_start();
+  wait_for_previous();
   if (a.plain && !a.plain->ctl.go) return;  // the chain of intervals has stopped
   const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   const bool counts = a.plain && a.plain->dist.on &&
@@ -802,6 +806,8 @@ __global__ void __launch_bounds__(kPopThreads) k_pop_fill(const __grid_constant_
   __shared__ DrainShared sh;
   __shared__ AdvanceArgs s_a;
   __shared__ PopPlan pl;
+  next_may_start();
+  wait_for_previous();
   // (a slot's spill count is final here except for its own drain, which only raises it)
   auto spilled = [](const AdvanceArgs& a) { return *(volatile const int*)a.spill_count != 0; };
   for (int s = blockIdx.x; s < src.count(); s += gridDim.x) {
@@ -822,6 +828,8 @@ __global__ void __launch_bounds__(kPopThreads) k_pop_fill(const __grid_constant_
 template <class Src>
 __global__ void __launch_bounds__(kPopThreads) k_pop_clone(Src src) {
   __shared__ PopPlan pl;
+  next_may_start();
+  wait_for_previous();
   pop_phase(src, pl, pop_left, [](const PopArgs& a, int item) {
     const int n_att = pop_attached(a), n_sec = pop_sec_total(a);
     if (n_att > n_sec) {
@@ -860,6 +868,8 @@ __global__ void __launch_bounds__(kPopThreads) k_pop_clone(Src src) {
 template <class Src>
 __global__ void __launch_bounds__(kPopThreads) k_pop_place(Src src) {
   __shared__ PopPlan pl;
+  next_may_start();
+  wait_for_previous();
   pop_phase(src, pl, pop_left, [](const PopArgs& a, int item) {
     const int n_att = pop_attached(a), n_sec = pop_sec_total(a);
     if (n_att > n_sec) {
@@ -880,9 +890,9 @@ __global__ void __launch_bounds__(kPopThreads) k_pop_place(Src src) {
 
 template <class Src>
 void launch_pop_phases(const Src& src, int grid, cudaStream_t s) {
-  k_pop_fill<<<grid, kPopThreads, 0, s>>>(src);
-  k_pop_clone<<<grid, kPopThreads, 0, s>>>(src);
-  k_pop_place<<<grid, kPopThreads, 0, s>>>(src);
+  launch_after(k_pop_fill<Src>, grid, kPopThreads, 0, s, src);
+  launch_after(k_pop_clone<Src>, grid, kPopThreads, 0, s, src);
+  launch_after(k_pop_place<Src>, grid, kPopThreads, 0, s, src);
 }
 
 // ---------------------------------------------------------- batch helpers
@@ -1069,11 +1079,11 @@ void launch_advance(const AdvanceArgs& args, cudaStream_t s) {
   const int all = grid * warps;
   a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
   switch (a.field.mode) {
-    case kFieldDC: k_advance<kFieldDC><<<grid, threads, 0, s>>>(a); break;
-    case kFieldAC: k_advance<kFieldAC><<<grid, threads, 0, s>>>(a); break;
-    case kFieldB: k_advance<kFieldB><<<grid, threads, 0, s>>>(a); break;
-    case kFieldECR: k_advance<kFieldECR><<<grid, threads, 0, s>>>(a); break;
-    default: k_advance<kFieldACB><<<grid, threads, 0, s>>>(a); break;
+    case kFieldDC: launch_after(k_advance<kFieldDC>, grid, threads, 0, s, a); break;
+    case kFieldAC: launch_after(k_advance<kFieldAC>, grid, threads, 0, s, a); break;
+    case kFieldB: launch_after(k_advance<kFieldB>, grid, threads, 0, s, a); break;
+    case kFieldECR: launch_after(k_advance<kFieldECR>, grid, threads, 0, s, a); break;
+    default: launch_after(k_advance<kFieldACB>, grid, threads, 0, s, a); break;
   }
 }
 
@@ -1102,19 +1112,19 @@ void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   const int sms = max(1, sm_count);
   const bool shared = a.plain && a.n >= kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
   if (shared) {
-    k_sample<true><<<min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s>>>(a);
+    launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s, a);
     return;
   }
   const int threads = a.n < sms * kSampleThreads ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
-  k_sample<false><<<grid, threads, a.plain ? a.dist_e_cells * (int)sizeof(unsigned int) : 0, s>>>(a);
+  launch_after(k_sample<false>, grid, threads, a.plain ? a.dist_e_cells * sizeof(unsigned int) : 0, s, a);
 }
 
 void launch_rebin(const RebinArgs& a, cudaStream_t s) {
   k_rebin<<<1 + a.n_cos + a.n_phases, kRebinThreads, 0, s>>>(a);
 }
 
-void launch_interval_end(const SampleArgs& a, cudaStream_t s) { k_interval_end<<<1, 128, 0, s>>>(a); }
+void launch_interval_end(const SampleArgs& a, cudaStream_t s) { launch_after(k_interval_end, 1, 128, 0, s, a); }
 
 void launch_hist(const HistArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;
