@@ -59,9 +59,11 @@ __device__ __forceinline__ int append_slot(int* counter) {
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// after_kernel: the last work on the stream is a kernel that calls next_may_start
+// (else an ordinary launch)
 template <class... Params, class... Args>
 cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                         const Args&... args) {
+                         bool after_kernel, const Args&... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;
@@ -71,8 +73,15 @@ cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
-  c.numAttrs = 1;
+  c.numAttrs = after_kernel ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+// the device's clock in nanoseconds
+__device__ __forceinline__ unsigned long long device_clock() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
 }
 
 // Launch shapes of the advance: threads per block, blocks per SM (which fix
@@ -787,13 +796,6 @@ __device__ __forceinline__ void drain_body(AdvanceArgs& a, Sh& sh) {
   __syncthreads();
 }
 
-// the device's clock in nanoseconds
-__device__ __forceinline__ unsigned long long device_clock() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
 // One condition per launch: every warp starts on its own a.share electrons and takes
 // kOwnChunk at a time after them.
 constexpr int kOwnChunk = 32;
@@ -848,11 +850,18 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
   __shared__ AdvanceArgs s_a;
   __shared__ IntervalView s_iv;
   __shared__ int s_slot;
+  next_may_start();
+  wait_for_previous();
   const int s0 = b.hdr->mode_slot[MODE], s1 = b.hdr->mode_slot[MODE + 1];
   if (s0 >= s1) return;  // no slot with this field branch (uniform over the grid)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t warp_tag = (uint32_t)(blockIdx.x * Sh::kWarps + wid);
   const int n_slots = b.hdr->n_slots;
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    atomicMin(&b.hdr->advance_begin, device_clock());
+    asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(&b.out->published), "r"(b.hdr->pos) : "memory");
+  }
+  bool ran = false;
   if (threadIdx.x == 0) {
     const int c0 = b.hdr->mode_chunk[MODE], c1 = b.hdr->mode_chunk[MODE + 1];
     const int c = c0 + (int)(((long long)blockIdx.x * (c1 - c0)) / gridDim.x);
@@ -864,19 +873,22 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
   for (;;) {
     const int slot = s_slot;
     if (slot < 0) break;
-    load_slot_args(&b.slots[slot].adv, &s_a);
-    __syncthreads();
-    load_block_consts(s_a, sh);
-    if (threadIdx.x == 0) s_iv = interval_view<-1>(s_a);
-    __syncthreads();
-    reset_tally(tl);
-    const WarpCursor<Sh::kChunk, false> cur;
-    if constexpr (Sh::kStash > 0)
-      warp_loop_stash<MODE>(s_a, sh, adv_stash + wid * 4 * Sh::kStash, s_iv, tl, sec_id, warp_tag, cur);
-    else
-      warp_loop<MODE, false>(s_a, sh, s_iv, tl, sec_id, warp_tag, cur);
-    __syncthreads();  // every warp is done with the slot
-    block_flush(s_a, sh, tl, lane, wid);
+    if (b.slots[slot].ctl.go) {  // else its chain of intervals has stopped
+      ran = true;
+      load_slot_args(&b.slots[slot].adv, &s_a);
+      __syncthreads();
+      load_block_consts(s_a, sh);
+      if (threadIdx.x == 0) s_iv = interval_view<-1>(s_a);
+      __syncthreads();
+      reset_tally(tl);
+      const WarpCursor<Sh::kChunk, false> cur;
+      if constexpr (Sh::kStash > 0)
+        warp_loop_stash<MODE>(s_a, sh, adv_stash + wid * 4 * Sh::kStash, s_iv, tl, sec_id, warp_tag, cur);
+      else
+        warp_loop<MODE, false>(s_a, sh, s_iv, tl, sec_id, warp_tag, cur);
+      __syncthreads();  // every warp is done with the slot
+      block_flush(s_a, sh, tl, lane, wid);
+    }
     __syncthreads();  // the flush has read the shared tallies and arguments
     // the next slot of the branch with electrons left, in rotation order from
     // this one: warp 0 checks 32 slots' counters per round
@@ -890,7 +902,7 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
         if (k <= cnt) {
           s = s0 + (slot - s0 + k) % cnt;
           const AdvanceArgs& o = b.slots[s].adv;
-          left = *(volatile int*)o.work_counter < o.n;
+          left = b.slots[s].ctl.go && *(volatile int*)o.work_counter < o.n;
         }
         const unsigned m = __ballot_sync(0xffffffffu, left);
         if (m) nxt = __shfl_sync(0xffffffffu, s, __ffs(m) - 1);
@@ -899,6 +911,7 @@ __global__ void __launch_bounds__(AdvShape<SHAPE>::kThreads, AdvShape<SHAPE>::kB
     }
     __syncthreads();
   }
+  if (ran && threadIdx.x == 0) atomicMax(&b.hdr->advance_end, device_clock());
 }
 
 }  // namespace
@@ -910,15 +923,15 @@ namespace {
 
 // The batched advance of every field branch in `parts`, in launch shape SHAPE.
 template <int SHAPE>
-int launch_batch_advance_shape(const BatchArgs& b, int sm_count, unsigned parts, cudaStream_t s) {
+int launch_batch_advance_shape(const BatchArgs& b, int sm_count, unsigned parts, bool after_kernel, cudaStream_t s) {
   constexpr int kT = AdvShape<SHAPE>::kThreads, kDyn = adv_stash_bytes<SHAPE>();
   const int grid = sm_count * AdvShape<SHAPE>::kBlocksPerSM;
   int n = 0;
-  if (parts & (1u << kFieldDC)) k_advance_batch<kFieldDC, SHAPE><<<grid, kT, kDyn, s>>>(b), ++n;
-  if (parts & (1u << kFieldAC)) k_advance_batch<kFieldAC, SHAPE><<<grid, kT, kDyn, s>>>(b), ++n;
-  if (parts & (1u << kFieldB)) k_advance_batch<kFieldB, SHAPE><<<grid, kT, kDyn, s>>>(b), ++n;
-  if (parts & (1u << kFieldECR)) k_advance_batch<kFieldECR, SHAPE><<<grid, kT, kDyn, s>>>(b), ++n;
-  if (parts & (1u << kFieldACB)) k_advance_batch<kFieldACB, SHAPE><<<grid, kT, kDyn, s>>>(b), ++n;
+  if (parts & (1u << kFieldDC)) launch_after(k_advance_batch<kFieldDC, SHAPE>, grid, kT, kDyn, s, after_kernel, b), ++n;
+  if (parts & (1u << kFieldAC)) launch_after(k_advance_batch<kFieldAC, SHAPE>, grid, kT, kDyn, s, after_kernel, b), ++n;
+  if (parts & (1u << kFieldB)) launch_after(k_advance_batch<kFieldB, SHAPE>, grid, kT, kDyn, s, after_kernel, b), ++n;
+  if (parts & (1u << kFieldECR)) launch_after(k_advance_batch<kFieldECR, SHAPE>, grid, kT, kDyn, s, after_kernel, b), ++n;
+  if (parts & (1u << kFieldACB)) launch_after(k_advance_batch<kFieldACB, SHAPE>, grid, kT, kDyn, s, after_kernel, b), ++n;
   return n;
 }
 

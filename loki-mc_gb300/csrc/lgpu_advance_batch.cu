@@ -5,14 +5,15 @@
 
 namespace lgpu {
 
-int launch_batch_advance(const BatchArgs& b, int sm_count, unsigned parts, int shape, cudaStream_t s) {
+int launch_batch_advance(const BatchArgs& b, int sm_count, unsigned parts, int shape, bool after_kernel,
+                         cudaStream_t s) {
   switch (shape) {
-    case 1: return launch_batch_advance_shape<1>(b, sm_count, parts, s);
-    case 2: return launch_batch_advance_shape<2>(b, sm_count, parts, s);
-    case 3: return launch_batch_advance_shape<3>(b, sm_count, parts, s);
+    case 1: return launch_batch_advance_shape<1>(b, sm_count, parts, after_kernel, s);
+    case 2: return launch_batch_advance_shape<2>(b, sm_count, parts, after_kernel, s);
+    case 3: return launch_batch_advance_shape<3>(b, sm_count, parts, after_kernel, s);
     case 4:
-    case 5: return launch_batch_advance_stash(b, sm_count, parts, shape, s);
-    default: return launch_batch_advance_shape<0>(b, sm_count, parts, s);
+    case 5: return launch_batch_advance_stash(b, sm_count, parts, shape, after_kernel, s);
+    default: return launch_batch_advance_shape<0>(b, sm_count, parts, after_kernel, s);
   }
 }
 

@@ -5,9 +5,10 @@
 
 namespace lgpu {
 
-int launch_batch_advance_stash(const BatchArgs& b, int sm_count, unsigned parts, int shape, cudaStream_t s) {
-  return shape == 5 ? launch_batch_advance_shape<5>(b, sm_count, parts, s)
-                    : launch_batch_advance_shape<4>(b, sm_count, parts, s);
+int launch_batch_advance_stash(const BatchArgs& b, int sm_count, unsigned parts, int shape, bool after_kernel,
+                         cudaStream_t s) {
+  return shape == 5 ? launch_batch_advance_shape<5>(b, sm_count, parts, after_kernel, s)
+                    : launch_batch_advance_shape<4>(b, sm_count, parts, after_kernel, s);
 }
 
 cudaError_t prepare_advance_stash() {

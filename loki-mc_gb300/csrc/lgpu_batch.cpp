@@ -59,10 +59,10 @@ int lgpu_batch_step(lgpu_batch* batch, int n, int* running, lgpu_batch_report* r
                n0 = b.null_, hm0 = b.host_ms_, se0 = b.secondaries_, sp0 = b.spilled_, at0 = b.attached_, rg0 = b.regrids_;
   const auto t0 = std::chrono::steady_clock::now();
   int rc = LGPU_OK;
-  for (int i = 0; i < n && rc == LGPU_OK; ++i) {
+  for (int i = 0, ran = 0; i < n && rc == LGPU_OK; i += ran) {
     b.admit();
     if (b.active_.empty()) break;
-    rc = b.step();
+    rc = b.step(n - i, &ran);
   }
   if (running) *running = (int)b.active_.size();
   if (report) {

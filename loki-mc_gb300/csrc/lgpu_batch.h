@@ -3,17 +3,20 @@
 // A Batch drives any number of Engines (one swarm condition each) through
 // their own solve steps - the control flow of BoltzmannMC::evaluateEEDF
 // (BoltzmannMC.C:299-426) stays per condition, on the host - while the device
-// work of one synchronisation interval of every running condition is two CUDA
-// graph launches: first the previous samples' distribution tallies (launched
-// before the host works through the conditions, so that its work runs beside
-// them), then slot control blocks and scalars (prep), one persistent advance
-// launch per field branch over all slots' electrons, spilled secondaries and
-// population control over all slots' items, the moment sums and a gather of every
-// slot's scalars into mapped host memory. Per interval the
-// host stages one BatchSlot per running condition (the argument blocks the
-// single-condition launches take, plus the interval's control block) into
-// pinned memory and copies it over once. A condition whose energy grid is
-// re-built sits an interval out while the re-build runs on its own stream.
+// work of one synchronisation interval of every running condition is one sequence
+// of launches: one persistent advance launch per field branch over all slots'
+// electrons, spilled secondaries and population control over all slots' items, the
+// samples (moments and, in the same read, distributions) and the interval's end,
+// which keeps every slot's scalars in mapped host memory and sets up its next
+// interval. Intervals are launched ahead of the host's part of the ones before
+// (ChainCtl) until a slot needs the host, which sits out the one or two already
+// launched. Before a chain the host stages one BatchSlot per
+// running condition (the argument blocks the single-condition launches take, plus
+// the chain's control blocks) into pinned memory and copies it over once. The
+// distributions of a small batch, and a sample that outgrew its energy grid, are
+// counted by launches of their own before the next chain, while the host works
+// through the conditions. A condition whose energy grid is re-built sits a chain out
+// while the re-build runs on its own stream.
 //
 // Slots: at most max_slots conditions run at a time; conditions beyond that
 // wait in order of addition and start as running ones finish, so a long run
@@ -38,24 +41,20 @@ class Batch {
   std::string err_;
   int device_ = 0, max_slots_ = 0, sm_count_ = 1;
   cudaStream_t stream_ = nullptr;
-  cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   // field branches after the first run their advance on side streams, forked
-  // from and joined to the batch stream inside the interval graph
+  // from and joined to the batch stream in every interval
   cudaStream_t side_[kFieldModes - 1] = {};
   cudaEvent_t fork_ = nullptr, join_[kFieldModes - 1] = {};
   char* h_stage_ = nullptr;
   char* d_stage_ = nullptr;
   char* h_hstage_ = nullptr;  // the distribution passes' staging (same layout)
   char* d_hstage_ = nullptr;
-  DevScalars* h_gather_ = nullptr;  // mapped pinned memory: the gather kernel writes it directly
-  DevScalars* d_gather_ = nullptr;  // its device address
-  // one instantiated graph per set of launch groups in use (BatchParts; the
-  // distribution passes' graphs carry kGraphHist)
-  static constexpr unsigned kGraphHist = 1u << 16;
-  std::map<unsigned, std::pair<cudaGraphExec_t, int>> graphs_;
+  // mapped pinned memory, written by the device, and its device addresses
+  DevScalars *h_gather_ = nullptr, *d_gather_ = nullptr;
+  BatchOut *h_out_ = nullptr, *d_out_ = nullptr;
   // scratch of the pass layouts (lgpu_chunks.h): electrons and inclusion per
   // slot, remainders
-  std::vector<int> n_;
+  std::vector<int> n_, seen_, rc_;  // seen_, rc_: a slot's intervals the host has worked through, and how
   std::vector<unsigned char> take_, all_;
   std::vector<std::pair<int, int>> rem_;
   // totals since creation
@@ -208,7 +207,6 @@ class Batch {
     if ((rc = cuda(prepare_kernels(), "kernel attributes"))) return rc;
     if ((rc = cuda(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device), "attribute"))) return rc;
     if ((rc = cuda(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "stream"))) return rc;
-    if ((rc = cuda(cudaEventCreate(&ev0_), "event")) || (rc = cuda(cudaEventCreate(&ev1_), "event"))) return rc;
     if ((rc = cuda(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "event"))) return rc;
     for (int k = 0; k < kFieldModes - 1; ++k)
       if ((rc = cuda(cudaStreamCreateWithFlags(&side_[k], cudaStreamNonBlocking), "stream")) ||
@@ -223,10 +221,12 @@ class Batch {
     if ((rc = cuda(cudaMalloc((void**)&d_hstage_, sb), "cudaMalloc"))) return rc;
     std::memset(h_hstage_, 0, sb);
     if ((rc = cuda(cudaMemsetAsync(d_hstage_, 0, sb, stream_), "memset"))) return rc;
-    if ((rc = cuda(cudaHostAlloc((void**)&h_gather_, (size_t)max_slots * sizeof(DevScalars), cudaHostAllocMapped),
-                   "cudaHostAlloc")))
+    if ((rc = cuda(cudaHostAlloc((void**)&h_gather_, (size_t)kBatchChain * max_slots * sizeof(DevScalars),
+                                 cudaHostAllocMapped), "cudaHostAlloc")))
       return rc;
     if ((rc = cuda(cudaHostGetDevicePointer((void**)&d_gather_, h_gather_, 0), "cudaHostGetDevicePointer"))) return rc;
+    if ((rc = cuda(cudaHostAlloc((void**)&h_out_, sizeof(BatchOut), cudaHostAllocMapped), "cudaHostAlloc"))) return rc;
+    if ((rc = cuda(cudaHostGetDevicePointer((void**)&d_out_, h_out_, 0), "cudaHostGetDevicePointer"))) return rc;
     return cuda(cudaStreamSynchronize(stream_), "init");
   }
 
@@ -235,19 +235,16 @@ class Batch {
     for (Member& m : members_)
       if (m.e && !m.done) m.e->leave_batch();
     clear_members();
-    for (auto& g : graphs_) cudaGraphExecDestroy(g.second.first);
-    graphs_.clear();
     if (d_stage_) cudaFree(d_stage_);
     if (h_stage_) cudaFreeHost(h_stage_);
     if (d_hstage_) cudaFree(d_hstage_);
     if (h_hstage_) cudaFreeHost(h_hstage_);
     d_hstage_ = h_hstage_ = nullptr;
     if (h_gather_) cudaFreeHost(h_gather_);
+    if (h_out_) cudaFreeHost(h_out_);
+    h_out_ = d_out_ = nullptr;
     d_stage_ = h_stage_ = nullptr;
     d_gather_ = h_gather_ = nullptr;
-    if (ev0_) cudaEventDestroy(ev0_);
-    if (ev1_) cudaEventDestroy(ev1_);
-    ev0_ = ev1_ = nullptr;
     if (fork_) cudaEventDestroy(fork_);
     fork_ = nullptr;
     for (int k = 0; k < kFieldModes - 1; ++k) {
@@ -270,61 +267,36 @@ class Batch {
     b.smp_part = b.hist2_prefix + (kBatchMaxSlots + 1);
     b.hist_part = b.smp_part + kBatchMaxSlots;
     b.hist2_part = b.hist_part + kBatchMaxSlots;
-    b.slots = reinterpret_cast<const BatchSlot*>(stage + batch_slots_offset());
+    b.slots = reinterpret_cast<BatchSlot*>(stage + batch_slots_offset());
     b.gather = d_gather_;
+    b.out = d_out_;
+    b.max_slots = max_slots_;
     return b;
   }
 
-  // the kernels of one interval (or of the distribution passes, kGraphHist),
-  // captured once per set of launch groups: their sizes come from the staged
-  // header, so one graph serves every interval and every membership
-  // graph keys: the launch groups (BatchParts) and, above bit 20, the shape
-  static constexpr int kGraphShapeShift = 20;
-  int graph(unsigned parts, cudaGraphExec_t* out, int* kernels) {
-    auto it = graphs_.find(parts);
-    if (it == graphs_.end()) {
-      cudaGraph_t g;
-      int rc;
-      if ((rc = cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture"))) return rc;
-      int n = 0;
-      if (parts & kGraphHist) {
-        n = launch_batch_hist(args(d_hstage_), sm_count_, parts, stream_);
-      } else {
-        const BatchArgs b = args(d_stage_);
-        n = launch_batch_pre(b, sm_count_, max_slots_, parts, stream_);
-        cudaEventRecordWithFlags(ev0_, stream_, cudaEventRecordExternal);
-        // one persistent launch per field branch; with several branches they
-        // run side by side, so the blocks of one fill the SMs another's tail
-        // leaves idle (each branch's slots are its own: nothing is shared)
-        const int shape = (int)(parts >> kGraphShapeShift);
-        const unsigned modes = parts & ((1u << kFieldModes) - 1u);
-        const unsigned rest = parts & ~((1u << kFieldModes) - 1u);
-        int first = 0;
-        while (first < kFieldModes && !(modes & (1u << first))) ++first;
-        int k = 0;
-        if (modes & ~(1u << first)) cudaEventRecord(fork_, stream_);
-        for (int m = first + 1; m < kFieldModes; ++m) {
-          if (!(modes & (1u << m))) continue;
-          cudaStreamWaitEvent(side_[k], fork_, 0);
-          n += launch_batch_advance(b, sm_count_, rest | (1u << m), shape, side_[k]);
-          cudaEventRecord(join_[k], side_[k]);
-          ++k;
-        }
-        if (first < kFieldModes) n += launch_batch_advance(b, sm_count_, rest | (1u << first), shape, stream_);
-        for (int j = 0; j < k; ++j) cudaStreamWaitEvent(stream_, join_[j], 0);
-        cudaEventRecordWithFlags(ev1_, stream_, cudaEventRecordExternal);
-        n += launch_batch_post(b, sm_count_, max_slots_, parts, stream_);
-      }
-      if ((rc = cuda(cudaStreamEndCapture(stream_, &g), "capture"))) return rc;
-      cudaGraphExec_t ge = nullptr;
-      rc = cuda(cudaGraphInstantiate(&ge, g, 0), "instantiate");
-      cudaGraphDestroy(g);
-      if (rc) return rc;
-      it = graphs_.emplace(parts, std::make_pair(ge, n)).first;
+  // The kernels of one interval; their sizes come from the staged header. first: the
+  // one right behind the staging copy. Returns the kernels launched.
+  int enqueue_interval(int n_slots, unsigned parts, int shape, bool first_of_chain) {
+    const BatchArgs b = args(d_stage_);
+    // one persistent launch per field branch; with several branches they
+    // run side by side, so the blocks of one fill the SMs another's tail
+    // leaves idle (each branch's slots are its own: nothing is shared)
+    const unsigned modes = parts & ((1u << kFieldModes) - 1u);
+    const unsigned rest = parts & ~((1u << kFieldModes) - 1u);
+    int first = 0, n = 0, k = 0;
+    while (first < kFieldModes && !(modes & (1u << first))) ++first;
+    const bool several = (modes & ~(1u << first)) != 0;
+    if (several) cudaEventRecord(fork_, stream_);
+    for (int m = first + 1; m < kFieldModes; ++m) {
+      if (!(modes & (1u << m))) continue;
+      cudaStreamWaitEvent(side_[k], fork_, 0);
+      n += launch_batch_advance(b, sm_count_, rest | (1u << m), shape, false, side_[k]);
+      cudaEventRecord(join_[k], side_[k]);
+      ++k;
     }
-    *out = it->second.first;
-    *kernels = it->second.second;
-    return LGPU_OK;
+    n += launch_batch_advance(b, sm_count_, rest | (1u << first), shape, !several && !first_of_chain, stream_);
+    for (int j = 0; j < k; ++j) cudaStreamWaitEvent(stream_, join_[j], 0);
+    return n + launch_batch_post(b, sm_count_, n_slots, parts, !several, stream_);
   }
 
   // ------------------------------------------------------------ membership
@@ -375,11 +347,12 @@ class Batch {
     active_.erase(std::remove(active_.begin(), active_.end(), idx), active_.end());
   }
 
-  // One synchronisation interval of every running member. Members whose stop
-  // criteria hold (or that fail) finish here; *finished lists them. A member
-  // whose energy grid is being re-built (on its own stream, concurrently with
-  // this interval) sits the interval out and goes on at the next step.
-  int step(std::vector<int>* finished = nullptr) {
+  // Up to `most` synchronisation intervals of every running member (*ran: how many
+  // were launched). Members whose stop criteria hold (or that fail) finish here;
+  // *finished lists them. A member whose energy grid is being re-built (on its own
+  // stream, concurrently) sits the chain out and goes on at the next step.
+  int step(int most = kBatchChain, int* ran = nullptr, std::vector<int>* finished = nullptr) {
+    if (ran) *ran = 1;
     const auto h0 = std::chrono::steady_clock::now();
     // the samples left to count first: the host work below (stop criteria, trial
     // frequencies, staging) runs while they are counted
@@ -453,18 +426,29 @@ class Batch {
     double sampled = 0;
     for (int s = 0; s < n; ++s) {
       const Engine* e = member(go[s]).e;
+      electrons += e->n_electrons();
       if (e->sampling_) sampled += e->n_electrons();
     }
+    // the chain's length: what every slot can run without the host (one interval
+    // while the schedule is tuned or a member waits for its tables)
+    int chain = std::min(most, tune_stage_ < 2 || !wait.empty() ? 1 : kBatchChain);
     for (int s = 0; s < n; ++s) {
       Engine* e = member(go[s]).e;
-      if (sampled < kBatchDistMin) e->sample_moments_only();
-      e->fill_slot(&sl[s]);
+      if (!e->sampling_ || (sampled < kBatchDistMin && e->sample_moments_only())) chain = 1;
+      if (chain > 1) chain = e->chain_limit(chain, true);
+    }
+    BatchSlot* d_sl = reinterpret_cast<BatchSlot*>(d_stage_ + batch_slots_offset());
+    int rc, kernels = 0;
+    for (int s = 0; s < n; ++s) {
+      Engine* e = member(go[s]).e;
+      e->fill_slot(&sl[s], &d_sl[s], chain);
+      if (!e->scalars_clear_ && (rc = cuda(e->clear_interval_scalars() ? cudaErrorUnknown : cudaSuccess, "clear"))) return rc;
+      e->scalars_clear_ = true;
       if (e->cfg_.advance_real_batch == 0) {
         sl[s].adv.real_batch = tune_threshold(cand);
         sl[s].adv.coarse = tune_coarse(cand);
       }
       const int N = e->n_electrons();
-      electrons += N;
       parts |= 1u << e->field_mode();
       if (sl[s].flags & kSlotIonAtt) parts |= kPartIonAtt;
       ap[s] = na;
@@ -489,19 +473,61 @@ class Batch {
       hdr->mode_chunk[m] = ap[s];
       hdr->mode_slot[m] = s;
     }
-    cudaGraphExec_t ge;
-    int rc, kernels = 0;
-    if ((rc = graph(parts | ((unsigned)shape << kGraphShapeShift), &ge, &kernels))) return rc;
+    hdr->advance_begin = ~0ull;
     const size_t up = batch_slots_offset() + (size_t)n * sizeof(BatchSlot);
-    const size_t down = (size_t)n * sizeof(DevScalars);
     if ((rc = cuda(cudaMemcpyAsync(d_stage_, h_stage_, up, cudaMemcpyHostToDevice, stream_), "stage"))) return rc;
-    if ((rc = cuda(cudaGraphLaunch(ge, stream_), "graph launch"))) return rc;
+    std::memset(h_out_, 0, offsetof(BatchOut, done) + (size_t)n * sizeof(int));
+    h_out_->published = -1;
+    // The intervals are launched two ahead of the one that runs, until a slot needs
+    // the host; meanwhile the host works through the scalars of those that are over
+    // (but a slot's last ones, after which it may have work for the stream).
+    seen_.assign(n, 0);
+    rc_.assign(n, LGPU_OK);
+    auto host_part = [&](int s, int upto) {
+      Engine& e = *member(go[s]).e;
+      for (; seen_[s] < upto && rc_[s] == LGPU_OK; ++seen_[s]) {
+        const DevScalars& r = h_gather_[(size_t)seen_[s] * max_slots_ + s];
+        real_ += (double)(r.real_count - e.h_sc_->real_count);
+        null_ += (double)(r.null_count - e.h_sc_->null_count);
+        secondaries_ += r.sec_count;
+        spilled_ += r.spill_count;
+        attached_ += r.att_count;
+        electron_steps_ += e.n_electrons();
+        d2h_bytes_ += sizeof(DevScalars);
+        rc_[s] = e.after_interval(r, seen_[s] == 0, true);
+      }
+    };
+    int launched = 0;
+    for (; launched < std::min(chain, 2); ++launched) kernels += enqueue_interval(n, parts, shape, launched == 0);
     const auto h1 = std::chrono::steady_clock::now();
+    for (int s = 0, idle = 0; chain > 1;) {
+      const int running = __atomic_load_n(&h_out_->published, __ATOMIC_ACQUIRE);
+      const bool more = launched < chain && !*(volatile int*)&h_out_->stopped &&
+                        std::chrono::steady_clock::now() - h1 < std::chrono::milliseconds(20);
+      if (more && running + 2 > launched) {
+        kernels += enqueue_interval(n, parts, shape, false);
+        ++launched;
+        continue;
+      }
+      // one slot's share at a time
+      const int before = seen_[s];
+      host_part(s, std::min((int)*(volatile int*)&h_out_->done[s], running) - 1);
+      idle = seen_[s] == before ? idle + 1 : 0;
+      if (++s == n) s = 0;
+      if (idle >= n) {
+        if (!more && running >= launched - 1) break;  // the last one runs, nothing is left to do beside it
+        if (idle % (64 * n) == 0 && cudaStreamQuery(stream_) != cudaErrorNotReady) break;
+      }
+    }
     if ((rc = cuda(cudaStreamSynchronize(stream_), "batched interval"))) return rc;
     const auto h2 = std::chrono::steady_clock::now();
     if ((rc = cuda(cudaGetLastError(), "batched interval"))) return rc;
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ev0_, ev1_);
+    const int intervals = *(volatile int*)&h_out_->intervals;
+    if (intervals < 1 || intervals > chain)
+      return fail(LGPU_ERR_STATE, "a chain of " + std::to_string(chain) + " batched intervals ran " + std::to_string(intervals));
+    if (ran) *ran = intervals;
+    double ms = 0;
+    for (int k = 0; k < intervals; ++k) ms += 1e-6 * h_out_->advance_ns[k];
     adv_ms_ += ms;
     if (tune_stage_ < 2 && electrons > 0) {
       // cost per trial event (real + null collisions of the interval): the
@@ -528,25 +554,19 @@ class Batch {
         }
       }
     }
-    electron_steps_ += electrons;
-    ++intervals_;
+    intervals_ += intervals;
     launches_ += kernels;
     h2d_bytes_ += (double)up;
-    d2h_bytes_ += (double)down;
     std::vector<int> still;
     still.reserve(go.size());
     for (int s = 0; s < n; ++s) {
       Member& m = member(go[s]);
-      real_ += (double)(h_gather_[s].real_count - m.e->h_sc_->real_count);
-      null_ += (double)(h_gather_[s].null_count - m.e->h_sc_->null_count);
-      secondaries_ += h_gather_[s].sec_count;
-      spilled_ += h_gather_[s].spill_count;
-      attached_ += h_gather_[s].att_count;
-      std::memcpy(m.e->h_sc_, &h_gather_[s], sizeof(DevScalars));
-      rc = m.e->interval_post();
-      if (rc == LGPU_OK) rc = m.e->solve_post();
-      if (rc != LGPU_OK) {
-        finish(m, rc);
+      const int done = *(volatile int*)&h_out_->done[s];
+      if (done < 1 || done > chain)
+        rc_[s] = m.e->fail(LGPU_ERR_STATE, "a chain of %d batched intervals ran %d", chain, done);
+      host_part(s, done);
+      if (rc_[s] != LGPU_OK) {
+        finish(m, rc_[s]);
         if (finished) finished->push_back(go[s]);
       } else {
         still.push_back(go[s]);
@@ -570,9 +590,9 @@ class Batch {
   }
 
   // The deferred distribution tallies of the running members' last samples (of a
-  // small batch, and samples that had to be re-binned first), staged in the second staging area and launched as their own graph on
-  // the batch stream, ahead of the interval that would otherwise advance the
-  // ensemble first.
+  // small batch, and samples that had to be re-binned first), staged in the second
+  // staging area and launched on the batch stream ahead of the interval that would
+  // otherwise advance the ensemble first.
   int launch_pending_hists() {
     auto* hdr = reinterpret_cast<BatchHeader*>(h_hstage_);
     int* hp = reinterpret_cast<int*>(h_hstage_ + batch_prefix_offset()) + 2 * (kBatchMaxSlots + 1);
@@ -605,14 +625,11 @@ class Batch {
     hdr->hist2_full = pb.first;
     hdr->hist_chunks = pa.first + pa.second;
     hdr->hist2_chunks = pb.first + pb.second;
-    const unsigned parts = kGraphHist | (hdr->hist_chunks ? kPartHistA : 0u) | (hdr->hist2_chunks ? kPartHistB : 0u);
-    cudaGraphExec_t ge;
-    int rc, kernels = 0;
-    if ((rc = graph(parts, &ge, &kernels))) return rc;
+    const unsigned parts = (hdr->hist_chunks ? kPartHistA : 0u) | (hdr->hist2_chunks ? kPartHistB : 0u);
+    int rc;
     const size_t up = batch_slots_offset() + (size_t)n * sizeof(BatchSlot);
     if ((rc = cuda(cudaMemcpyAsync(d_hstage_, h_hstage_, up, cudaMemcpyHostToDevice, stream_), "stage"))) return rc;
-    if ((rc = cuda(cudaGraphLaunch(ge, stream_), "graph launch"))) return rc;
-    launches_ += kernels;
+    launches_ += launch_batch_hist(args(d_hstage_), sm_count_, parts, stream_);
     h2d_bytes_ += (double)up;
     return LGPU_OK;
   }

@@ -826,8 +826,13 @@ class Engine {
     std::memcpy(&adv_max, &h_sc_->max_energy_bits, 4);
     return h_plain_->dist.on && adv_max <= h_plain_->dist.e_bound;
   }
-  // a batch that leaves the distributions to passes of their own (after interval_pre)
-  void sample_moments_only() { h_plain_->dist.on = 0; }
+  // a batch that leaves the distributions to passes of their own (after
+  // interval_pre); whether this sample has any
+  bool sample_moments_only() {
+    const bool on = h_plain_->dist.on != 0;
+    h_plain_->dist.on = 0;
+    return on;
+  }
 
   // The second half, once the interval's device work is done and its scalars
   // are in h_sc_.
@@ -894,12 +899,9 @@ class Engine {
 
   // How many intervals may follow one another before the host has to look: up to a
   // steady-state or error check (solve_post), a stop criterion (solve_next) or the
-  // caps on steps and wall time. A chain is short at first and after one that
-  // stopped early, whose launches left were for nothing, and holds the host for a
-  // few milliseconds at most.
+  // cap on steps.
   int chain_limit(int want, bool solving) const {
-    int n = std::min({want, kChain, chain_len_});
-    if (interval_ms_ > 0) n = std::min(n, std::max(1, (int)(5.0 / interval_ms_)));
+    int n = std::min(want, kChain);
     if (!solving) return n;
     if (cfg_.sync_oversampling != 1) return 1;
     const bool ss = ss_time_ != kNonDef;
@@ -918,6 +920,43 @@ class Engine {
     return n;
   }
 
+  // the chain's part of the control blocks, n intervals from the present one on
+  // (after interval_pre)
+  void fill_chain(ChainCtl* c, int n) {
+    chain_energies();
+    c->n = n;
+    c->pos = 0;
+    c->e_lo = e_lo_;
+    c->e_hi = e_hi_;
+    c->sec_stop = sec_cap_ / 4;
+    double t = time_;
+    for (int k = 0; k < n; ++k) {
+      c->phi0[k] = (float)phase_at(t);
+      t += pending_dt_;
+      c->row[k] = h_plain_->dist.on ? hist_args(t).eedf_periodic_row : nullptr;
+    }
+  }
+
+  // The host's part of one interval of a chain, which ended with the scalars r;
+  // `first` of the chain: its interval_pre is done already.
+  int after_interval(const DevScalars& r, bool first, bool solving) {
+    if (!first) {
+      // what the device went on without: the host's own checks agree
+      bool end = false;
+      if (solving) LGPU_TRY(solve_next(&end, true));
+      if (end || !frequency_holds(cur_max_energy_))
+        return fail(LGPU_ERR_STATE, "an interval ran that the host would not have started");
+      const int dist = h_plain_->dist.on;
+      LGPU_TRY(interval_pre());
+      h_plain_->dist.on = dist;
+    }
+    *h_sc_ = r;
+    LGPU_TRY(interval_post());
+    if (solving) return solve_post();
+    ++n_samp_;
+    return process_sample();
+  }
+
   // Up to `want` synchronisation intervals on this context's own stream, without
   // a look by the host in between (PlainCtl), each followed by its part of the
   // solve loop (solving) or a sample. *ran: the intervals run, at least one.
@@ -930,25 +969,12 @@ class Engine {
     const auto t0 = std::chrono::steady_clock::now();
     LGPU_TRY(interval_pre());
     const bool sample = !solving || sampling_;
-    chain_energies();
-    const int n = sample ? chain_limit(want, solving) : 1;
-    PlainCtl& pl = *h_plain_;
-    pl.n = n;
-    pl.pos = 0;
-    pl.ticket = 0;
-    pl.e_lo = e_lo_;
-    pl.e_hi = e_hi_;
-    pl.sec_stop = sec_cap_ / 4;
-    double t = time_;
-    for (int k = 0; k < n; ++k) {
-      IntervalCtl c = pl.ctl;
-      c.interval = interval_ + k;
-      c.phi0 = (float)phase_at(t);
-      c.shift_x = c.shift_y = c.shift_z = 0.0f;
-      pl.next[k] = c;
-      t += pending_dt_;
-      pl.row[k] = pl.dist.on ? hist_args(t).eedf_periodic_row : nullptr;
-    }
+    // short at first and after one that stopped early, whose launches left were for
+    // nothing, and a few milliseconds at most
+    const int cap = interval_ms_ > 0 ? std::max(1, (int)(5.0 / interval_ms_)) : kChain;
+    const int n = sample ? chain_limit(std::min({want, cap, chain_len_}), solving) : 1;
+    fill_chain(&h_plain_->chain, n);
+    h_plain_->ticket = 0;
     LGPU_CU(copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice));
     if (!scalars_clear_) LGPU_TRY(clear_interval_scalars());
     h_out_->done = 0;
@@ -969,29 +995,13 @@ class Engine {
     const int done = *(volatile int*)&h_out_->done;
     if (done < 1 || done > n) return fail(LGPU_ERR_STATE, "a chain of %d intervals ran %d", n, done);
     interval_ms_ = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() / done;
-    chain_len_ = done == n ? std::min(2 * std::max(n, chain_len_ / 2), kChain) : 2;
-    for (int k = 0; k < done; ++k) {
-      if (k > 0) {
-        // what the device went on without: the host's own checks agree
-        bool end = false;
-        if (solving) LGPU_TRY(solve_next(&end, true));
-        if (end || !frequency_holds(cur_max_energy_))
-          return fail(LGPU_ERR_STATE, "an interval ran that the host would not have started");
-        LGPU_TRY(interval_pre());
-      }
-      *h_sc_ = h_out_->sc[k];
-      d2h_bytes_ += sizeof(DevScalars);
-      adv_ms_ += 1e-6 * (double)(h_sc_->advance_end - h_sc_->advance_begin);
-      ++adv_launches_;
-      adv_electron_steps_ += N_;
-      LGPU_TRY(interval_post());
-      if (solving) {
-        LGPU_TRY(solve_post());
-      } else {
-        ++n_samp_;
-        LGPU_TRY(process_sample());
-      }
-    }
+    for (int k = 0; k < done; ++k)
+      adv_ms_ += 1e-6 * (double)(h_out_->sc[k].advance_end - h_out_->sc[k].advance_begin);
+    adv_launches_ += done;
+    adv_electron_steps_ += (double)N_ * done;
+    d2h_bytes_ += (double)done * sizeof(DevScalars);
+    chain_len_ = done == n ? std::min(std::max(2 * n, chain_len_), kChain) : 2;
+    for (int k = 0; k < done; ++k) LGPU_TRY(after_interval(h_out_->sc[k], k == 0, solving));
     *ran = done;
     return LGPU_OK;
   }
@@ -1415,16 +1425,16 @@ class Engine {
     s.max_energy_bits = &d_sc_->sample_max_bits;
     return s;
   }
-  // this context's slot of the next batched interval (after interval_pre);
-  // the argument blocks are fixed once the ensemble starts, so they are
-  // built once per solve and only the control block and flags change
-  void fill_slot(BatchSlot* sl) {
+  // this context's slot of the next chain of n batched intervals (after
+  // interval_pre), which the device finds at d_sl; the argument blocks are fixed once
+  // the ensemble starts, so they are built once per solve and only the control
+  // blocks and flags change
+  void fill_slot(BatchSlot* sl, BatchSlot* d_sl, int n) {
     if (slot_built_ != solve_serial_) {
       std::memset(&slot_, 0, sizeof(slot_));
       slot_.adv = advance_args();
       slot_.pop = pop_args();
       slot_.smp = sample_args();
-      slot_.ctl_dst = d_ctl_;
       slot_.sc = d_sc_;
       slot_built_ = solve_serial_;
     }
@@ -1432,6 +1442,8 @@ class Engine {
     sl->ctl = *h_ctl_;
     sl->flags = (have_ion_att_ ? kSlotIonAtt : 0) | (sampling_ ? kSlotSample : 0);
     sl->dist = h_plain_->dist;
+    sl->adv.ctl = sl->pop.ctl = &d_sl->ctl;
+    fill_chain(&sl->chain, n);
   }
   // the deferred tallies of the last sample, handed to the batch's
   // distribution passes (false when there are none)

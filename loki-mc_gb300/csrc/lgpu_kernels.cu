@@ -299,48 +299,51 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
   }
 }
 
-// The end of an interval of one condition (every thread of one block calls this;
-// all other work of the interval is done): its scalars go to the host, the ones of
-// one interval are cleared, and the next interval of the chain is set up or the chain
-// stopped.
-__device__ __forceinline__ void end_interval(const SampleArgs& a, bool sampled) {
-  PlainCtl& pl = *a.plain;
-  const int pos = pl.pos;
+// The end of an interval of one condition with n electrons (every thread of one
+// block calls this; all other work of the interval is done): its scalars go to the
+// host (out[pos * stride]), the ones of one interval are cleared, and the next
+// interval of the chain is set up or the chain stopped.
+__device__ __forceinline__ void end_interval(IntervalCtl& ctl, DistCtl& dist, ChainCtl& ch, DevScalars* sc, int n,
+                                             DevScalars* out, int stride, int* done, bool sampled) {
+  const int pos = ch.pos;
   constexpr int kWords = (int)(sizeof(DevScalars) / sizeof(int));
-  const int* src = reinterpret_cast<const int*>(a.sc);
-  int* dst = reinterpret_cast<int*>(&a.out->sc[pos]);
+  const int* src = reinterpret_cast<const int*>(sc);
+  int* dst = reinterpret_cast<int*>(&out[(size_t)pos * stride]);
   for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = __ldcg(&src[k]);
   if (threadIdx.x == 0) {
-    const float e = __uint_as_float(__ldcg(&a.sc->sample_max_bits));
-    const bool counted = !pl.dist.on || __uint_as_float(__ldcg(&a.sc->max_energy_bits)) <= pl.dist.e_bound;
-    const bool go = sampled && pos + 1 < pl.n && counted && e >= pl.e_lo && e <= pl.e_hi &&
-                    __ldcg(&a.sc->error_flag) == 0 && __ldcg(&a.sc->sec_count) <= pl.sec_stop;
+    const float e = __uint_as_float(__ldcg(&sc->sample_max_bits));
+    const bool counted = !dist.on || __uint_as_float(__ldcg(&sc->max_energy_bits)) <= dist.e_bound;
+    const bool go = sampled && pos + 1 < ch.n && counted && e >= ch.e_lo && e <= ch.e_hi &&
+                    __ldcg(&sc->error_flag) == 0 && __ldcg(&sc->sec_count) <= ch.sec_stop;
     if (go) {
-      IntervalCtl c = pl.next[pos + 1];
       // the host's arithmetic: the FP64 mean, rounded to FP32
-      const double n = (double)a.n;
-      c.shift_x = (float)(__ldcg(&a.moments[1]) / n);
-      c.shift_y = (float)(__ldcg(&a.moments[2]) / n);
-      c.shift_z = (float)(__ldcg(&a.moments[3]) / n);
-      pl.ctl = c;
-      pl.dist.h.eedf_periodic_row = pl.row[pos + 1];
-      pl.pos = pos + 1;
+      ctl.shift_x = (float)(__ldcg(&sc->moments[1]) / (double)n);
+      ctl.shift_y = (float)(__ldcg(&sc->moments[2]) / (double)n);
+      ctl.shift_z = (float)(__ldcg(&sc->moments[3]) / (double)n);
+      ctl.phi0 = ch.phi0[pos + 1];
+      ++ctl.interval;
+      dist.h.eedf_periodic_row = ch.row[pos + 1];
+      ch.pos = pos + 1;
     } else {
-      pl.ctl.go = 0;
+      ctl.go = 0;
     }
-    a.out->done = pos + 1;
+    *done = pos + 1;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < (int)(offsetof(DevScalars, null_count) / sizeof(int)); k += blockDim.x)
-    reinterpret_cast<int*>(a.sc)[k] = 0;
-  if (threadIdx.x < kMoments) a.moments[threadIdx.x] = 0.0;
-  if (threadIdx.x == 0) a.sc->sample_max_bits = 0u;
+    reinterpret_cast<int*>(sc)[k] = 0;
+  if (threadIdx.x < kMoments) sc->moments[threadIdx.x] = 0.0;
+  if (threadIdx.x == 0) sc->sample_max_bits = 0u;
+}
+
+__device__ __forceinline__ void end_plain_interval(const SampleArgs& a, bool sampled) {
+  end_interval(a.plain->ctl, a.plain->dist, a.plain->chain, a.sc, a.n, a.out->sc, 1, &a.out->done, sampled);
 }
 
 __global__ void k_interval_end(SampleArgs a) {
   next_may_start();
   wait_for_previous();
-  if (a.plain->ctl.go) end_interval(a, false);
+  if (a.plain->ctl.go) end_plain_interval(a, false);
 }
 
 // The cells a block counts in shared memory (16-bit, two per word: a block sees fewer
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(SHARED ? kSampleSharedThreads : kSampleThreads
     __threadfence();
   }
   __syncthreads();
-  if (s_last) end_interval(a, true);
+  if (s_last) end_plain_interval(a, true);
 }
 
 // Below this many electrons a chunk counts EADF and EVDF with global atomics:
@@ -889,39 +892,13 @@ __global__ void __launch_bounds__(kPopThreads) k_pop_place(Src src) {
 }
 
 template <class Src>
-void launch_pop_phases(const Src& src, int grid, cudaStream_t s) {
-  launch_after(k_pop_fill<Src>, grid, kPopThreads, 0, s, src);
-  launch_after(k_pop_clone<Src>, grid, kPopThreads, 0, s, src);
-  launch_after(k_pop_place<Src>, grid, kPopThreads, 0, s, src);
+void launch_pop_phases(const Src& src, int grid, bool after_kernel, cudaStream_t s) {
+  launch_after(k_pop_fill<Src>, grid, kPopThreads, 0, s, after_kernel, src);
+  launch_after(k_pop_clone<Src>, grid, kPopThreads, 0, s, true, src);
+  launch_after(k_pop_place<Src>, grid, kPopThreads, 0, s, true, src);
 }
 
 // ---------------------------------------------------------- batch helpers
-// Before the advance: each slot's interval values to its control block, the
-// per-interval scalars cleared (and the moment sums of sampling slots), the
-// advance counter reset. One warp per slot.
-__global__ void k_batch_prep(BatchArgs b) {
-  const int n = b.hdr->n_slots;
-  const int lane = threadIdx.x & 31;
-  const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (s >= n) return;
-  const BatchSlot& sl = b.slots[s];
-  DevScalars* sc = sl.sc;
-  if (lane == 0) {
-    *sl.ctl_dst = sl.ctl;
-    sc->sec_count = 0;
-    sc->att_count = 0;
-    sc->spill_count = 0;
-    sc->error_flag = 0;
-    sc->max_energy_bits = 0u;
-    sc->work_counter = 0;
-    sc->pop_counts[0] = sc->pop_counts[1] = 0;
-  }
-  if (sl.flags & kSlotSample) {
-    if (lane < kMoments) sc->moments[lane] = 0.0;
-    if (lane == 0) sc->sample_max_bits = 0u;
-  }
-}
-
 // distribution tallies of the slots that sample them this interval
 // the chunk this block takes in round r (snake order, lgpu_chunks.h)
 __device__ __forceinline__ int snake_chunk(int r) { return snake_index(r, gridDim.x, blockIdx.x); }
@@ -965,12 +942,15 @@ constexpr int kSampleBatchShared = 8192;  // electrons of a chunk that are worth
 __global__ void __launch_bounds__(kSampleSharedThreads) k_sample_batch(BatchArgs b) {
   __shared__ double s_m[kSampleSharedThreads / 32][kMoments];
   extern __shared__ unsigned int sm_dist[];
+  next_may_start();
+  wait_for_previous();
   const int n_slots = b.hdr->n_slots, total = b.hdr->smp_chunks, n_full = b.hdr->smp_full, chunk = b.hdr->smp_chunk;
   for (int r = 0; r * (int)gridDim.x < total; ++r) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
     const ChunkRef k = pass_chunk(b.smp_prefix, b.smp_part, n_slots, n_full, chunk, c);
     const BatchSlot& sl = b.slots[k.slot];
+    if (!sl.ctl.go) continue;  // its chain has stopped
     const SampleArgs& a = sl.smp;
     const int last = min(k.first + chunk, a.n);
     if (sl.dist.on && __uint_as_float(sl.sc->max_energy_bits) <= sl.dist.e_bound) {
@@ -983,15 +963,28 @@ __global__ void __launch_bounds__(kSampleSharedThreads) k_sample_batch(BatchArgs
   }
 }
 
-// every slot's scalars into one contiguous array for a single read-back
-__global__ void k_batch_gather(BatchArgs b) {
-  const int n = b.hdr->n_slots;
-  constexpr int kWords = (int)(sizeof(DevScalars) / sizeof(int));
-  for (int s = blockIdx.x; s < n; s += gridDim.x) {
-    const int* src = reinterpret_cast<const int*>(b.slots[s].sc);
-    int* dst = reinterpret_cast<int*>(&b.gather[s]);
-    for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = src[k];
+// the end of the interval: one block per slot, and the advance's time
+constexpr int kBatchEndThreads = 128;
+
+__global__ void __launch_bounds__(kBatchEndThreads) k_batch_end(BatchArgs b) {
+  next_may_start();
+  wait_for_previous();
+  BatchHeader& h = *b.hdr;
+  const int s = blockIdx.x;
+  if (s == 0 && threadIdx.x == 0) {
+    if (h.advance_end) {  // a slot ran
+      b.out->advance_ns[h.pos] = (double)(h.advance_end - h.advance_begin);
+      b.out->intervals = h.pos + 1;
+    }
+    ++h.pos;
+    h.advance_begin = ~0ull;
+    h.advance_end = 0ull;
   }
+  BatchSlot& sl = b.slots[s];
+  if (!sl.ctl.go) return;
+  end_interval(sl.ctl, sl.dist, sl.chain, sl.sc, sl.adv.n, b.gather + s, b.max_slots, &b.out->done[s],
+               (sl.flags & kSlotSample) != 0);
+  if (threadIdx.x == 0 && !sl.ctl.go) b.out->stopped = 1;
 }
 
 // --------------------------------------------------------------- replay
@@ -1079,11 +1072,11 @@ void launch_advance(const AdvanceArgs& args, cudaStream_t s) {
   const int all = grid * warps;
   a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
   switch (a.field.mode) {
-    case kFieldDC: launch_after(k_advance<kFieldDC>, grid, threads, 0, s, a); break;
-    case kFieldAC: launch_after(k_advance<kFieldAC>, grid, threads, 0, s, a); break;
-    case kFieldB: launch_after(k_advance<kFieldB>, grid, threads, 0, s, a); break;
-    case kFieldECR: launch_after(k_advance<kFieldECR>, grid, threads, 0, s, a); break;
-    default: launch_after(k_advance<kFieldACB>, grid, threads, 0, s, a); break;
+    case kFieldDC: launch_after(k_advance<kFieldDC>, grid, threads, 0, s, true, a); break;
+    case kFieldAC: launch_after(k_advance<kFieldAC>, grid, threads, 0, s, true, a); break;
+    case kFieldB: launch_after(k_advance<kFieldB>, grid, threads, 0, s, true, a); break;
+    case kFieldECR: launch_after(k_advance<kFieldECR>, grid, threads, 0, s, true, a); break;
+    default: launch_after(k_advance<kFieldACB>, grid, threads, 0, s, true, a); break;
   }
 }
 
@@ -1112,19 +1105,19 @@ void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
   const int sms = max(1, sm_count);
   const bool shared = a.plain && a.n >= kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
   if (shared) {
-    launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s, a);
+    launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s, true, a);
     return;
   }
   const int threads = a.n < sms * kSampleThreads ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
-  launch_after(k_sample<false>, grid, threads, a.plain ? a.dist_e_cells * sizeof(unsigned int) : 0, s, a);
+  launch_after(k_sample<false>, grid, threads, a.plain ? a.dist_e_cells * sizeof(unsigned int) : 0, s, true, a);
 }
 
 void launch_rebin(const RebinArgs& a, cudaStream_t s) {
   k_rebin<<<1 + a.n_cos + a.n_phases, kRebinThreads, 0, s>>>(a);
 }
 
-void launch_interval_end(const SampleArgs& a, cudaStream_t s) { launch_after(k_interval_end, 1, 128, 0, s, a); }
+void launch_interval_end(const SampleArgs& a, cudaStream_t s) { launch_after(k_interval_end, 1, 128, 0, s, true, a); }
 
 void launch_hist(const HistArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;
@@ -1137,7 +1130,7 @@ void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s
   PopOne one;
   one.a = a;
   one.adv = adv;
-  launch_pop_phases(one, kPopBlocks, s);
+  launch_pop_phases(one, kPopBlocks, true, s);
 }
 
 cudaError_t prepare_kernels() {
@@ -1159,12 +1152,6 @@ size_t batch_slots_offset() {
   return (batch_prefix_offset() + (4 * (kBatchMaxSlots + 1) + 3 * kBatchMaxSlots) * sizeof(int) + 255) / 256 * 256;
 }
 
-int launch_batch_pre(const BatchArgs& b, int sm_count, int max_slots, unsigned parts, cudaStream_t s) {
-  const int slots = max(1, min(max_slots, kBatchMaxSlots));
-  k_batch_prep<<<(slots + 7) / 8, 256, 0, s>>>(b);
-  return 1;
-}
-
 int launch_batch_hist(const BatchArgs& b, int sm_count, unsigned parts, cudaStream_t s) {
   int n = 0;
   if (parts & kPartHistA) {
@@ -1178,21 +1165,23 @@ int launch_batch_hist(const BatchArgs& b, int sm_count, unsigned parts, cudaStre
   return n;
 }
 
-int launch_batch_post(const BatchArgs& b, int sm_count, int max_slots, unsigned parts, cudaStream_t s) {
-  const int slots = max(1, min(max_slots, kBatchMaxSlots));
+int launch_batch_post(const BatchArgs& b, int sm_count, int n_slots, unsigned parts, bool after_kernel,
+                      cudaStream_t s) {
   int n = 1;
   if (parts & kPartIonAtt) {
     PopBatch pb;
     pb.hdr = b.hdr;
     pb.slots = b.slots;
-    launch_pop_phases(pb, sm_count * kPopBlocksPerSM, s);
+    launch_pop_phases(pb, sm_count * kPopBlocksPerSM, after_kernel, s);
     n += kPopLaunches;
+    after_kernel = true;
   }
   if (parts & kPartSample) {
-    k_sample_batch<<<sm_count, kSampleSharedThreads, kSampleSmem, s>>>(b);
+    launch_after(k_sample_batch, sm_count, kSampleSharedThreads, kSampleSmem, s, after_kernel, b);
     ++n;
+    after_kernel = true;
   }
-  k_batch_gather<<<min(slots, 64), 64, 0, s>>>(b);
+  launch_after(k_batch_end, n_slots, kBatchEndThreads, 0, s, after_kernel, b);
   return n;
 }
 

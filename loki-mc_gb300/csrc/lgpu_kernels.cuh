@@ -174,24 +174,29 @@ struct DistCtl {
 constexpr int kDistInSample = 9000000;
 
 // A chain of intervals of one condition: the host launches up to kChain of them
-// without a look in between. The last block of each interval's sample keeps the
-// interval's scalars for the host, clears them and writes the next interval's
-// control block (the origin shift is the new ensemble mean), or stops the chain,
-// whose launches left then do nothing, when the host has something to do first:
-// a look at the trial frequency or energy tables (the largest energy left
-// [e_lo, e_hi]), a re-binning, larger buffers, or an error to report.
+// without a look in between. At the end of each the device keeps the interval's
+// scalars for the host, clears them and writes the next interval's control block
+// (the origin shift is the new ensemble mean), or stops the chain, whose launches
+// left then do nothing for the condition, when the host has something to do first: a
+// look at the trial frequency or energy tables (the largest energy left [e_lo,
+// e_hi]), a re-binning, larger buffers, or an error to report.
 constexpr int kChain = 16;
 
-struct PlainCtl {
-  IntervalCtl ctl;            // the interval being run
-  DistCtl dist;
+struct ChainCtl {
   int n;                      // intervals of the chain
   int pos;                    // index of the one being run
   float e_lo, e_hi;
   int sec_stop;               // more secondaries than this stop the chain
-  unsigned int ticket;        // blocks of the sample that are done (left zero)
-  IntervalCtl next[kChain];   // the control blocks of the chain, origin shifts left out
+  float phi0[kChain];         // the intervals' phases
   double* row[kChain];        // their samples' per-phase EEDF rows
+};
+
+// what the host sends before a chain of a context on its own
+struct PlainCtl {
+  IntervalCtl ctl;            // the interval being run
+  DistCtl dist;
+  ChainCtl chain;
+  unsigned int ticket;        // blocks of the sample that are done (left zero)
 };
 
 // where a chain's scalars go: host memory the device can write
@@ -257,14 +262,14 @@ constexpr int kPopLaunches = 3;
 enum SlotFlags : int { kSlotIonAtt = 1, kSlotSample = 2 };
 
 struct BatchSlot {
-  AdvanceArgs adv;        // adv.ctl points at ctl_dst
+  AdvanceArgs adv;        // adv.ctl points at this slot's ctl (the device's copy)
   PopArgs pop;
   SampleArgs smp;
   HistArgs hist;          // distribution staging only: the deferred tallies of a previous sample
   DistCtl dist;           // distributions counted with this interval's sample
-  IntervalCtl ctl;        // this interval's values, copied to *ctl_dst by the prep kernel
-  IntervalCtl* ctl_dst;
-  DevScalars* sc;         // the condition's scalars; the per-interval part is cleared by prep
+  IntervalCtl ctl;        // this interval's values
+  ChainCtl chain;
+  DevScalars* sc;         // the condition's scalars; the per-interval part is zero before an interval
   int flags;              // SlotFlags
   int pad;
 };
@@ -284,6 +289,22 @@ struct BatchHeader {
   // so that the blocks' static shares of the list come out even
   int smp_full, hist_full, hist2_full;
   int smp_chunk, hist_chunk;                // electrons per chunk of the samples and of the histograms
+  int pos;                                  // index of the interval in the chain
+  // device clock (ns) of the advance's first block's start and last block's end
+  unsigned long long advance_begin, advance_end;
+};
+
+// Where a chain of batched intervals goes: host memory the device can write. The
+// advance publishes the index of the interval it begins: what the intervals before it
+// wrote can then be read, while it runs.
+constexpr int kBatchChain = kChain;
+struct BatchOut {
+  int published;                            // -1 before the chain
+  int stopped;                              // a slot's chain has stopped
+  int intervals;                            // launched intervals in which a slot ran
+  int pad;
+  double advance_ns[kBatchChain];
+  int done[1024];                           // intervals each slot ran (kBatchMaxSlots)
 };
 
 constexpr int kBatchMaxSlots = 1024;
@@ -303,7 +324,7 @@ constexpr double kBatchDistMin = 150000;
 // passes' staging (same layout) the hist parts and each slot's `hist`.
 struct BatchArgs {
   BatchHeader* hdr;
-  const BatchSlot* slots;
+  BatchSlot* slots;
   const int* adv_prefix;
   const int* smp_prefix;    // full chunks before each slot
   const int* hist_prefix;   // energy and energy-angle distributions
@@ -311,15 +332,17 @@ struct BatchArgs {
   const int* smp_part;      // slots with a partial chunk, largest partial first
   const int* hist_part;
   const int* hist2_part;
-  DevScalars* gather;       // [kBatchMaxSlots]: each slot's scalars after the interval
+  DevScalars* gather;       // [kBatchChain x max_slots]: each slot's scalars after each interval
+  BatchOut* out;
+  int max_slots;
 };
 size_t batch_prefix_offset();   // bytes from the staging start to adv_prefix
 size_t batch_slots_offset();    // bytes from the staging start to slots[0]
-// One batched interval is three launch groups on one stream:
-//   pre:     slot control blocks and per-interval scalars
+static_assert(kBatchMaxSlots == 1024 && kBatchChain <= kChain, "BatchOut, ChainCtl");
+// One batched interval is two launch groups on one stream:
 //   advance: one persistent launch per field mode
-//   post:    spilled secondaries and population control, moments, gather
-// ahead of them, from a second staging area of the same layout, the
+//   post:    spilled secondaries and population control, samples, the interval's end
+// ahead of a chain of them, from a second staging area of the same layout, the
 // distribution passes of the previous interval's samples (`hist` of each
 // slot), launched before the host prepares the interval so that its work
 // runs beside them.
@@ -332,7 +355,6 @@ enum BatchParts : unsigned {
   kPartSample = 1u << 10, // a slot samples its moments
   kPartIonAtt = 1u << 11, // a slot has ionization or attachment (spilled secondaries, population control)
 };
-int launch_batch_pre(const BatchArgs& b, int sm_count, int max_slots, unsigned parts, cudaStream_t s);
 int launch_batch_hist(const BatchArgs& b, int sm_count, unsigned parts, cudaStream_t s);
 // The batched advance in one of kAdvShapes launch shapes (threads per block,
 // blocks per SM, electrons a warp takes at a time, records of a warp's
@@ -340,12 +362,15 @@ int launch_batch_hist(const BatchArgs& b, int sm_count, unsigned parts, cudaStre
 // shapes (lgpu_advance_stash.cu).
 constexpr int kAdvShapes = 6;
 constexpr int kFirstStashShape = 4;
-int launch_batch_advance(const BatchArgs& b, int sm_count, unsigned parts, int shape, cudaStream_t s);
-int launch_batch_advance_stash(const BatchArgs& b, int sm_count, unsigned parts, int shape, cudaStream_t s);
+int launch_batch_advance(const BatchArgs& b, int sm_count, unsigned parts, int shape, bool after_kernel,
+                         cudaStream_t s);
+int launch_batch_advance_stash(const BatchArgs& b, int sm_count, unsigned parts, int shape, bool after_kernel,
+                         cudaStream_t s);
 void advance_shape(int shape, int* threads, int* blocks_per_sm, int* chunk, int* stash);
 // dynamic shared memory of the stash shapes' kernels (part of prepare_kernels)
 cudaError_t prepare_advance_stash();
-int launch_batch_post(const BatchArgs& b, int sm_count, int max_slots, unsigned parts, cudaStream_t s);
+// after_kernel: the last work on the stream is a kernel of this interval
+int launch_batch_post(const BatchArgs& b, int sm_count, int n_slots, unsigned parts, bool after_kernel, cudaStream_t s);
 
 // End-of-job EEDF post-processing in FP64 (lgpu_post.cu): the EEDF-convolved
 // rate coefficient of every MC process (Collision.C:355-397) for each of

@@ -403,7 +403,7 @@ class Server {
       if (running_.empty()) continue;
       // ---- one interval of every running job
       std::vector<int> finished;
-      const int rc = batch_.step(&finished);
+      const int rc = batch_.step(kBatchChain, nullptr, &finished);
       if (rc != LGPU_OK) {
         // the launch sequence itself failed: every running job fails with it
         for (JobRec* r : running_) {
