@@ -54,11 +54,14 @@ __global__ void k_init(InitArgs a) {
 // Linear interpolation of the raw table (the bracketing index by bisection,
 // largest i with x_i <= x clamped to n-2, then y_i + (x-x_i)/(x_{i+1}-x_i)*(y_{i+1}-y_i)),
 // with explicit round-to-nearest operations so no FMA contraction happens.
-__device__ double interp_raw(const double* xs, const double* ys, int n, double x) {
+// x is not negative, so that its bits order against the points' as integers do: the
+// bisection stays off the FP64 pipe.
+__device__ __forceinline__ double interp_raw(const double* xs, const double* ys, int n, double x) {
+  const long long xb = __double_as_longlong(x);
   int lo = 0, hi = n - 1;
   while (hi > lo + 1) {
     const int mid = (hi + lo) >> 1;
-    if (xs[mid] > x) hi = mid; else lo = mid;
+    if (__double_as_longlong(__ldg(&xs[mid])) > xb) hi = mid; else lo = mid;
   }
   const double dx = __dsub_rn(xs[lo + 1], xs[lo]);
   return __dadd_rn(ys[lo], __dmul_rn(__ddiv_rn(__dsub_rn(x, xs[lo]), dx), __dsub_rn(ys[lo + 1], ys[lo])));
@@ -66,7 +69,7 @@ __device__ double interp_raw(const double* xs, const double* ys, int n, double x
 
 // sigma*n of process p at `energy` (a superelastic process reads its
 // inelastic partner's raw table at energy + threshold)
-__device__ double table_value(const TableBuildArgs& a, int p, double energy) {
+__device__ __forceinline__ double table_value(const TableBuildArgs& a, int p, double energy) {
   if (a.is_super[p]) {
     if (energy > a.emin[p] && energy <= a.emax[p]) {
       const double thr = a.emin[p - 1];
@@ -80,112 +83,134 @@ __device__ double table_value(const TableBuildArgs& a, int p, double energy) {
   return 0.0;
 }
 
-// One warp per energy row: the lanes interpolate the processes of the row in
-// parallel, then the cumulative row is summed in process order (the order
-// fixes the FP64 rounding) and written as FP32 row pairs.
-constexpr int kTableWarps = 4;
+// 32 energy rows per block, one per lane: the warps interpolate a process each for
+// all rows (neighbouring energies share raw intervals, and rows below a threshold
+// cost nothing), then one warp sums every lane's row over the processes in their order
+// (which fixes the FP64 rounding) and all warps write FP32 row pairs.
+//
+// Bound by FP64 issue: a warp-wide FP64 operation takes the pipe 16 cycles whatever its
+// active lanes. With the lanes on the processes of one row, a row's sum and its
+// frequency ran on one lane each: 10,000 rows of 2, 40 and 65 processes took 34, 95
+// and 140 us, 8, 31 and 44 here (44 ms of the 64-point sweep's 395: 64 first tables
+// and 200 re-grids beside its intervals).
+constexpr int kTableRows = 32, kTablePitch = kTableRows + 1;  // shared-memory pitch of a process's rows
+constexpr int kTableThreads = 256;
 
-__global__ void __launch_bounds__(32 * kTableWarps) k_build_tables(TableBuildArgs a) {
-  __shared__ double s_val[kTableWarps][kMaxProcesses];
-  __shared__ double s_cum[kTableWarps][kMaxProcesses];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int i = blockIdx.x * kTableWarps + w;
-  if (i >= a.M) return;  // whole warps
-  const int P = a.P;
+constexpr int table_smem(int P) { return P * kTablePitch * (int)(sizeof(double) + sizeof(float)); }
+
+__global__ void __launch_bounds__(kTableThreads) k_build_tables(TableBuildArgs a) {
+  extern __shared__ double s_val[];  // [P][kTablePitch] sigma*n, then the FP32 cumulative sums
+  const int P = a.P, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float* s_cum = reinterpret_cast<float*>(s_val + P * kTablePitch);
+  const int i0 = blockIdx.x * kTableRows, rows = min(kTableRows, a.M - i0), i = i0 + lane;
   const double energy = __dmul_rn((double)i, a.step);
-  for (int p = lane; p < P; p += 32) s_val[w][p] = table_value(a, p, energy);
-  __syncwarp();
-  if (lane == 0) {
+  for (int p = w; p < P; p += kTableThreads / 32)
+    s_val[p * kTablePitch + lane] = lane < rows ? table_value(a, p, energy) : 0.0;
+  __syncthreads();
+  if (w == 0) {
     double cur = 0.0;
+#pragma unroll 8
     for (int p = 0; p < P; ++p) {
-      cur = __dadd_rn(cur, s_val[w][p]);
-      s_cum[w][p] = cur;
+      cur = __dadd_rn(cur, s_val[p * kTablePitch + lane]);
+      s_cum[p * kTablePitch + lane] = (float)cur;
+      if (a.cum64 && lane < rows) a.cum64[(size_t)i * P + p] = cur;
+    }
+    if (lane < rows) {
+      const double kq = 1.6021766208e-19, km = 9.10938356e-31;
+      const double nu = __dmul_rn(cur, __dmul_rn(a.N, __dsqrt_rn(__ddiv_rn(__dmul_rn(__dmul_rn(energy, 2.0), kq), km))));
+      a.nu_tot[i] = nu;
+      a.nu_pair[i].x = (float)nu;
+      if (i > 0) a.nu_pair[i - 1].y = (float)nu;
+      if (i == a.M - 1) a.nu_pair[i].y = (float)nu;
     }
   }
-  __syncwarp();
-  for (int p = lane; p < a.stride; p += 32) {
-    const size_t k = (size_t)i * a.stride + p;
-    if (p < P) {
-      const double value = s_val[w][p], cur = s_cum[w][p];
-      if (a.sig64) a.sig64[(size_t)i * P + p] = value;
-      if (a.cum64) a.cum64[(size_t)i * P + p] = cur;
-      const float vf = (float)value, cf = (float)cur;
-      a.sig_pair[k].x = vf;
-      a.cum_pair[k].x = cf;
-      if (i > 0) {
-        a.sig_pair[k - a.stride].y = vf;
-        a.cum_pair[k - a.stride].y = cf;
-      }
-      if (i == a.M - 1) {
-        a.sig_pair[k].y = vf;
-        a.cum_pair[k].y = cf;
-      }
-    } else {
+  __syncthreads();
+  // pair (row, next row); the next block's first row completes this one's last
+  for (int k = threadIdx.x; k < rows * a.stride; k += kTableThreads) {
+    const int r = k / a.stride, p = k - r * a.stride;
+    const size_t o = (size_t)(i0 + r) * a.stride + p;
+    if (p >= P) {
       // row padding: a cumulative value no random number reaches, zero rate
-      a.cum_pair[k] = make_float2(3.0e38f, 3.0e38f);
-      a.sig_pair[k] = make_float2(0.0f, 0.0f);
+      a.cum_pair[o] = make_float2(3.0e38f, 3.0e38f);
+      a.sig_pair[o] = make_float2(0.0f, 0.0f);
+      continue;
     }
-  }
-  if (lane == 0) {
-    const double cur = s_cum[w][P - 1];
-    const double kq = 1.6021766208e-19, km = 9.10938356e-31;
-    const double nu = __dmul_rn(cur, __dmul_rn(a.N, __dsqrt_rn(__ddiv_rn(__dmul_rn(__dmul_rn(energy, 2.0), kq), km))));
-    a.nu_tot[i] = nu;
-    a.nu_pair[i].x = (float)nu;
-    if (i > 0) a.nu_pair[i - 1].y = (float)nu;
-    if (i == a.M - 1) a.nu_pair[i].y = (float)nu;
+    const double value = s_val[p * kTablePitch + r];
+    const float vf = (float)value, cf = s_cum[p * kTablePitch + r];
+    if (a.sig64) a.sig64[(size_t)(i0 + r) * P + p] = value;
+    const int next = i0 + r == a.M - 1 ? r : r + 1;  // the last row pairs with itself
+    if (next < rows) {
+      a.sig_pair[o] = make_float2(vf, (float)s_val[p * kTablePitch + next]);
+      a.cum_pair[o] = make_float2(cf, s_cum[p * kTablePitch + next]);
+    } else {
+      a.sig_pair[o].x = vf;
+      a.cum_pair[o].x = cf;
+    }
+    if (r == 0 && i0 > 0) {
+      a.sig_pair[o - a.stride].y = vf;
+      a.cum_pair[o - a.stride].y = cf;
+    }
   }
 }
 
-// running maximum of nu_tot (one block of 1024 threads, tiles of 1024 rows;
-// max is exact in any order)
+// Running maximum of nu_tot (block 0: a run of rows per warp; max is exact in any
+// order) and the block bounds of the total frequency for
+// the coarse null test (other blocks, one warp each): the largest FP32 value of rows
+// [b R, (b+1) R] (row pairs cover the next row), raised by 2^-20 relative against
+// the rounding of the interpolation. Tiles of 1024 rows one after the other, and one
+// thread per bound in a launch of its own, took 33 + 8.6 us for 10,000 rows; this
+// takes 12.
 constexpr int kPrefixThreads = 1024;
 
-__global__ void __launch_bounds__(kPrefixThreads) k_prefix_max(const double* nu_tot, double* nu_max, int M) {
-  __shared__ double s_w[kPrefixThreads / 32];
+__global__ void __launch_bounds__(kPrefixThreads) k_table_bounds(const double* nu_tot, double* nu_max, int M,
+                                                                const float2* nu_pair, int shift, float* coarse,
+                                                                int n_coarse) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  double carry = 0.0;
-  for (int base = 0; base < M; base += kPrefixThreads) {
-    const int i = base + t;
-    double v = i < M ? nu_tot[i] : 0.0;
+  if (blockIdx.x > 0) {
+    const int b = (blockIdx.x - 1) * (kPrefixThreads / 32) + w;
+    if (b >= n_coarse) return;
+    const int last = min((b + 1) << shift, M);
+    float m = 0.0f;
+    for (int i = (b << shift) + lane; i < last; i += 32) {
+      const float2 v = nu_pair[i];
+      m = fmaxf(m, fmaxf(v.x, v.y));
+    }
+    m = warp_max(m);
+    if (lane == 0) coarse[b] = m * (1.0f + 9.5367431640625e-7f);
+    return;
+  }
+  // each warp has a run of rows of its own, 32 at a time; the frequencies' bits are
+  // compared as integers, off the FP64 pipe (from 0 up, and no number never the
+  // larger one, as fmax has it)
+  __shared__ long long s_w[kPrefixThreads / 32];
+  auto key = [&](int i) {
+    const long long k = i < M ? __double_as_longlong(nu_tot[i]) : 0;
+    return k <= 0x7ff0000000000000ll ? max(k, 0ll) : 0ll;
+  };
+  const int run = (M + kPrefixThreads - 1) / kPrefixThreads * 32;
+  const int first = (int)min((long long)w * run, (long long)M), last = (int)min((long long)first + run, (long long)M);
+  long long v = 0;
+#pragma unroll 4
+  for (int i = first + lane; i < last; i += 32) v = max(v, key(i));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (lane == 0) s_w[w] = v;
+  __syncthreads();
+  long long before = lane < w ? s_w[lane] : 0;  // the rows of the warps before this one
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before = max(before, __shfl_xor_sync(0xffffffffu, before, o));
+#pragma unroll 4
+  for (int i0 = first; i0 < last; i0 += 32) {
+    v = key(i0 + lane);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const double u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v = fmax(v, u);
+      const long long u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v = max(v, u);
     }
-    if (lane == 31) s_w[w] = v;
-    __syncthreads();
-    if (w == 0) {
-      double x = s_w[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double u = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x = fmax(x, u);
-      }
-      s_w[lane] = x;
-    }
-    __syncthreads();
-    double r = fmax(carry, v);
-    if (w > 0) r = fmax(r, s_w[w - 1]);
-    if (i < M) nu_max[i] = r;
-    carry = fmax(carry, s_w[kPrefixThreads / 32 - 1]);
-    __syncthreads();
+    v = max(v, before);
+    if (i0 + lane < last) nu_max[i0 + lane] = __longlong_as_double(v);
+    before = __shfl_sync(0xffffffffu, v, 31);
   }
-}
-
-// block bounds of the total frequency for the coarse null test: the largest
-// FP32 value of rows [b R, (b+1) R] (row pairs cover the next row), raised
-// by 2^-20 relative against the rounding of the interpolation
-__global__ void k_coarse_max(const float2* nu_pair, int M, int shift, float* coarse, int n_coarse) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_coarse) return;
-  const int i0 = b << shift, i1 = min((b + 1) << shift, M);
-  float m = 0.0f;
-  for (int i = i0; i < i1; ++i) {
-    const float2 v = nu_pair[i];
-    m = fmaxf(m, fmaxf(v.x, v.y));
-  }
-  coarse[b] = m * (1.0f + 9.5367431640625e-7f);
 }
 
 // ---------------------------------------------------------------- sample
@@ -1086,9 +1111,10 @@ void launch_init(const InitArgs& a, cudaStream_t s) {
 }
 
 void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
-  k_build_tables<<<blocks_for(a.M, kTableWarps), 32 * kTableWarps, 0, s>>>(a);
-  k_prefix_max<<<1, kPrefixThreads, 0, s>>>(a.nu_tot, a.nu_max, a.M);
-  if (a.nu_coarse) k_coarse_max<<<1, kMaxCoarse, 0, s>>>(a.nu_pair, a.M, a.coarse_shift, a.nu_coarse, a.n_coarse);
+  k_build_tables<<<blocks_for(a.M, kTableRows), kTableThreads, table_smem(a.P), s>>>(a);
+  const int bounds = a.nu_coarse ? blocks_for(a.n_coarse, kPrefixThreads / 32) : 0;
+  k_table_bounds<<<1 + bounds, kPrefixThreads, 0, s>>>(a.nu_tot, a.nu_max, a.M, a.nu_pair, a.coarse_shift, a.nu_coarse,
+                                                       a.n_coarse);
 }
 
 // Blocks of the single-condition sample: half-size ones while the ensemble does
@@ -1134,7 +1160,9 @@ void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s
 }
 
 cudaError_t prepare_kernels() {
-  cudaError_t e = cudaFuncSetAttribute(k_hist_a, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistASmem);
+  static_assert(table_smem(kMaxProcesses) <= 227 * 1024, "the tables of the most processes fit a block");
+  cudaError_t e = cudaFuncSetAttribute(k_build_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, table_smem(kMaxProcesses));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_a, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistASmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_b, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistBSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_hist_a_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistASmem);
