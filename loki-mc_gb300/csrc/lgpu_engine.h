@@ -238,6 +238,8 @@ class Engine {
     for (void* p : ptrs)
       if (p) cudaFree(p);
     d_core_ = d_secbuf_ = d_procbuf_ = nullptr;
+    if (h_post_) cudaFreeHost(h_post_);
+    h_post_ = nullptr;
     if (h_pinned_) cudaFreeHost(h_pinned_);
     h_pinned_ = nullptr;
     h_sc_ = nullptr;
@@ -1656,8 +1658,10 @@ class Engine {
   double* d_tt_d_ = nullptr;
   double* d_tt_raw_ = nullptr;
   size_t tt_int_total_ = 0, tt_mom_total_ = 0;
-  double* d_post_ = nullptr;  // external EEDF, scratch, outputs
+  double* d_post_ = nullptr;  // external EEDF, scratch
   size_t post_cap_ = 0;
+  double *h_post_ = nullptr, *d_post_out_ = nullptr;  // the outputs, as the host and the device see them
+  size_t post_out_cap_ = 0;
 
   int set_twoterm(const lgpu_twoterm_process* q, int n) {
     if (P_ <= 0) return fail(LGPU_ERR_STATE, "set the processes before their two-term inputs");
@@ -1754,16 +1758,29 @@ class Engine {
     if (rate && n != P_) return fail(LGPU_ERR_BAD_ARG, "expected %d processes", P_);
     if (nc < 2 || !(max_e > 0))
       return fail(LGPU_ERR_BAD_ARG, "an EEDF needs at least 2 cells and a positive maximum energy");
-    // [ticket | EEDFs | node shares and block sums (with the parameters) | rates | parameters]
+    // [tickets | EEDFs | node shares and block sums (with the parameters) | tile sums | rates | parameters]
     const size_t nn = (size_t)nc + 1, n_f = (size_t)n_eedf * nc;
     const size_t n_shares = rates_only ? 0 : 3 * (size_t)P_ * nn, n_sums = rates_only ? 0 : eedf_post_sums(nc);
-    const size_t need = 1 + n_f + n_shares + n_sums + (size_t)n_eedf * P_ + 16;
+    constexpr size_t kTickets = (kMaxProcesses + 2) / 2;  // of 8 bytes
+    const int tile = eedf_post_tile(nc, P_, sm_count_);
+    const size_t n_parts = (size_t)P_ * n_eedf * ((nc + tile - 1) / tile);
+    const size_t n_out = std::max((size_t)n_eedf * P_ + 16, (size_t)4096);
+    const size_t need = kTickets + n_f + n_shares + n_sums + n_parts + (size_t)n_eedf * P_;
+    if (n_out > post_out_cap_) {
+      // (the device writes the results there)
+      if (h_post_) cudaFreeHost(h_post_);
+      h_post_ = nullptr;
+      post_out_cap_ = 0;
+      LGPU_CU(cudaHostAlloc((void**)&h_post_, n_out * sizeof(double), cudaHostAllocMapped));
+      LGPU_CU(cudaHostGetDevicePointer((void**)&d_post_out_, h_post_, 0));
+      post_out_cap_ = n_out;
+    }
     if (need > post_cap_) {
       if (d_post_) cudaFree(d_post_);
       d_post_ = nullptr;
       post_cap_ = 0;
       LGPU_TRY(dalloc(&d_post_, need));
-      LGPU_CU(cudaMemsetAsync(d_post_, 0, sizeof(double), stream_));
+      LGPU_CU(cudaMemsetAsync(d_post_, 0, kTickets * sizeof(double), stream_));
       post_cap_ = need;
     }
     EedfPostArgs a{};
@@ -1776,7 +1793,7 @@ class Engine {
     a.omega = omega_;
     a.omega_c = omega_c_;
     a.ticket = reinterpret_cast<unsigned int*>(d_post_);
-    double* d_eedf = d_post_ + 1;
+    double* d_eedf = d_post_ + kTickets;
     if (eedf) {
       LGPU_CU(cudaMemcpyAsync(d_eedf, eedf, n_f * sizeof(double), cudaMemcpyHostToDevice, stream_));
       a.eedf_in = d_eedf;
@@ -1785,8 +1802,9 @@ class Engine {
     a.eedf_norm = d_eedf;
     a.shares = d_eedf + n_f;
     a.sums = a.shares + n_shares;
-    a.rates = a.sums + n_sums;
-    a.params = a.rates + (size_t)n_eedf * P_;
+    a.parts = a.sums + n_sums;
+    a.rates = a.parts + n_parts;
+    a.out = d_post_out_;
     a.kind = d_tt_i_;
     a.ion = d_tt_i_ + P_;
     a.int_off = d_tt_i_ + 2 * P_;
@@ -1803,12 +1821,10 @@ class Engine {
     a.raw_mv = d_tt_raw_ + 2 * tt_int_total_ + tt_mom_total_;
     launches_ += launch_eedf_post(a, sm_count_, stream_);
     LGPU_CU(cudaGetLastError());
-    std::vector<double> res((size_t)n_eedf * P_ + 16);
-    LGPU_CU(cudaMemcpyAsync(res.data(), a.rates, res.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_));
     LGPU_TRY(sync("eedf post-processing"));
-    if (rate) std::copy(res.begin(), res.begin() + (size_t)n_eedf * P_, rate);
+    if (rate) std::copy(h_post_, h_post_ + (size_t)n_eedf * P_, rate);
     if (out) {
-      const double* v = res.data() + (size_t)n_eedf * P_;
+      const double* v = h_post_ + (size_t)n_eedf * P_;
       *out = lgpu_eedf_params{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10], v[11], v[12],
                               v[13], v[14], v[15]};
     }

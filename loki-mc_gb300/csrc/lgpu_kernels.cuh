@@ -398,11 +398,13 @@ struct EedfPostArgs {
   double* eedf_norm;       // [n_eedf][nc]: the normalised EEDFs when eeh is given
   double* shares;          // [3][P][nc + 1]: each process's share of the node totals (unless rates_only)
   double* sums;            // [eedf_post_sums(nc)]: block sums of the parameters (unless rates_only)
-  unsigned int* ticket;    // zero before the first call, left zero by each
+  double* parts;           // [P][n_eedf][tiles]: the rates' sums over tiles of cells
+  unsigned int* ticket;    // [1 + P] zero before the first call, left zero by each
   double* rates;           // [n_eedf][P]
-  double* params;          // [16], lgpu_eedf_params order
+  double* out;             // host memory: the rates, then [16] parameters (lgpu_eedf_params order)
 };
 size_t eedf_post_sums(int nc);
+int eedf_post_tile(int nc, int P, int sm_count);  // cells of a tile
 // returns the kernels it launched
 int launch_eedf_post(const EedfPostArgs& a, int sm_count, cudaStream_t s);
 

@@ -9,6 +9,7 @@
 // bit; the sums over cells run as fixed-order reductions, so they agree with
 // the reference's to rounding.
 #include "lgpu_kernels.cuh"
+#include "lgpu_launch.cuh"
 
 namespace lgpu {
 
@@ -47,18 +48,21 @@ struct PostGrid {
 // bisection), zero outside the table.
 __device__ double raw_at(const double* e, const double* v, int n, double x) {
   if (n < 2 || x < e[0] || x > e[n - 1]) return 0.0;
+  // (x is not negative, so the bits order as integers do, negative points included, and
+  // the bisection stays off the FP64 pipe)
+  const long long xb = __double_as_longlong(x);
   int lo = 0, hi = n - 1;
   while (hi > lo + 1) {
     const int mid = (hi + lo) >> 1;
-    if (e[mid] > x) hi = mid;
+    if (__double_as_longlong(e[mid]) > xb) hi = mid;
     else lo = mid;
   }
   return v[lo] + (x - e[lo]) / (e[lo + 1] - e[lo]) * (v[lo + 1] - v[lo]);
 }
 
-constexpr int kPostTile = 1024;       // cells whose cross sections a block holds at a time
+constexpr int kPostTile = 1024;       // cells of a block of the rates at most
+constexpr int kPostRateThreads = 256;
 constexpr int kPostStage = 512;       // raw points of a table staged in shared memory (longer ones stay global)
-constexpr int kPostRows = 256;        // EEDFs of one block at most
 constexpr int kPostCells = 32;        // cells per block of the parameter sums
 constexpr int kPostSums = 13;
 
@@ -77,6 +81,7 @@ __device__ __forceinline__ PostGrid post_grid(const EedfPostArgs& a) {
 // (sqrt(cell) sum(h) step)), one block per EEDF.
 __global__ void __launch_bounds__(kPostThreads) k_post_normalise(EedfPostArgs a, double* out) {
   __shared__ double red[kPostThreads / 32];
+  next_may_start();
   const PostGrid g = post_grid(a);
   const double* h = a.eeh + (size_t)blockIdx.x * a.nc;
   double* f = out + (size_t)blockIdx.x * a.nc;
@@ -98,29 +103,29 @@ __device__ __forceinline__ void stage_table(const double*& e, const double*& v, 
   v = sv;
 }
 
-// EEDF-convolved rate coefficients: one block per group of EEDFs
-// (blockIdx.x) and process (blockIdx.y). The process's cross section on a tile of the
-// grid's nodes goes to shared memory once and every EEDF of the group is summed
-// against it by a team of warps. With the parameters (one EEDF) the block also
-// writes the process's share of the momentum-transfer and energy-relaxation
-// totals at every node, which k_post_params adds up in process order.
+// EEDF-convolved rate coefficients: one block per tile of the grid's cells
+// (blockIdx.x) and process (blockIdx.y). The process's cross section on the tile's
+// nodes goes to shared memory and every EEDF is summed against it by a team of
+// warps; the last block of a process to finish adds up the tiles' sums in their order.
+// With the parameters (one EEDF) a block also writes the process's share of the
+// momentum-transfer and energy-relaxation totals at its nodes, which k_post_params
+// adds up in process order.
 //
-// Bound by FP64 issue (a few operations per SM and clock on this device), so
-// the work is spread over the SMs. Whole calls, before (one block for all
-// processes of an EEDF, one after the other) -> now: one EEDF of 1000 cells
-// with the parameters, 40 processes, 1201 -> 89 us; the rates of 100 EEDFs, 65
-// processes, 1763 -> 104 us.
-__global__ void __launch_bounds__(kPostThreads) k_post_rates(EedfPostArgs a, const double* eedf, int rows_per_block) {
-  constexpr int kWarps = kPostThreads / 32;
+// Bound by FP64 issue (a warp-wide operation takes the pipe 16 cycles), so the nodes
+// are spread over all SMs and the products go to the sums fused. One EEDF of 1000 cells,
+// 40 processes, took 1.2 ms with one block for all, 43 us with one block per process, 19
+// here; 100 EEDFs, 65 processes, 64 us before the four EEDFs side by side, 36 here.
+__global__ void __launch_bounds__(kPostRateThreads) k_post_rates(EedfPostArgs a, const double* eedf, int tile) {
+  constexpr int kWarps = kPostRateThreads / 32;
+  next_may_start();
   __shared__ double s_e[kPostStage], s_v[kPostStage];
   __shared__ double s_me[kPostStage], s_mv[kPostStage];
   __shared__ double s_sig[kPostTile + 1];
-  __shared__ double s_acc[kPostRows > kWarps ? kPostRows : kWarps];
+  __shared__ double s_acc[kWarps];
+  __shared__ bool s_last;
   const PostGrid g = post_grid(a);
-  const int nc = a.nc, nn = nc + 1, p = blockIdx.y;
+  const int nc = a.nc, nn = nc + 1, p = blockIdx.y, tiles = gridDim.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int row0 = blockIdx.x * rows_per_block, rows = min(rows_per_block, a.n_eedf - row0);
-  if (rows <= 0) return;
   const bool super = a.kind[p] == 2;
   // a superelastic copy convolves the forward collision's cross section with
   // the EEDF shifted by the threshold (Collision.C:390)
@@ -137,81 +142,120 @@ __global__ void __launch_bounds__(kPostThreads) k_post_rates(EedfPostArgs a, con
   const double *oe = a.raw_ie + a.int_off[p], *ov = a.raw_iv + a.int_off[p];
   stage_table(ie, iv, ni, s_e, s_v);
   if (shares) stage_table(me, mv, nm, s_me, s_mv);
-  for (int k = threadIdx.x; k < rows; k += blockDim.x) s_acc[k] = 0.0;
-  // warps of a team share an EEDF's cells; with fewer than kWarps EEDFs a team
-  // has several, whose partial sums are added up in a fixed order
-  int team = 1;
-  while (2 * team * rows <= kWarps) team *= 2;
-  const int t = wid % team, r_first = wid / team, r_step = kWarps / team;
-  double part = 0.0;  // this warp's sum when its team has one EEDF at most (team > 1)
-  for (int c0 = 0; c0 < nc; c0 += kPostTile) {
-    const int cells = min(kPostTile, nc - c0);
-    __syncthreads();  // the tables are staged, the previous tile is done with
-    for (int j = threadIdx.x; j <= cells; j += blockDim.x) {
-      const int i = c0 + j;
-      const double x = g.node(i);
-      // on the nodes: every one for elastic collisions, from the first above the
-      // threshold otherwise (Collision.C:221-228)
-      const double s_int = (elastic || x > fthr) ? raw_at(ie, iv, ni, x) : 0.0;
-      s_sig[j] = s_int;
-      if (!shares || (j == cells && i != nc)) continue;  // the next tile's first node writes its share
-      double w_mt = 0.0, w_er = 0.0, w_erc = 0.0;
-      if (super) {
-        // Klein-Rosseland at the nodes (Collision.C:290-353), zero at the
-        // zero-energy node (BoltzmannMC.C:2205-2217)
-        if (i > 0) {
-          const double y = x + thr, kr = 1.0 + thr / x;
-          const double w = kr * (raw_at(oe, ov, no, y) * a.stat[p]) * dens;
-          w_mt = kr * (raw_at(me, mv, nm, y) * a.stat[p]) * dens;
-          w_er = w * thr / x;
-          w_erc = w;
-        }
-      } else {
-        w_mt = ((elastic || x > thr) ? raw_at(me, mv, nm, x) : 0.0) * dens;
-        if (elastic) {
-          w_er = 2.0 * a.mass_ratio[p] * s_int * dens;
-        } else {
-          const double w = s_int * dens;
-          w_er = i > 0 ? w * thr / x : 0.0;
-          w_erc = w;
-        }
+  wait_for_previous();  // the normalisation, if there is one
+  __syncthreads();
+  const int c0 = blockIdx.x * tile, cells = min(tile, nc - c0);
+  for (int j = threadIdx.x; j <= cells; j += blockDim.x) {
+    const int i = c0 + j;
+    const double x = g.node(i);
+    // on the nodes: every one for elastic collisions, from the first above the
+    // threshold otherwise (Collision.C:221-228)
+    const double s_int = (elastic || x > fthr) ? raw_at(ie, iv, ni, x) : 0.0;
+    s_sig[j] = s_int;
+    if (!shares || (j == cells && i != nc)) continue;  // the next tile's first node writes its share
+    double w_mt = 0.0, w_er = 0.0, w_erc = 0.0;
+    if (super) {
+      // Klein-Rosseland at the nodes (Collision.C:290-353), zero at the
+      // zero-energy node (BoltzmannMC.C:2205-2217)
+      if (i > 0) {
+        const double y = x + thr, kr = 1.0 + thr / x;
+        const double w = kr * (raw_at(oe, ov, no, y) * a.stat[p]) * dens;
+        w_mt = kr * (raw_at(me, mv, nm, y) * a.stat[p]) * dens;
+        w_er = w * thr / x;
+        w_erc = w;
       }
-      double* o = a.shares + (size_t)p * nn + i;
-      o[0] = w_mt;
-      o[(size_t)a.P * nn] = w_er;
-      o[2 * (size_t)a.P * nn] = w_erc;
+    } else {
+      w_mt = ((elastic || x > thr) ? raw_at(me, mv, nm, x) : 0.0) * dens;
+      if (elastic) {
+        w_er = 2.0 * a.mass_ratio[p] * s_int * dens;
+      } else {
+        const double w = s_int * dens;
+        w_er = i > 0 ? w * thr / x : 0.0;
+        w_erc = w;
+      }
     }
-    __syncthreads();
-    // the tile's cells from lmin on, as weights (sig_l + sig_l+1) / 2 * cell_l in place
-    double keep[(kPostTile + kPostThreads - 1) / kPostThreads];
-    int m = 0;
-    for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m)
-      keep[m] = c0 + j >= lmin ? (s_sig[j] + s_sig[j + 1]) / 2.0 * g.cell(c0 + j) : 0.0;
-    __syncthreads();
-    m = 0;
-    for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m) s_sig[j] = keep[m];
-    __syncthreads();
-    const int j0 = max(0, lmin - c0);
-    for (int r = r_first; r < rows; r += r_step) {
-      const double* fr = eedf + (size_t)(row0 + r) * nc + c0 - shift;
-      double s = 0.0;
-      for (int j = j0 + 32 * t + lane; j < cells; j += 32 * team) s += s_sig[j] * fr[j];
+    double* o = a.shares + (size_t)p * nn + i;
+    o[0] = w_mt;
+    o[(size_t)a.P * nn] = w_er;
+    o[2 * (size_t)a.P * nn] = w_erc;
+  }
+  __syncthreads();
+  // the tile's cells from lmin on, as weights (sig_l + sig_l+1) / 2 * cell_l in place
+  double keep[(kPostTile + kPostRateThreads - 1) / kPostRateThreads];
+  int m = 0;
+  for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m)
+    keep[m] = c0 + j >= lmin ? (s_sig[j] + s_sig[j + 1]) / 2.0 * g.cell(c0 + j) : 0.0;
+  __syncthreads();
+  m = 0;
+  for (int j = threadIdx.x; j < cells; j += blockDim.x, ++m) s_sig[j] = keep[m];
+  __syncthreads();
+  const int j0 = max(0, lmin - c0);
+  double* part = a.parts + (size_t)p * a.n_eedf * tiles + blockIdx.x;  // [EEDF][tile]
+  // warps of a team share an EEDF's cells; with fewer EEDFs than warps a team has
+  // several, whose sums are added up in their order
+  int team = 1;
+  while (2 * team * a.n_eedf <= kWarps) team *= 2;
+  const int t = wid % team;
+  // a warp takes four EEDFs at a time: four chains of sums in flight, and the lanes'
+  // sums of all four in six steps (each lane hands half of what it has to its partner)
+  constexpr int kSide = 4;
+  for (int r0 = wid / team; r0 < a.n_eedf; r0 += kSide * (kWarps / team)) {
+    const int stride = kWarps / team, rows = min(kSide, (a.n_eedf - r0 + stride - 1) / stride);
+    const double* fr = eedf + (size_t)r0 * nc + c0 - shift;
+    const size_t dr = (size_t)stride * nc;
+    double s[kSide] = {0.0, 0.0, 0.0, 0.0};
+    if (rows == kSide) {
+      for (int j = j0 + 32 * t + lane; j < cells; j += 32 * team) {
+        const double w = s_sig[j];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (team > 1) part += s;
-      else if (lane == 0) s_acc[r] += s;
+        for (int q = 0; q < kSide; ++q) s[q] = __fma_rn(w, fr[q * dr + j], s[q]);
+      }
+    } else {
+      for (int q = 0; q < rows; ++q) {
+        double v = 0.0;
+        for (int j = j0 + 32 * t + lane; j < cells; j += 32 * team) v = __fma_rn(s_sig[j], fr[q * dr + j], v);
+        s[0] = q == 0 ? v : s[0];
+        s[1] = q == 1 ? v : s[1];
+        s[2] = q == 2 ? v : s[2];
+      }
+    }
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double u0 = (h16 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h16 ? s[0] : s[2], 16);
+    const double u1 = (h16 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h16 ? s[1] : s[3], 16);
+    double v = (h8 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, h8 ? u0 : u1, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int q = (h16 ? 2 : 0) + (h8 ? 1 : 0);  // the EEDF that this lane's sum is of
+    if ((lane & 7) == 0 && q < rows) {
+      if (team > 1) s_acc[wid] = v;  // (one EEDF per team then)
+      else part[(size_t)(r0 + q * stride) * tiles] = v;
     }
   }
   __syncthreads();
-  if (team > 1) {  // at most one EEDF per team: r_first
-    if (lane == 0) s_acc[wid] = part;
-    __syncthreads();
-  }
-  const double k = sqrt(2.0 * kQeP / kMeP) * (super ? a.stat[p] : 1.0);
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+  if (team > 1 && threadIdx.x < a.n_eedf) {
     double s = 0.0;
-    for (int w = 0; w < team; ++w) s += s_acc[r * team + w];
-    a.rates[(size_t)(row0 + r) * a.P + p] = nc > lmin ? k * s * g.step : 0.0;
+    for (int w = 0; w < team; ++w) s += s_acc[threadIdx.x * team + w];
+    part[(size_t)threadIdx.x * tiles] = s;
+  }
+  // the process's last block adds up the tiles
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.ticket[1 + p], 1u) == (unsigned)tiles - 1;
+    if (s_last) a.ticket[1 + p] = 0u;  // for the next call
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  const double k = sqrt(2.0 * kQeP / kMeP) * (super ? a.stat[p] : 1.0);
+  for (int r = threadIdx.x; r < a.n_eedf; r += blockDim.x) {
+    const double* q = a.parts + ((size_t)p * a.n_eedf + r) * tiles;
+    double s = 0.0;
+#pragma unroll 4
+    for (int w = 0; w < tiles; ++w) s += __ldcg(&q[w]);
+    s = nc > lmin ? k * s * g.step : 0.0;
+    a.rates[(size_t)r * a.P + p] = s;
+    a.out[(size_t)r * a.P + p] = s;
   }
 }
 
@@ -226,6 +270,7 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
   const PostGrid g = post_grid(a);
   const int nc = a.nc, nn = nc + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c0 = blockIdx.x * kPostCells;
+  wait_for_previous();
   if (wid < 3) {
     for (int j = lane; j <= kPostCells; j += 32) {
       const int i = c0 + j;
@@ -316,7 +361,7 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
     const double* s = s_sum;
     const double pre = N * 3.0 * factor * g.step;
     const double v_d = 2.0 * factor * g.step * s[4], v_m = -factor * s[6];
-    double* o = a.params;
+    double* o = a.out + a.P;
     o[0] = k_ion;
     o[1] = k_att;
     o[2] = pre * s[0];
@@ -338,6 +383,14 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
 
 }  // namespace
 
+// Tiles, of 32 cells at least, so that the blocks about fill the device twice (100 EEDFs
+// of 1000 cells, 65 processes: 40.5 us filling it once, 36 twice).
+int eedf_post_tile(int nc, int P, int sm_count) {
+  const int tiles = max(1, 2 * sm_count / max(P, 1));
+  const int tile = ((nc + tiles - 1) / tiles + 31) / 32 * 32;
+  return min(tile, kPostTile);
+}
+
 size_t eedf_post_sums(int nc) { return (size_t)((nc + kPostCells - 1) / kPostCells) * kPostSums; }
 
 int launch_eedf_post(const EedfPostArgs& a, int sm_count, cudaStream_t s) {
@@ -348,15 +401,10 @@ int launch_eedf_post(const EedfPostArgs& a, int sm_count, cudaStream_t s) {
     eedf = a.eedf_norm;
     ++n;
   }
-  // groups of EEDFs so that the blocks about fill the device once: a block
-  // interpolates its process's cross section itself, so more groups than that
-  // only repeat it
-  const int fill = max(1, sm_count / max(a.P, 1));
-  const int groups = max((a.n_eedf + kPostRows - 1) / kPostRows, min(a.n_eedf, fill));
-  const int rows = (a.n_eedf + groups - 1) / groups;
-  k_post_rates<<<dim3((a.n_eedf + rows - 1) / rows, a.P), kPostThreads, 0, s>>>(a, eedf, rows);
+  const int tile = eedf_post_tile(a.nc, a.P, sm_count);
+  launch_after(k_post_rates, dim3((a.nc + tile - 1) / tile, a.P), kPostRateThreads, 0, s, n > 1, a, eedf, tile);
   if (!a.rates_only) {
-    k_post_params<<<(a.nc + kPostCells - 1) / kPostCells, 128, 0, s>>>(a, eedf);
+    launch_after(k_post_params, (a.nc + kPostCells - 1) / kPostCells, 128, 0, s, true, a, eedf);
     ++n;
   }
   return n;
