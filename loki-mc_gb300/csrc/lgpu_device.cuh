@@ -172,9 +172,8 @@ __device__ __forceinline__ void free_flight(const FieldF& f, float phi0, float d
       sincosf(phi0, &sPhi, &cPhi);
       const float wdt = __fmul_rn(w, dt);
       sincosf(__fadd_rn(phi0, wdt), &sPh, &cPh);
-      const float k = __fdiv_rn(f.e_me, w);  // e/(m w)
-      const float aux1 = __fmul_rn(__fdiv_rn(k, w), __fsub_rn(__fmaf_rn(wdt, sPhi, cPh), cPhi));
-      const float aux2 = __fmul_rn(k, __fsub_rn(sPhi, sPh));
+      const float aux1 = __fmul_rn(f.k_w, __fsub_rn(__fmaf_rn(wdt, sPhi, cPh), cPhi));
+      const float aux2 = __fmul_rn(f.k, __fsub_rn(sPhi, sPh));
       p.x = __fadd_rn(p.x, __fmaf_rn(v.x, dt, __fmul_rn(f.Ex, aux1)));
       p.y = __fmaf_rn(v.y, dt, p.y);
       p.z = __fadd_rn(p.z, __fmaf_rn(v.z, dt, __fmul_rn(f.Ez, aux1)));
@@ -192,7 +191,7 @@ __device__ __forceinline__ void free_flight(const FieldF& f, float phi0, float d
       const float cWm1 = __fmul_rn(__fmul_rn(-2.0f, sh), sh);  // cos(W dt) - 1 without cancellation
       const float sW_W = __fdiv_rn(sW, W);
       const float aux2 = __fdiv_rn(cWm1, W);
-      const float vEx = __fdiv_rn(__fmul_rn(f.e_me, f.Ex), W);
+      const float vEx = f.vEx;
       const float az = __fmul_rn(f.e_me, f.Ez);
       const float vx0 = v.x, vy0 = v.y, vz0 = v.z;
       p.x = __fadd_rn(p.x, __fmaf_rn(vx0, sW_W, __fmul_rn(__fadd_rn(vy0, vEx), aux2)));
@@ -214,8 +213,7 @@ __device__ __forceinline__ void free_flight(const FieldF& f, float phi0, float d
       const float cOpp = cosf(phi0 - Wdt);
       const float sh = sinf(0.5f * Wdt);
       const float cWm1 = -2.0f * sh * sh;
-      const float k = f.e_me / W;
-      const float vEx = k * f.Ex, vEz = k * f.Ez;
+      const float vEx = f.vEx, vEz = f.vEz;
       const float sW_W = sW / W, cWm1_W = cWm1 / W, cPh_W = cPh / W;
       const float vx0 = v.x, vy0 = v.y, vz0 = v.z;
       p.x += vx0 * sW_W + vy0 * cWm1_W - 0.25f * vEx * (cPh_W - cOpp / W + 2.0f * dt * sPh);
@@ -238,16 +236,14 @@ __device__ __forceinline__ void free_flight(const FieldF& f, float phi0, float d
       sincosf(Wdt, &sW, &cW);
       const float sh = sinf(0.5f * Wdt);
       const float cWm1 = -2.0f * sh * sh;
-      const float w2 = w * w, W2 = W * W, d = w2 - W2;
-      const float vEx = f.e_me / W * f.Ex;
-      const float vEz = f.e_me / w * f.Ez;
-      const float vEx_d = vEx / d;
+      const float w2 = w * w, W2 = W * W;
+      const float vEz = f.vEz, vEx_d = f.vEx_d;
       const float WvEx_d = W * vEx_d;
       const float sW_W = sW / W, cWm1_W = cWm1 / W;
       const float wsPhi = w * sPhi;
       const float vx0 = v.x, vy0 = v.y, vz0 = v.z;
       p.x += vx0 * sW_W + vy0 * cWm1_W + WvEx_d * (cPhi * (cw - cW) + (wsPhi * sW_W - sPhi * sw));
-      p.y += -vx0 * cWm1_W + vy0 * sW_W - vEx_d / w * ((W2 + w2 * cW - w2) * sPhi + W2 * (w * cPhi * sW_W - sPh));
+      p.y += -vx0 * cWm1_W + vy0 * sW_W - f.vEx_dw * ((W2 + w2 * cW - w2) * sPhi + W2 * (w * cPhi * sW_W - sPh));
       p.z += vz0 * dt + vEz * ((cPh - cPhi) / w + dt * sPhi);
       v.x = vx0 * cW - vy0 * sW + WvEx_d * w * (cW * sPhi - sPh + cPhi / w * W * sW);
       v.y = vx0 * sW + vy0 * cW + vEx_d * W2 * (cPh - cPhi * cW + wsPhi * sW_W);

@@ -438,6 +438,7 @@ class Engine {
     else if (freq_ == 0) f.mode = kFieldB;
     else if (std::abs(omega_ - omega_c_) / omega_ < 1E-6) f.mode = kFieldECR;
     else f.mode = kFieldACB;
+    f.set_quotients();
     field_ = f;
     chain_nu_ = 0;  // the chains' energy limits follow the field
     return LGPU_OK;

@@ -140,6 +140,7 @@ int run_flights(int device, const double e_field[3], double freq_hz, double red_
   else if (freq_hz == 0) f.mode = lgpu::kFieldB;
   else if (std::abs(omega - cyclotron) / omega < 1E-6) f.mode = lgpu::kFieldECR;
   else f.mode = lgpu::kFieldACB;
+  f.set_quotients();
   double phase_rate = 0.0;
   if (f.mode == lgpu::kFieldAC || f.mode == lgpu::kFieldACB) phase_rate = omega;
   else if (f.mode == lgpu::kFieldECR) phase_rate = cyclotron;
