@@ -65,7 +65,8 @@ typedef struct lgpu_config {
   double max_seconds;               /* wall-clock cap of one solve (<= 0: none) */
   long long max_sync_steps;         /* interval cap of one solve (<= 0: none) */
   int advance_real_batch;           /* lanes of a warp with a pending real collision that start its
-                                       collision turn (1..32); 0: 20 alone, tuned on line in a batch.
+                                       collision turn (1..32); 0: 16 (20 with thermal targets) alone,
+                                       tuned on line in a batch.
                                        Scheduling only: no result depends on it */
   int advance_queue;                /* secondaries a warp keeps in its own queue before it spills them to
                                        the global buffer the drain launch works off (1..32; 0: 32).

@@ -733,7 +733,8 @@ class Engine {
     a.advance_end = &d_sc_->advance_end;
     a.sm_count = sm_count_;
     a.ctl = d_ctl_;
-    a.real_batch = cfg_.advance_real_batch > 0 ? std::min(cfg_.advance_real_batch, 32) : kDefaultRealBatch;
+    a.real_batch = cfg_.advance_real_batch > 0 ? std::min(cfg_.advance_real_batch, 32)
+                   : cfg_.gas_temperature_effect == kGasTempFalse ? kRealBatchCold : kRealBatchThermal;
     a.coarse = 1;
     a.local_q = cfg_.advance_queue > 0 ? cfg_.advance_queue : 32;
     return a;

@@ -86,7 +86,12 @@ struct AdvanceArgs {
   int share;
   unsigned long long *advance_begin, *advance_end;
 };
-constexpr int kDefaultRealBatch = 20;
+// Lanes with a pending collision that start a warp's collision turn. Cold gases take
+// their null test in the flight, so that the lanes that wait idle through other
+// lanes' flights: 16 (4e6 electrons, atomic gas: 168 us, 176 with 20, 190 with 24; 1e6,
+// N2-like: 62 at 16 and 20, 65 at 24). With thermal targets every event waits for the
+// turn: 20 (1e6, mixture under crossed B: 95 us, 99 with 16, 94 with 24).
+constexpr int kRealBatchCold = 16, kRealBatchThermal = 20;
 
 void launch_advance(const AdvanceArgs& a, cudaStream_t s);
 
