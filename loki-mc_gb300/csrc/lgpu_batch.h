@@ -457,9 +457,7 @@ class Batch {
       take_[s] = (sl[s].flags & kSlotSample) ? 1 : 0;
     }
     ap[n] = na;
-    // one chunk per block of the samples (one per SM) while the electrons last; more
-    // and smaller ones cost more in clearing and adding up than they even out
-    const int chunk = even_chunk(sampled, sm_count_, kBatchSampleChunk, 1024);
+    const int chunk = even_chunk(n, n_.data(), take_.data(), sm_count_, kBatchSampleChunk, 1024);
     const auto smp = layout_pass(n, n_.data(), take_.data(), chunk, sp, spart, rem_);
     std::memset(hdr, 0, sizeof(BatchHeader));
     hdr->smp_chunk = chunk;
@@ -582,13 +580,6 @@ class Batch {
     return LGPU_OK;
   }
 
-  // The electrons of a chunk, at most `most`, with which `electrons` make equally
-  // many chunks for each of `blocks`.
-  static int even_chunk(double electrons, int blocks, int most, int least) {
-    const double rounds = std::max(1.0, std::ceil(electrons / ((double)blocks * most)));
-    return std::min(most, std::max(least, (int)std::ceil(electrons / (blocks * rounds))));
-  }
-
   // The deferred distribution tallies of the running members' last samples (of a
   // small batch, and samples that had to be re-binned first), staged in the second
   // staging area and launched on the batch stream ahead of the interval that would
@@ -615,7 +606,7 @@ class Batch {
     if (n == 0) return LGPU_OK;
     all_.assign(n, 1);
     const int chunk = electrons < kBatchDistMin ? kBatchHistChunk
-                                                : even_chunk(electrons, sm_count_, kBatchHistChunk, 4096);
+                                                : even_chunk(n, n_.data(), all_.data(), sm_count_, kBatchHistChunk, 4096);
     const auto pa = layout_pass(n, n_.data(), all_.data(), chunk, hp, hpart, rem_);
     const auto pb = layout_pass(n, n_.data(), take_.data(), chunk, vp, vpart, rem_);
     std::memset(hdr, 0, sizeof(BatchHeader));

@@ -18,6 +18,7 @@
 
 #if !defined(__CUDA_ARCH__)
 #include <algorithm>
+#include <cmath>
 #include <utility>
 #include <vector>
 #endif
@@ -76,6 +77,37 @@ inline std::pair<int, int> layout_pass(int n_slots, const int* n, const unsigned
                    [](const std::pair<int, int>& x, const std::pair<int, int>& y) { return x.first > y.first; });
   for (size_t k = 0; k < rem.size(); ++k) part_slot[k] = rem[k].second;
   return {full, (int)rem.size()};
+}
+
+// The electrons of a chunk of a pass over the conditions with take[s], between `least`
+// and `most`. While one round over the blocks does: as few as leave one chunk to a
+// block, the conditions' remainders included. A block's second chunk, however small, adds
+// a whole pass's latency: with an even share of all electrons instead, and the
+// remainders on top of a round of chunks, the samples of 32 conditions of
+// 10,000-30,000 electrons took 33 us, now 25, those of 16 served jobs 53, now 41. With
+// several rounds the chunks even out, and the even share is as good (sweep: 178 us,
+// 182 with as few chunks as fit two rounds).
+inline int even_chunk(int n_slots, const int* n, const unsigned char* take, int blocks, int most, int least) {
+  double all = 0;
+  for (int s = 0; s < n_slots; ++s)
+    if (take[s]) all += n[s];
+  auto one_round = [&](int chunk) {
+    int c = 0;
+    for (int s = 0; s < n_slots; ++s)
+      if (take[s]) c += (n[s] - 1) / chunk + 1;
+    return c <= blocks;
+  };
+  if (!one_round(most)) {
+    const double rounds = std::max(1.0, std::ceil(all / ((double)blocks * most)));
+    return std::min(most, std::max(least, (int)std::ceil(all / (blocks * rounds))));
+  }
+  int lo = least, hi = most;
+  while (lo < hi) {
+    const int mid = lo + (hi - lo) / 2;
+    if (one_round(mid)) hi = mid;
+    else lo = mid + 1;
+  }
+  return hi;
 }
 #endif
 

@@ -960,9 +960,9 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b_batch(BatchArgs b) {
 // own, took 123 + 195 us per interval; all of it takes 178 here (3.6 TB/s), about
 // half of it the counts (issue, shared additions) and a third the addition of every
 // chunk's occupied cells to the tallies at L2. 32 conditions of 10,000-30,000
-// electrons: 21 + 66 -> 34 us. Loads in flight are not what it waits for: a ring of
+// electrons: 21 + 66 -> 25 us. Loads in flight are not what it waits for: a ring of
 // asynchronous copies in place of the four records in registers took 193.
-constexpr int kSampleBatchShared = 8192;  // electrons of a chunk that are worth shared cells (16 jobs: 62 us with 4096, 53)
+constexpr int kSampleBatchShared = 8192;  // electrons of a chunk that are worth shared cells (16 jobs: 41 us, 56 with 16384)
 
 __global__ void __launch_bounds__(kSampleSharedThreads) k_sample_batch(BatchArgs b) {
   __shared__ double s_m[kSampleSharedThreads / 32][kMoments];
