@@ -608,29 +608,42 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b(HistArgs a) {
 // two at most). As in the reference, the per-phase sums are not cleared first and
 // take every old cell once per phase (BoltzmannMC.C:1523-1541).
 //
-// On the host, between two copies of all tallies and with every per-phase cell added
-// once per phase one by one, re-binning was most of the 311 us of host work per
-// interval of 32 conditions in crossed B and AC fields (64 phases); 28 are left.
+// Bound by the FP64 divisions that place an old cell: done once per cell, to shared
+// memory, 1000 cells and 100 angles take 19 us, and took 75 with every new cell
+// placing the old ones about it again. On the host, between two copies of all tallies
+// and with every per-phase cell added once per phase one by one, re-binning was most of
+// the 311 us of host work per interval of 32 conditions in crossed B and AC fields (64
+// phases); 28 are left.
 constexpr int kRebinThreads = 256;
+// old value, its share of the lower new cell, that cell (twice, plus one if the old cell
+// reaches into the next)
+constexpr int kRebinCell = 2 * sizeof(double) + sizeof(int);
 
 __global__ void __launch_bounds__(kRebinThreads) k_rebin(RebinArgs a) {
-  __shared__ double old[kMaxEnergyCells];
+  extern __shared__ double rebin_old[];
   const int col = blockIdx.x, nE = a.n_e;
+  double* old = rebin_old;
+  double* share = old + nE;
+  int* place = reinterpret_cast<int*>(share + nE);
   const bool phase = col > a.n_cos;
   double* v = col == 0 ? a.eedf : phase ? a.eedf_per + (size_t)(col - 1 - a.n_cos) * nE : a.eadf + (col - 1);
   const int stride = col == 0 || phase ? 1 : a.n_cos;
-  for (int o = threadIdx.x; o < nE; o += blockDim.x) old[o] = v[(size_t)o * stride];
+  for (int o = threadIdx.x; o < nE; o += blockDim.x) {
+    old[o] = v[(size_t)o * stride];
+    const double lo = o * a.old_step, hi = o + 1 == nE ? a.old_max : (o + 1) * a.old_step;
+    const int nl = (int)(lo / a.step), nr = (int)(hi / a.step);
+    share[o] = nl == nr ? 1.0 : (nr * a.step - lo) / a.old_step;
+    place[o] = 2 * nl + (nl != nr);
+  }
   __syncthreads();
   const double ratio = a.step / a.old_step;
   for (int c = threadIdx.x; c < nE; c += blockDim.x) {
     double s = 0.0;
     const int first = max(0, (int)fmin(c * ratio, (double)nE) - 2), last = min(nE - 1, (int)fmin((c + 1) * ratio, (double)nE) + 2);
     for (int o = first; o <= last; ++o) {
-      const double lo = o * a.old_step, hi = o + 1 == nE ? a.old_max : (o + 1) * a.old_step;
-      const int nl = (int)(lo / a.step), nr = (int)(hi / a.step);
-      const double lf = nl == nr ? 1.0 : (nr * a.step - lo) / a.old_step;
-      if (nl == c) s += lf * old[o];
-      if (nr == c && nl != nr) s += (1.0 - lf) * old[o];
+      const int at = place[o];
+      if (at >> 1 == c) s += share[o] * old[o];
+      else if (at == 2 * c - 1) s += (1.0 - share[o]) * old[o];
     }
     v[(size_t)c * stride] = phase ? old[c] + a.n_phases * s : s;
   }
@@ -1140,7 +1153,7 @@ void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
 }
 
 void launch_rebin(const RebinArgs& a, cudaStream_t s) {
-  k_rebin<<<1 + a.n_cos + a.n_phases, kRebinThreads, 0, s>>>(a);
+  k_rebin<<<1 + a.n_cos + a.n_phases, kRebinThreads, a.n_e * kRebinCell, s>>>(a);
 }
 
 void launch_interval_end(const SampleArgs& a, cudaStream_t s) { launch_after(k_interval_end, 1, 128, 0, s, true, a); }
@@ -1170,6 +1183,8 @@ cudaError_t prepare_kernels() {
     e = cudaFuncSetAttribute(k_hist_b_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistBSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sample_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
+  static_assert(kMaxEnergyCells * kRebinCell <= 227 * 1024, "the cells of a column fit a block");
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rebin, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxEnergyCells * kRebinCell);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sample<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
   if (e == cudaSuccess) e = prepare_advance_stash();
   return e;
