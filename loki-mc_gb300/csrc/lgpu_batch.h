@@ -322,16 +322,25 @@ class Batch {
     m.e->leave_batch();
   }
 
-  // starts waiting members while slots are free
+  // starts waiting members while slots are free, those of one call side by side
   void admit() {
-    while ((int)active_.size() < max_slots_ && next_start_ < end_id()) {
-      Member& m = member(next_start_);
-      m.started = true;
-      const int rc = m.e->solve_begin();
-      if (rc != LGPU_OK) finish(m, rc);
-      else active_.push_back(next_start_);
-      ++next_start_;
-    }
+    std::vector<int> fresh;
+    do {
+      fresh.clear();
+      while ((int)(active_.size() + fresh.size()) < max_slots_ && next_start_ < end_id()) {
+        member(next_start_).started = true;
+        fresh.push_back(next_start_++);
+      }
+      for (int step = 0; step < Engine::kBeginSteps; ++step)
+        for (int idx : fresh) {
+          Member& m = member(idx);
+          if (m.done) continue;
+          const int rc = m.e->solve_begin(step, true);
+          if (rc != LGPU_OK) finish(m, rc);
+        }
+      for (int idx : fresh)
+        if (!member(idx).done) active_.push_back(idx);
+    } while (!fresh.empty());
   }
 
   bool idle() const { return active_.empty() && next_start_ >= end_id(); }
