@@ -263,13 +263,32 @@ __global__ void __launch_bounds__(kPostRateThreads) k_post_rates(EedfPostArgs a,
 // shares: kPostCells cells per block, one node per lane and total per warp (the
 // sum over processes is in their order, as the reference's), then each block's
 // sums over its cells; the last block to finish adds those up in block order.
+//
+// Bound by latency: the loads go out many at a time, the processes' terms of the
+// total ionization and attachment on a lane each, and the roots and powers of the nodes
+// while k_post_rates still runs (1000 cells, 40 processes: with the sums eight loads at
+// a time and everything else behind them the whole call took 60 us, 55 now).
 __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const double* eedf) {
   __shared__ double s_tot[3][kPostCells + 1];
   __shared__ double s_k[2];
+  __shared__ double s_term[2][kMaxProcesses];
+  __shared__ double s_grow[kPostCells + 1];
   __shared__ bool s_last;
   const PostGrid g = post_grid(a);
   const int nc = a.nc, nn = nc + 1, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c0 = blockIdx.x * kPostCells;
+  const double factor = sqrt(2.0 * kQeP / kMeP) / 3.0;
+  // what the grid alone gives
+  if (wid == 0)
+    for (int j = lane; j <= kPostCells; j += 32)
+      s_grow[j] = c0 + j > 0 && c0 + j < nn ? 1.0 / (3.0 * factor * sqrt(g.node(c0 + j))) : 0.0;
+  const int l = c0 + lane;
+  const double x = l < nc ? g.node(l) : 0.0;
+  double pow_x = 0.0, sqrt_x = 0.0;
+  if (wid >= 2 && l >= 1 && l < nc) {
+    pow_x = -2.0 / 3.0 * kQeP / kMeP * pow(x, 1.5);
+    sqrt_x = sqrt(x);
+  }
   wait_for_previous();
   if (wid < 3) {
     for (int j = lane; j <= kPostCells; j += 32) {
@@ -277,30 +296,34 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
       if (i >= nn) break;
       const double* q = a.shares + (size_t)wid * a.P * nn + i;
       double s = 0.0;
-#pragma unroll 8
+#pragma unroll 32
       for (int p = 0; p < a.P; ++p) s = s + q[(size_t)p * nn];
       s_tot[wid][j] = s;
     }
-  } else if (lane < 2) {
+  } else {
     // ionization and attachment rate coefficients of the forward collisions
-    double k = 0.0;
-#pragma unroll 8
-    for (int p = 0; p < a.P; ++p)
-      if (a.kind[p] != 2 && a.ion[p] == lane + 1) k += a.dens[p] * a.rates[p];
-    s_k[lane] = k;
+    for (int p = lane; p < a.P; p += 32) {
+      const int kind = a.kind[p], ion = a.ion[p];
+      const double term = a.dens[p] * a.rates[p];
+      s_term[0][p] = kind != 2 && ion == 1 ? term : 0.0;
+      s_term[1][p] = kind != 2 && ion == 2 ? term : 0.0;
+    }
+    __syncwarp();
+    if (lane < 2) {
+      double k = 0.0;
+      for (int p = 0; p < a.P; ++p) k += s_term[lane][p];
+      s_k[lane] = k;
+    }
   }
   __syncthreads();
-  const double factor = sqrt(2.0 * kQeP / kMeP) / 3.0;
   const double N = a.gas_density, w = a.omega, wc = a.omega_c;
   const double k_ion = s_k[0], k_att = s_k[1], growth = k_ion - k_att;
   auto mta = [&](int j) {  // momentum transfer plus the growth term (BoltzmannMC.C:2233-2234)
-    const int i = c0 + j;
-    return i == 0 ? s_tot[0][j] : s_tot[0][j] + 1.0 / (3.0 * factor * sqrt(g.node(i))) * growth;
+    return c0 + j == 0 ? s_tot[0][j] : s_tot[0][j] + s_grow[j] * growth;
   };
   // the warps share the sums: 0..6 and, of the mobility tensor, xx and xy on
   // one warp, zz on another
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int l = c0 + lane;
   if (l < nc) {
     const double c = g.cell(l), f = eedf[l];
     if (wid == 0) {
@@ -310,13 +333,13 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
       v[4] = c * f / den;
     }
     if (wid > 0 && l >= 1) {
-      const double x = g.node(l), m = mta(lane), df = f - eedf[l - 1];
+      const double m = mta(lane), df = f - eedf[l - 1];
       if (wid == 1) {
         v[0] = x * x * df / m;
         v[1] = x * df / m;
       } else {
-        const double aux1 = -2.0 / 3.0 * kQeP / kMeP * pow(x, 1.5) * df;
-        const double fr = N * m * 3.0 * factor * sqrt(x);
+        const double aux1 = pow_x * df;
+        const double fr = N * m * 3.0 * factor * sqrt_x;
         const double f2 = fr * fr;
         if (wid == 2) {
           const double aux2 = (f2 + (w - wc) * (w - wc)) * (f2 + (w + wc) * (w + wc));
@@ -352,7 +375,7 @@ __global__ void __launch_bounds__(128) k_post_params(EedfPostArgs a, const doubl
   __shared__ double s_sum[kPostSums];
   if (threadIdx.x < kPostSums) {
     double s = 0.0;
-#pragma unroll 8
+#pragma unroll 32
     for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(&a.sums[(size_t)b * kPostSums + threadIdx.x]);
     s_sum[threadIdx.x] = s;
   }
