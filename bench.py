@@ -8,8 +8,8 @@ at 4.4 eV; 200-point log grids over 1e-3..1e4 eV), N = 3.22e22 m^-3, cold gas, u
 (seeded log-uniform 1e4..2e6, 1.98e7 in all), FP32 push with FP64 tallies.
 Three forms of the same work are measured:
 
-* batched: all 64 conditions in one lgpu_batch - one launch sequence (CUDA
-  graph) per synchronisation interval advances every condition;
+* batched: all 64 conditions in one lgpu_batch - one launch sequence per
+  synchronisation interval advances every condition;
 * plain: one condition per launch sequence (lgpu_solve / lgpu_advance), the
   drop-in path, one condition after the other;
 * served: the 64 conditions submitted to lgpu_server with Poisson arrivals,

@@ -280,8 +280,8 @@ int lgpu_replay_flights_noalloc(int device, const double e_field[3], double freq
  * (lokimc.C:78-80); a sweep there is one run per setup. A batch solves many
  * contexts together: each context keeps its own ensemble, tables, tallies and
  * host control flow (the steps of lgpu_solve, BoltzmannMC.C:299-426), while
- * each synchronisation interval of all of them is one launch sequence (a CUDA
- * graph) over every context's electrons. Contexts are created on the batch's
+ * each synchronisation interval of all of them is one launch sequence over
+ * every context's electrons. Contexts are created on the batch's
  * device with processes and conditions set, and may differ in everything
  * (mixture, field, electron count, numerics). When more contexts are added
  * than the batch has slots, the rest start as running ones finish. After

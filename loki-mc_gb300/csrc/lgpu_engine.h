@@ -977,7 +977,7 @@ class Engine {
   // a look by the host in between (PlainCtl), each followed by its part of the
   // solve loop (solving) or a sample. *ran: the intervals run, at least one.
   //
-  // A look per interval (graph launch, copies of control block and scalars, wait)
+  // A look per interval (launches, copies of control block and scalars, wait)
   // cost 11-17 us of each: 10,000 atomic-gas electrons 53 -> 37 us per interval,
   // 200,000 under AC 84 -> 66, 1e6 N2-like 135 -> 124.
   int run_chain(int want, bool solving, int* ran) {

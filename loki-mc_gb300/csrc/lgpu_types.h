@@ -109,7 +109,7 @@ struct Consts {
 };
 
 // Per-interval parameters, written by the host into device memory before each
-// synchronisation interval so that one captured CUDA graph serves every interval.
+// chain of synchronisation intervals and by the device from one interval to the next.
 struct IntervalCtl {
   float dt_sync;          // interval length (s)
   float phi0;             // phase at the interval start (rad), reduced in FP64 on the host
