@@ -24,8 +24,8 @@ namespace lgpu {
 namespace {
 
 // the main pass over the ensemble
-template <int MODE>
-__global__ void __launch_bounds__(kAdvanceThreads, kAdvanceBlocksPerSM) k_advance(const __grid_constant__ AdvanceArgs a) {
+template <int MODE, int BLOCKS_PER_SM>
+__global__ void __launch_bounds__(kAdvanceThreads, BLOCKS_PER_SM) k_advance(const __grid_constant__ AdvanceArgs a) {
   __shared__ AdvShared sh;
   advance_body<MODE>(a, sh);
 }
@@ -1087,6 +1087,24 @@ __global__ void k_replay_collide(ReplayCollArgs a) {
   a.used[i] = rng.pos;
 }
 
+template <int BLOCKS_PER_SM>
+void launch_advance_modes(const AdvanceArgs& args, cudaStream_t s) {
+  AdvanceArgs a = args;
+  // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
+  const int threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
+  const int warps = threads / 32, per_sm = BLOCKS_PER_SM * kAdvanceThreads / threads;
+  const int grid = max(1, min(a.sm_count * per_sm, (a.n + threads - 1) / threads));
+  const int all = grid * warps;
+  a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
+  switch (a.field.mode) {
+    case kFieldDC: launch_after(k_advance<kFieldDC, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+    case kFieldAC: launch_after(k_advance<kFieldAC, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+    case kFieldB: launch_after(k_advance<kFieldB, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+    case kFieldECR: launch_after(k_advance<kFieldECR, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+    default: launch_after(k_advance<kFieldACB, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+  }
+}
+
 inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; }
 
 }  // namespace
@@ -1101,21 +1119,17 @@ inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; 
 // (mixture, crossed B, thermal) 58 -> 38, 1e6 (N2-like) 85 -> 74, 4e6 unchanged
 // at 194. The collision stash of the batched shapes waits for 32 collisions at the
 // end of every condition and is no faster here (79 us at 1e6, 194 at 4e6).
-void launch_advance(const AdvanceArgs& args, cudaStream_t s) {
-  AdvanceArgs a = args;
-  // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
-  const int threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
-  const int warps = threads / 32, per_sm = kAdvanceBlocksPerSM * kAdvanceThreads / threads;
-  const int grid = max(1, min(a.sm_count * per_sm, (a.n + threads - 1) / threads));
-  const int all = grid * warps;
-  a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
-  switch (a.field.mode) {
-    case kFieldDC: launch_after(k_advance<kFieldDC>, grid, threads, 0, s, true, a); break;
-    case kFieldAC: launch_after(k_advance<kFieldAC>, grid, threads, 0, s, true, a); break;
-    case kFieldB: launch_after(k_advance<kFieldB>, grid, threads, 0, s, true, a); break;
-    case kFieldECR: launch_after(k_advance<kFieldECR>, grid, threads, 0, s, true, a); break;
-    default: launch_after(k_advance<kFieldACB>, grid, threads, 0, s, true, a); break;
-  }
+//
+// While one electron per lane needs fewer lanes than four blocks per SM hold, two or
+// three blocks hold them all, with the registers of the others: no spills, and more
+// of an electron's chain of loads and divisions side by side. 10,000 electrons (atomic
+// gas) 15.4 -> 14.5 us, 33,333 (Reid) 10.8 -> 10.0 by the device's clock with two;
+// 100,000 (mixture, crossed B, thermal) 31.7 -> 30.3 with three.
+void launch_advance(const AdvanceArgs& a, cudaStream_t s) {
+  const int lanes = a.sm_count * kAdvanceThreads;  // of one block per SM
+  if (a.n <= 2 * lanes) launch_advance_modes<2>(a, s);
+  else if (a.n <= 3 * lanes) launch_advance_modes<3>(a, s);
+  else launch_advance_modes<kAdvanceBlocksPerSM>(a, s);
 }
 
 void launch_init(const InitArgs& a, cudaStream_t s) {
