@@ -13,10 +13,9 @@
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 
-#include <cstddef>
-
 #include "lgpu_advance.cuh"
 #include "lgpu_device.cuh"
+#include "lgpu_interval_end.h"
 #include "lgpu_kernels.cuh"
 
 namespace lgpu {
@@ -324,51 +323,24 @@ __device__ __forceinline__ void hist_cells(const HistArgs& a, float4 B, int& c, 
   }
 }
 
-// The end of an interval of one condition with n electrons (every thread of one
-// block calls this; all other work of the interval is done): its scalars go to the
-// host (out[pos * stride]), the ones of one interval are cleared, and the next
-// interval of the chain is set up or the chain stopped.
-__device__ __forceinline__ void end_interval(IntervalCtl& ctl, DistCtl& dist, ChainCtl& ch, DevScalars* sc, int n,
-                                             DevScalars* out, int stride, int* done, bool sampled) {
-  const int pos = ch.pos;
-  constexpr int kWords = (int)(sizeof(DevScalars) / sizeof(int));
-  const int* src = reinterpret_cast<const int*>(sc);
-  int* dst = reinterpret_cast<int*>(&out[(size_t)pos * stride]);
-  for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = __ldcg(&src[k]);
-  if (threadIdx.x == 0) {
-    const float e = __uint_as_float(__ldcg(&sc->sample_max_bits));
-    const bool counted = !dist.on || __uint_as_float(__ldcg(&sc->max_energy_bits)) <= dist.e_bound;
-    const bool go = sampled && pos + 1 < ch.n && counted && e >= ch.e_lo && e <= ch.e_hi &&
-                    __ldcg(&sc->error_flag) == 0 && __ldcg(&sc->sec_count) <= ch.sec_stop;
-    if (go) {
-      // the host's arithmetic: the FP64 mean, rounded to FP32
-      ctl.shift_x = (float)(__ldcg(&sc->moments[1]) / (double)n);
-      ctl.shift_y = (float)(__ldcg(&sc->moments[2]) / (double)n);
-      ctl.shift_z = (float)(__ldcg(&sc->moments[3]) / (double)n);
-      ctl.phi0 = ch.phi0[pos + 1];
-      ++ctl.interval;
-      dist.h.eedf_periodic_row = ch.row[pos + 1];
-      ch.pos = pos + 1;
-    } else {
-      ctl.go = 0;
-    }
-    *done = pos + 1;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < (int)(offsetof(DevScalars, null_count) / sizeof(int)); k += blockDim.x)
-    reinterpret_cast<int*>(sc)[k] = 0;
-  if (threadIdx.x < kMoments) sc->moments[threadIdx.x] = 0.0;
-  if (threadIdx.x == 0) sc->sample_max_bits = 0u;
-}
+// the calling block, for end_interval
+struct ThisBlock {
+  __device__ __forceinline__ int thread() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ int threads() const { return (int)blockDim.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+  template <class T>
+  __device__ __forceinline__ T load(const T* p) const { return __ldcg(p); }
+};
 
 __device__ __forceinline__ void end_plain_interval(const SampleArgs& a, bool sampled) {
-  end_interval(a.plain->ctl, a.plain->dist, a.plain->chain, a.sc, a.n, a.out->sc, 1, &a.out->done, sampled);
+  end_interval(ThisBlock(), a.plain->ctl, a.plain->dist, a.plain->chain, a.sc, a.n, a.out->sc, 1, &a.out->done, nullptr,
+               sampled);
 }
 
 __global__ void k_interval_end(SampleArgs a) {
   next_may_start();
   wait_for_previous();
-  if (a.plain->ctl.go) end_plain_interval(a, false);
+  end_plain_interval(a, false);
 }
 
 // The cells a block counts in shared memory (16-bit, two per word: a block sees fewer
@@ -1019,10 +991,8 @@ __global__ void __launch_bounds__(kBatchEndThreads) k_batch_end(BatchArgs b) {
     h.advance_end = 0ull;
   }
   BatchSlot& sl = b.slots[s];
-  if (!sl.ctl.go) return;
-  end_interval(sl.ctl, sl.dist, sl.chain, sl.sc, sl.adv.n, b.gather + s, b.max_slots, &b.out->done[s],
-               (sl.flags & kSlotSample) != 0);
-  if (threadIdx.x == 0 && !sl.ctl.go) b.out->stopped = 1;
+  end_interval(ThisBlock(), sl.ctl, sl.dist, sl.chain, sl.sc, sl.adv.n, b.gather + s, b.max_slots, &b.out->done[s],
+               &b.out->stopped, (sl.flags & kSlotSample) != 0);
 }
 
 // --------------------------------------------------------------- replay
