@@ -467,7 +467,9 @@ int lgpu_server_job_rates(lgpu_server* server, long long job_id, unsigned long l
  * parameters and each process's EEDF-convolved rate coefficient, computed on
  * the device at the job's end. LGPU_ERR_STATE for other jobs. */
 int lgpu_server_job_eedf(lgpu_server* server, long long job_id, lgpu_eedf_params* params, double* rate, int n);
-/* A queued job is dropped; a running one stops at its next interval. */
+/* A queued job is dropped; a running one stops after the intervals that are
+ * launched already (the running one and at most one more). Jobs that arrive
+ * while others run are admitted then, too. */
 int lgpu_server_cancel(lgpu_server* server, long long job_id);
 /* Drops the record of a finished (done, failed or cancelled) job: its status,
  * results and rates are no longer available (LGPU_ERR_STATE for a job still

@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <chrono>
 #include <array>
+#include <atomic>
 #include <deque>
 #include <mutex>
 #include <map>
@@ -359,8 +360,11 @@ class Batch {
   // Up to `most` synchronisation intervals of every running member (*ran: how many
   // were launched). Members whose stop criteria hold (or that fail) finish here;
   // *finished lists them. A member whose energy grid is being re-built (on its own
-  // stream, concurrently) sits the chain out and goes on at the next step.
-  int step(int most = kBatchChain, int* ran = nullptr, std::vector<int>* finished = nullptr) {
+  // stream, concurrently) sits the chain out and goes on at the next step. Once *look is
+  // set no further interval is launched: the running one and the one behind it end the
+  // chain.
+  int step(int most = kBatchChain, int* ran = nullptr, std::vector<int>* finished = nullptr,
+           const std::atomic<bool>* look = nullptr) {
     if (ran) *ran = 1;
     const auto h0 = std::chrono::steady_clock::now();
     // the samples left to count first: the host work below (stop criteria, trial
@@ -509,7 +513,7 @@ class Batch {
     const auto h1 = std::chrono::steady_clock::now();
     for (int s = 0, idle = 0; chain > 1;) {
       const int running = __atomic_load_n(&h_out_->published, __ATOMIC_ACQUIRE);
-      const bool more = launched < chain && !*(volatile int*)&h_out_->stopped &&
+      const bool more = launched < chain && !*(volatile int*)&h_out_->stopped && !(look && *look) &&
                         std::chrono::steady_clock::now() - h1 < std::chrono::milliseconds(20);
       if (more && running + 2 > launched) {
         kernels += enqueue_interval(n, parts, shape, false);

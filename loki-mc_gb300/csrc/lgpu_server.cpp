@@ -16,6 +16,7 @@
 // owns every CUDA call.
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <condition_variable>
 #include <deque>
 #include <map>
@@ -78,6 +79,9 @@ class Server {
   std::deque<long long> finished_;
   long long running_count_ = 0;
   bool stop_ = false;
+  // set (mutex held) when a job arrives, is cancelled or the server stops: no further
+  // interval of the running chain is launched
+  std::atomic<bool> look_{false};
   long long next_id_ = 1;
   long long submitted_ = 0, completed_ = 0, failed_ = 0, intervals_ = 0;
   double real_ = 0, null_ = 0, busy_ = 0;
@@ -160,6 +164,7 @@ class Server {
     queue_.push_back(r->id);
     jobs_[r->id] = std::move(r);
     ++submitted_;
+    look_ = true;
     cv_work_.notify_one();
     return LGPU_OK;
   }
@@ -243,6 +248,7 @@ class Server {
       cv_done_.notify_all();
     } else if (r.state == LGPU_JOB_RUNNING) {
       r.cancel = true;
+      look_ = true;
     }
     return LGPU_OK;
   }
@@ -266,6 +272,7 @@ class Server {
     {
       std::lock_guard<std::mutex> lock(mu_);
       stop_ = true;
+      look_ = true;
       cv_work_.notify_all();
     }
     if (worker_.joinable()) worker_.join();
@@ -350,6 +357,7 @@ class Server {
         std::unique_lock<std::mutex> lock(mu_);
         cv_work_.wait(lock, [&] { return stop_ || !running_.empty() || !queue_.empty(); });
         if (stop_) break;
+        look_ = false;
         while (!queue_.empty() && (int)(running_.size() + admit.size()) < max_slots_) {
           JobRec* r = jobs_[queue_.front()].get();
           if (held_ + r->footprint > budget_) {
@@ -384,7 +392,7 @@ class Server {
           running_.push_back(r);
         }
       }
-      // ---- cancellations between intervals
+      // ---- cancellations
       {
         std::vector<JobRec*> cancelled;
         {
@@ -401,9 +409,9 @@ class Server {
         }
       }
       if (running_.empty()) continue;
-      // ---- one interval of every running job
+      // ---- a chain of intervals of every running job
       std::vector<int> finished;
-      const int rc = batch_.step(kBatchChain, nullptr, &finished);
+      const int rc = batch_.step(kBatchChain, nullptr, &finished, &look_);
       if (rc != LGPU_OK) {
         // the launch sequence itself failed: every running job fails with it
         for (JobRec* r : running_) {
