@@ -58,6 +58,7 @@ class Batch {
   std::vector<int> n_, seen_, rc_;  // seen_, rc_: a slot's intervals the host has worked through, and how
   std::vector<unsigned char> take_, all_;
   std::vector<std::pair<int, int>> rem_;
+  double interval_ms_ = 0;  // wall time of an interval of the last chain
   // totals since creation
   long long intervals_ = 0, launches_ = 0;
   double adv_ms_ = 0, electron_steps_ = 0, h2d_bytes_ = 0, d2h_bytes_ = 0;
@@ -448,7 +449,7 @@ class Batch {
     for (int s = 0; s < n; ++s) {
       Engine* e = member(go[s]).e;
       if (!e->sampling_ || (sampled < kBatchDistMin && e->sample_moments_only())) chain = 1;
-      if (chain > 1) chain = e->chain_limit(chain, true);
+      if (chain > 1) chain = e->chain_limit(chain, true, interval_ms_);
     }
     BatchSlot* d_sl = reinterpret_cast<BatchSlot*>(d_stage_ + batch_slots_offset());
     int rc, kernels = 0;
@@ -537,6 +538,7 @@ class Batch {
     if (intervals < 1 || intervals > chain)
       return fail(LGPU_ERR_STATE, "a chain of " + std::to_string(chain) + " batched intervals ran " + std::to_string(intervals));
     if (ran) *ran = intervals;
+    interval_ms_ = 1e3 * std::chrono::duration<double>(h2 - h0).count() / intervals;
     double ms = 0;
     for (int k = 0; k < intervals; ++k) ms += 1e-6 * h_out_->advance_ns[k];
     adv_ms_ += ms;

@@ -914,9 +914,10 @@ class Engine {
   }
 
   // How many intervals may follow one another before the host has to look: up to a
-  // steady-state or error check (solve_post), a stop criterion (solve_next) or the
-  // cap on steps.
-  int chain_limit(int want, bool solving) const {
+  // steady-state or error check (solve_post), a stop criterion (solve_next) or a cap.
+  // interval_ms: what one took lately (0: not known, and a cap on time is looked at
+  // after each).
+  int chain_limit(int want, bool solving, double interval_ms) const {
     int n = std::min(want, kChain);
     if (!solving) return n;
     if (cfg_.sync_oversampling != 1) return 1;
@@ -924,6 +925,10 @@ class Engine {
     // a stop criterion on the count of collisions may hold after any interval
     if (ss && cfg_.max_coll_after_ss * N_ < 1e18) return 1;
     if (cfg_.max_sync_steps > 0) n = (int)std::min<long long>(n, std::max<long long>(1, cfg_.max_sync_steps - solve_steps_));
+    if (cfg_.max_seconds > 0) {
+      const double fit = interval_ms > 0 ? 1e3 * (cfg_.max_seconds - solve_seconds()) / interval_ms : 0.0;
+      if (fit < n) n = std::max(1, (int)fit);
+    }
     double t = time_;
     for (int i = 1; i < n; ++i) {
       t += pending_dt_;
@@ -988,7 +993,7 @@ class Engine {
     // short at first and after one that stopped early, whose launches left were for
     // nothing, and a few milliseconds at most
     const int cap = interval_ms_ > 0 ? std::max(1, (int)(5.0 / interval_ms_)) : kChain;
-    const int n = sample ? chain_limit(std::min({want, cap, chain_len_}), solving) : 1;
+    const int n = sample ? chain_limit(std::min({want, cap, chain_len_}), solving, interval_ms_) : 1;
     fill_chain(&h_plain_->chain, n);
     h_plain_->ticket = 0;
     LGPU_CU(copy(d_plain_, h_plain_, sizeof(PlainCtl), cudaMemcpyHostToDevice));
@@ -1337,6 +1342,10 @@ class Engine {
     }
   }
 
+  double solve_seconds() const {
+    return std::chrono::duration<double>(std::chrono::steady_clock::now() - solve_t0_).count();
+  }
+
   // *done when a stop criterion holds (BoltzmannMC.C:311-316) or a cap is hit;
   // otherwise sampling_ says whether the next interval ends with a sample
   // (BoltzmannMC.C:311-316) with n_int integration points over int_time
@@ -1355,7 +1364,8 @@ class Engine {
     return n_int > 200 && n_int % (long long)std::pow(2, dec) == 0 && cfg_.errors_checked;
   }
 
-  // (within a chain of intervals the caps wait for its end)
+  // (within a chain of intervals the caps wait for its end, which chain_limit puts
+  // where they may hold)
   int solve_next(bool* done, bool within = false) {
     *done = false;
     if (!wants_more(n_int_, total_int_time_)) {
@@ -1369,8 +1379,7 @@ class Engine {
         return LGPU_OK;
       }
     }
-    const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - solve_t0_).count();
-    if (!within && ((cfg_.max_seconds > 0 && el > cfg_.max_seconds) ||
+    if (!within && ((cfg_.max_seconds > 0 && solve_seconds() > cfg_.max_seconds) ||
                     (cfg_.max_sync_steps > 0 && solve_steps_ >= cfg_.max_sync_steps))) {
       solve_capped_ = 1;
       *done = true;
@@ -1407,7 +1416,7 @@ class Engine {
     finals(r);
     r->capped = solve_capped_;
     r->sync_steps = solve_steps_;
-    r->elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - solve_t0_).count();
+    r->elapsed = solve_seconds();
     solved_ = true;
     return LGPU_OK;
   }
