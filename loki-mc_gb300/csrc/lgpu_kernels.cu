@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(kHistAThreads) k_hist_a_batch(BatchArgs b) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
     const ChunkRef k = pass_chunk(b.hist_prefix, b.hist_part, n_slots, n_full, b.hdr->hist_chunk, c);
-    const HistArgs& a = b.slots[k.slot].hist;
+    const HistArgs& a = b.hists[k.slot];
     hist_chunk_a(a, k.first, min(k.first + b.hdr->hist_chunk, a.n), sm_hist, kHistASmem / 4);
   }
 }
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b_batch(BatchArgs b) {
     const int c = snake_chunk(r);
     if (c >= total) continue;
     const ChunkRef k = pass_chunk(b.hist2_prefix, b.hist2_part, n_slots, n_full, b.hdr->hist_chunk, c);
-    const HistArgs& a = b.slots[k.slot].hist;
+    const HistArgs& a = b.hists[k.slot];
     hist_chunk_b(a, k.first, min(k.first + b.hdr->hist_chunk, a.n), sm_hist, kHistBSmem / 4);
   }
 }

@@ -270,7 +270,6 @@ struct BatchSlot {
   AdvanceArgs adv;        // adv.ctl points at this slot's ctl (the device's copy)
   PopArgs pop;
   SampleArgs smp;
-  HistArgs hist;          // distribution staging only: the deferred tallies of a previous sample
   DistCtl dist;           // distributions counted with this interval's sample
   IntervalCtl ctl;        // this interval's values
   ChainCtl chain;
@@ -326,10 +325,12 @@ constexpr double kBatchDistMin = 150000;
 //   BatchHeader | adv_prefix | smp_prefix | hist_prefix | hist2_prefix (kBatchMaxSlots+1 ints
 //   each) | smp_part | hist_part | hist2_part (kBatchMaxSlots ints each, padded) | BatchSlot[...]
 // The interval's staging fills the advance and moment parts, the distribution
-// passes' staging (same layout) the hist parts and each slot's `hist`.
+// passes' staging the hist parts and, in place of the slots, the deferred tallies of a
+// previous sample (HistArgs[...]).
 struct BatchArgs {
   BatchHeader* hdr;
   BatchSlot* slots;
+  const HistArgs* hists;    // (distribution passes)
   const int* adv_prefix;
   const int* smp_prefix;    // full chunks before each slot
   const int* hist_prefix;   // energy and energy-angle distributions
@@ -347,9 +348,8 @@ static_assert(kBatchMaxSlots == 1024 && kBatchChain <= kChain, "BatchOut, ChainC
 // One batched interval is two launch groups on one stream:
 //   advance: one persistent launch per field mode
 //   post:    spilled secondaries and population control, samples, the interval's end
-// ahead of a chain of them, from a second staging area of the same layout, the
-// distribution passes of the previous interval's samples (`hist` of each
-// slot), launched before the host prepares the interval so that its work
+// ahead of a chain of them, from a second staging area, the distribution passes of the
+// previous interval's samples, launched before the host prepares the interval so that its work
 // runs beside them.
 // `parts` leaves out the launches no slot of the interval needs: bit m (m <
 // kFieldModes) for field mode m, then the flags below. Each returns the
