@@ -778,11 +778,12 @@ class Engine {
   // The device work of one interval: the advance of every electron and of the
   // secondaries they create, any secondary its warps could not queue and population
   // control (when the mixture ionizes or attaches), the ensemble sample and the end
-  // of the interval (k_sample, or k_interval_end without a sample).
-  void enqueue_interval(bool sample) {
-    launch_advance(chain_adv_, stream_);
+  // of the interval (k_sample, or k_interval_end without a sample). The first one of a
+  // chain follows copies, not a kernel: its advance starts when they are done.
+  void enqueue_interval(bool sample, bool first_of_chain) {
+    launch_advance(chain_adv_, !first_of_chain, stream_);
     if (have_ion_att_) launch_pop_control(chain_adv_, chain_pop_, stream_);
-    if (sample) launch_sample(chain_smp_, sm_count_, stream_);
+    if (sample) launch_sample(chain_smp_, sm_count_, true, stream_);
     else launch_interval_end(chain_smp_, stream_);
     launches_ += 2 + (have_ion_att_ ? kPopLaunches : 0);
   }
@@ -1010,7 +1011,7 @@ class Engine {
       chain_smp_.dist_e_cells = cfg_.n_energy_cells;
       chain_built_ = true;
     }
-    for (int k = 0; k < n; ++k) enqueue_interval(sample);
+    for (int k = 0; k < n; ++k) enqueue_interval(sample, k == 0);
     scalars_clear_ = true;
     LGPU_TRY(sync("interval"));
     const int done = *(volatile int*)&h_out_->done;
@@ -1054,7 +1055,7 @@ class Engine {
   int launch_moments() {
     LGPU_CU(cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_));
     LGPU_CU(cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_));
-    launch_sample(sample_args(), sm_count_, stream_);
+    launch_sample(sample_args(), sm_count_, false, stream_);
     ++launches_;
     LGPU_CU(copy(h_sc_, d_sc_, sizeof(DevScalars), cudaMemcpyDeviceToHost));
     return LGPU_OK;

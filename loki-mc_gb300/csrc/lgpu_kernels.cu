@@ -1058,7 +1058,7 @@ __global__ void k_replay_collide(ReplayCollArgs a) {
 }
 
 template <int BLOCKS_PER_SM>
-void launch_advance_modes(const AdvanceArgs& args, cudaStream_t s) {
+void launch_advance_modes(const AdvanceArgs& args, bool after_kernel, cudaStream_t s) {
   AdvanceArgs a = args;
   // blocks of two warps while that puts at most four warps on an SM: 24 -> 22.5 us at 10,000
   const int threads = a.n <= a.sm_count * 4 * 32 ? 64 : kAdvanceThreads;
@@ -1067,11 +1067,11 @@ void launch_advance_modes(const AdvanceArgs& args, cudaStream_t s) {
   const int all = grid * warps;
   a.share = a.n <= all * 32 ? 32 : (int)(0.8 * a.n / all) / 32 * 32;
   switch (a.field.mode) {
-    case kFieldDC: launch_after(k_advance<kFieldDC, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
-    case kFieldAC: launch_after(k_advance<kFieldAC, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
-    case kFieldB: launch_after(k_advance<kFieldB, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
-    case kFieldECR: launch_after(k_advance<kFieldECR, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
-    default: launch_after(k_advance<kFieldACB, BLOCKS_PER_SM>, grid, threads, 0, s, true, a); break;
+    case kFieldDC: launch_after(k_advance<kFieldDC, BLOCKS_PER_SM>, grid, threads, 0, s, after_kernel, a); break;
+    case kFieldAC: launch_after(k_advance<kFieldAC, BLOCKS_PER_SM>, grid, threads, 0, s, after_kernel, a); break;
+    case kFieldB: launch_after(k_advance<kFieldB, BLOCKS_PER_SM>, grid, threads, 0, s, after_kernel, a); break;
+    case kFieldECR: launch_after(k_advance<kFieldECR, BLOCKS_PER_SM>, grid, threads, 0, s, after_kernel, a); break;
+    default: launch_after(k_advance<kFieldACB, BLOCKS_PER_SM>, grid, threads, 0, s, after_kernel, a); break;
   }
 }
 
@@ -1095,11 +1095,11 @@ inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; 
 // of an electron's chain of loads and divisions side by side. 10,000 electrons (atomic
 // gas) 15.4 -> 14.5 us, 33,333 (Reid) 10.8 -> 10.0 by the device's clock with two;
 // 100,000 (mixture, crossed B, thermal) 31.7 -> 30.3 with three.
-void launch_advance(const AdvanceArgs& a, cudaStream_t s) {
+void launch_advance(const AdvanceArgs& a, bool after_kernel, cudaStream_t s) {
   const int lanes = a.sm_count * kAdvanceThreads;  // of one block per SM
-  if (a.n <= 2 * lanes) launch_advance_modes<2>(a, s);
-  else if (a.n <= 3 * lanes) launch_advance_modes<3>(a, s);
-  else launch_advance_modes<kAdvanceBlocksPerSM>(a, s);
+  if (a.n <= 2 * lanes) launch_advance_modes<2>(a, after_kernel, s);
+  else if (a.n <= 3 * lanes) launch_advance_modes<3>(a, after_kernel, s);
+  else launch_advance_modes<kAdvanceBlocksPerSM>(a, after_kernel, s);
 }
 
 void launch_init(const InitArgs& a, cudaStream_t s) {
@@ -1123,17 +1123,19 @@ void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
 // AC 17.4 -> 28).
 constexpr int kSampleShared = 600000;
 
-void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s) {
+void launch_sample(const SampleArgs& a, int sm_count, bool after_kernel, cudaStream_t s) {
   if (a.n <= 0) return;
   const int sms = max(1, sm_count);
   const bool shared = a.plain && a.n >= kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
   if (shared) {
-    launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s, true, a);
+    launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s,
+                 after_kernel, a);
     return;
   }
   const int threads = a.n < sms * kSampleThreads ? kSampleThreads / 2 : kSampleThreads;
   const int grid = min(blocks_for(a.n, threads), sms * (1024 / threads));
-  launch_after(k_sample<false>, grid, threads, a.plain ? a.dist_e_cells * sizeof(unsigned int) : 0, s, true, a);
+  launch_after(k_sample<false>, grid, threads, a.plain ? a.dist_e_cells * sizeof(unsigned int) : 0, s, after_kernel,
+               a);
 }
 
 void launch_rebin(const RebinArgs& a, cudaStream_t s) {

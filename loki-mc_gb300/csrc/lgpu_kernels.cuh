@@ -93,7 +93,8 @@ struct AdvanceArgs {
 // turn: 20 (1e6, mixture under crossed B: 95 us, 99 with 16, 94 with 24).
 constexpr int kRealBatchCold = 16, kRealBatchThermal = 20;
 
-void launch_advance(const AdvanceArgs& a, cudaStream_t s);
+// after_kernel: as launch_after's
+void launch_advance(const AdvanceArgs& a, bool after_kernel, cudaStream_t s);
 
 // Per-process kernel attributes (dynamic shared memory of the histogram
 // kernels); called on the current device before any launch or capture.
@@ -224,10 +225,10 @@ struct SampleArgs {
   ChainOut* out;
   int dist_e_cells;                // EEDF cells (with plain)
 };
-// the end of an interval without a sample
+// the end of an interval without a sample, behind its other kernels
 void launch_interval_end(const SampleArgs& a, cudaStream_t s);
 // grid: at most four blocks per SM (sm_count = the device's multiprocessors)
-void launch_sample(const SampleArgs& a, int sm_count, cudaStream_t s);
+void launch_sample(const SampleArgs& a, int sm_count, bool after_kernel, cudaStream_t s);
 
 void launch_hist(const HistArgs& a, cudaStream_t s);
 
