@@ -252,6 +252,14 @@ int lgpu_replay_collisions(lgpu_ctx* ctx, int n, const double* nu_trial, const d
 int lgpu_replay_collisions_coarse(lgpu_ctx* ctx, int n, const double* nu_trial, const double* vel,
                                   const double* energy, const double* uniforms, int u_stride, double* out, int* used);
 
+/* The re-binning of the tallies on the energy grid when an electron outgrows it
+ * (BoltzmannMC.C:1495-1548), in place: n_cells EEDF sums, the EADF's [n_cells x n_cos]
+ * (n_cos 0: none) and the per-phase EEDFs' [n_phases x n_cells] (0: none), from a grid
+ * up to old_max to one of as many cells up to new_max > old_max. At most 4096 cells and
+ * 65536 angles and phases. */
+int lgpu_replay_rebin(lgpu_ctx* ctx, int n_cells, int n_cos, int n_phases, double old_max, double new_max,
+                      double* eedf, double* eadf, double* eedf_per);
+
 /* ---- free flights without device allocation ----
  *
  * No counterpart in the reference. For callers that cannot allocate device

@@ -1968,6 +1968,32 @@ class Engine {
     return sync("replay_collisions");
   }
 
+  int replay_rebin(int n_e, int n_cos, int n_phases, double old_max, double new_max, double* eedf, double* eadf,
+                   double* eedf_per) {
+    const size_t ne = (size_t)n_e, na = ne * n_cos, np = ne * n_phases;
+    LGPU_TRY(rp_reserve(ne + na + np, 0));
+    RebinArgs a{};
+    a.n_e = n_e;
+    a.n_cos = n_cos;
+    a.n_phases = n_phases;
+    a.old_max = old_max;
+    a.old_step = old_max / n_e;
+    a.step = new_max / n_e;
+    a.eedf = d_rp_in_;
+    a.eadf = a.eedf + ne;
+    a.eedf_per = a.eadf + na;
+    LGPU_CU(copy(a.eedf, eedf, ne * sizeof(double), cudaMemcpyHostToDevice));
+    if (na) LGPU_CU(copy(a.eadf, eadf, na * sizeof(double), cudaMemcpyHostToDevice));
+    if (np) LGPU_CU(copy(a.eedf_per, eedf_per, np * sizeof(double), cudaMemcpyHostToDevice));
+    launch_rebin(a, stream_);
+    ++launches_;
+    LGPU_CU(cudaGetLastError());
+    LGPU_CU(copy(eedf, a.eedf, ne * sizeof(double), cudaMemcpyDeviceToHost));
+    if (na) LGPU_CU(copy(eadf, a.eadf, na * sizeof(double), cudaMemcpyDeviceToHost));
+    if (np) LGPU_CU(copy(eedf_per, a.eedf_per, np * sizeof(double), cudaMemcpyDeviceToHost));
+    return sync("replay_rebin");
+  }
+
   int tables_out(double max_energy, double* nu_tot, double* nu_max, float* sig, float* cum) {
     if (!have_procs_ || !(Ngas_ > 0)) return fail(LGPU_ERR_STATE, "set_processes and set_conditions come first");
     max_interp_ = -1.0;

@@ -28,7 +28,7 @@ EXPORTED = ("lgpu_config_default", "lgpu_create", "lgpu_destroy", "lgpu_last_err
             "lgpu_get_process_results", "lgpu_get_distributions", "lgpu_get_periodic", "lgpu_get_series",
             "lgpu_get_timing", "lgpu_set_twoterm", "lgpu_eedf_postprocess", "lgpu_eedf_rates",
             "lgpu_build_tables", "lgpu_set_field_raw", "lgpu_replay_flights", "lgpu_replay_collisions",
-            "lgpu_replay_collisions_coarse", "lgpu_replay_flights_noalloc",
+            "lgpu_replay_collisions_coarse", "lgpu_replay_rebin", "lgpu_replay_flights_noalloc",
             "lgpu_batch_create", "lgpu_batch_destroy", "lgpu_batch_last_error", "lgpu_batch_add", "lgpu_batch_run",
             "lgpu_batch_start", "lgpu_batch_step", "lgpu_batch_stream", "lgpu_batch_set_schedule",
             "lgpu_server_start", "lgpu_server_submit", "lgpu_server_poll", "lgpu_server_wait",
@@ -207,6 +207,7 @@ def load(path: str | None = None):
     lib.lgpu_replay_flights.argtypes = [ctypes.c_void_p, I] + [P_(D)] * 8
     lib.lgpu_replay_collisions.argtypes = [ctypes.c_void_p, I, P_(D), P_(D), P_(D), P_(D), I, P_(D), P_(I)]
     lib.lgpu_replay_collisions_coarse.argtypes = lib.lgpu_replay_collisions.argtypes
+    lib.lgpu_replay_rebin.argtypes = [ctypes.c_void_p, I, I, I, D, D, P_(D), P_(D), P_(D)]
     lib.lgpu_replay_flights_noalloc.argtypes = [I, P_(D), D, D, D, I] + [P_(D)] * 8
     VP = ctypes.c_void_p
     lib.lgpu_batch_create.argtypes = [I, I, P_(VP)]
@@ -496,6 +497,15 @@ class Context:
         self.check(fn(self.h, n, dptr(nu), dptr(vel), dptr(energy), dptr(u), u.shape[1], dptr(out),
                       used.ctypes.data_as(P_(I))))
         return out, used
+
+    def replay_rebin(self, old_max, new_max, eedf, eadf=None, eedf_per=None):
+        """lgpu_replay_rebin on copies: (eedf, eadf, eedf_per), absent ones None."""
+        out = [None if a is None else np.array(a, np.float64, order="C") for a in (eedf, eadf, eedf_per)]
+        n_cos = 0 if eadf is None else out[1].shape[1]
+        n_ph = 0 if eedf_per is None else out[2].shape[0]
+        self.check(self.lib.lgpu_replay_rebin(self.h, len(out[0]), n_cos, n_ph, float(old_max), float(new_max),
+                                              *[None if a is None else dptr(a) for a in out]))
+        return tuple(out)
 
 
 class Batch:
