@@ -69,7 +69,7 @@ typedef struct lgpu_config {
                                        tuned on line in a batch.
                                        Scheduling only: no result depends on it */
   int advance_queue;                /* secondaries a warp keeps in its own queue before it spills them to
-                                       the global buffer the drain launch works off (1..32; 0: 32).
+                                       a global buffer, worked off behind the advance (1..32; 0: 32).
                                        Scheduling only: a small value exercises the spill path */
 } lgpu_config;
 
@@ -145,7 +145,7 @@ typedef struct lgpu_step_report {
 } lgpu_step_report;
 
 /* Device-time accounting of the main advance kernel (by the device's clock,
- * from its first block's start to its last one's end). */
+ * from the start of its block 0 to the end of its last one). */
 typedef struct lgpu_timing {
   double advance_ms;          /* summed duration of the main advance launches */
   long long advance_launches;
@@ -338,8 +338,10 @@ int lgpu_batch_run(lgpu_batch* batch, lgpu_result* results, int* status, int n, 
  * *running counts those still running), and a later lgpu_batch_run completes
  * what is left. report counts only this call. A context whose energy grid
  * must be re-built (the trial-frequency check, BoltzmannMC.C:617-688) sits
- * one batched interval out while the re-build runs beside it, so n batched
- * intervals advance it by n or fewer of its own; its own sequence of
+ * one batched interval out while the re-build runs beside it, and one that
+ * needs the host for anything else (a new trial frequency, a wider EEDF grid,
+ * larger buffers) the interval that is launched already, so n batched
+ * intervals advance a context by n or fewer of its own; its own sequence of
  * intervals, and so its results, do not change. */
 int lgpu_batch_start(lgpu_batch* batch);
 int lgpu_batch_step(lgpu_batch* batch, int n, int* running, lgpu_batch_report* report);

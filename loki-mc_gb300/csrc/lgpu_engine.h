@@ -1046,12 +1046,8 @@ class Engine {
     return LGPU_OK;
   }
 
-  // ensemble moments at t = 0 (BoltzmannMC.C:306-310), outside the intervals
-  int sample_moments() {
-    LGPU_TRY(launch_moments());
-    LGPU_TRY(sync("read_scalars"));
-    return process_sample();
-  }
+  // ensemble moments at t = 0 (BoltzmannMC.C:306-310), outside the intervals; init_end
+  // waits for them
   int launch_moments() {
     LGPU_CU(cudaMemsetAsync(d_sc_->moments, 0, sizeof(double) * kMoments, stream_));
     LGPU_CU(cudaMemsetAsync(&d_sc_->sample_max_bits, 0, sizeof(unsigned int), stream_));

@@ -229,8 +229,8 @@ struct NoExtra {
   __device__ __forceinline__ void operator()(float4) const {}
 };
 
-// `extra` sees every electron's (vx, vy, vz, flag) in the same pass (the
-// batched kernel counts the EVDF with it)
+// `extra` sees every electron's (vx, vy, vz, flag) in the same pass (the distributions
+// are counted with it)
 template <class Extra = NoExtra>
 __device__ __forceinline__ void sample_range(const SampleArgs& a, int begin, int end, int step,
                                              double (*s_m)[kMoments], Extra extra = Extra()) {

@@ -22,7 +22,7 @@ struct DevScalars {
   unsigned int max_energy_bits;
   int work_counter;
   int pop_counts[2];    // population control: removed slots, surviving secondaries
-  // device clock (ns) of the advance's first block's start and last block's end
+  // device clock (ns) at which block 0 of the advance starts and its last block ends
   // (one condition per launch)
   unsigned long long advance_begin, advance_end;
   unsigned long long null_count;
@@ -295,7 +295,8 @@ struct BatchHeader {
   int smp_full, hist_full, hist2_full;
   int smp_chunk, hist_chunk;                // electrons per chunk of the samples and of the histograms
   int pos;                                  // index of the interval in the chain
-  // device clock (ns) of the advance's first block's start and last block's end
+  // device clock (ns) at which the first branch's block 0 starts the advance and the last
+  // block of any ends it
   unsigned long long advance_begin, advance_end;
 };
 

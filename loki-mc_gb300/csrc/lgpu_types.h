@@ -108,7 +108,7 @@ struct Consts {
   int G;
 };
 
-// Per-interval parameters, written by the host into device memory before each
+// Per-interval parameters of one condition, written by the host into device memory before each
 // chain of synchronisation intervals and by the device from one interval to the next.
 struct IntervalCtl {
   float dt_sync;          // interval length (s)
@@ -118,7 +118,7 @@ struct IntervalCtl {
   float inv_step;         // 1 / table energy step (1/eV)
   float shift_x, shift_y, shift_z;  // origin shift subtracted from every position on load
   unsigned long long interval;      // interval index (random-number counter)
-  int go;                 // 0: the chain of intervals has stopped (one condition per launch)
+  int go;                 // 0: the condition's chain of intervals has stopped
   int pad;
 };
 
