@@ -1119,14 +1119,17 @@ void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
 // side by side; 10,000 electrons with distributions 9.1 -> 7.1 us), full ones
 // from there (fewer EEDF additions per electron: 200,000 electrons under AC
 // 21.9 -> 15.9 us), one large one per SM with EADF and EVDF cells in shared memory
-// from kSampleShared electrons on (1e6: 46 -> 35 us, 4e6 109 -> 65, but 200,000 under
-// AC 17.4 -> 28).
-constexpr int kSampleShared = 600000;
+// from kSampleShared electrons per SM on, 798,000 on 152 SMs. Below, clearing and
+// adding up the shared cells costs more than the additions at L2 that they save: per
+// interval with and without them, atomic gas DC 62.4 and 59.2 us at 450,000, 68.6 and 65.7
+// at 600,000, 77.8 and 77.1 at 800,000, 86.3 and 86.7 at 1e6; N2-like 77.1 and 75.9, 85.2
+// and 83.9, 94.1 and 95.4, 103.4 and 107.3.
+constexpr int kSampleShared = 5250;
 
 void launch_sample(const SampleArgs& a, int sm_count, bool after_kernel, cudaStream_t s) {
   if (a.n <= 0) return;
   const int sms = max(1, sm_count);
-  const bool shared = a.plain && a.n >= kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
+  const bool shared = a.plain && a.n >= sms * kSampleShared && a.n <= sms * 64512ll;  // below 2^16 a block
   if (shared) {
     launch_after(k_sample<true>, min(blocks_for(a.n, kSampleSharedThreads), sms), kSampleSharedThreads, kSampleSmem, s,
                  after_kernel, a);
