@@ -914,8 +914,9 @@ class Engine {
     return LGPU_OK;
   }
 
-  // How many intervals may follow one another before the host has to look: up to a
-  // steady-state or error check (solve_post), a stop criterion (solve_next) or a cap.
+  // How many intervals may follow one another before the host has to look (after
+  // interval_pre): up to a steady-state or error check (solve_post), a stop criterion
+  // (solve_next) or a cap.
   // interval_ms: what one took lately (0: not known, and a cap on time is looked at
   // after each).
   int chain_limit(int want, bool solving, double interval_ms) const {
@@ -923,6 +924,9 @@ class Engine {
     if (!solving) return n;
     if (cfg_.sync_oversampling != 1) return 1;
     const bool ss = ss_time_ != kNonDef;
+    // distributions that the sample leaves to passes of their own are counted before the
+    // next interval moves the electrons on
+    if (ss && !h_plain_->dist.on) return 1;
     // a stop criterion on the count of collisions may hold after any interval
     if (ss && cfg_.max_coll_after_ss * N_ < 1e18) return 1;
     if (cfg_.max_sync_steps > 0) n = (int)std::min<long long>(n, std::max<long long>(1, cfg_.max_sync_steps - solve_steps_));
