@@ -512,7 +512,7 @@ class Engine {
     a.coarse_shift = coarse_shift_;
     a.n_coarse = n_coarse_;
     cudaStream_t st = async && batch_ ? own_stream_ : stream_;
-    launch_build_tables(a, st);
+    launch_build_tables(a, sm_count_, st);
     launches_ += 2;
     d2h_bytes_ += (double)M_ * sizeof(double);
     LGPU_CU(cudaMemcpyAsync(h_nu_max_, d_nu_max_, M_ * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -93,17 +93,18 @@ __device__ __forceinline__ double table_value(const TableBuildArgs& a, int p, do
 // and 140 us, 8, 31 and 44 here (44 ms of the 64-point sweep's 395: 64 first tables
 // and 200 re-grids beside its intervals).
 constexpr int kTableRows = 32, kTablePitch = kTableRows + 1;  // shared-memory pitch of a process's rows
-constexpr int kTableThreads = 256;
+constexpr int kTableThreads = 256, kTableThreadsAlone = 1024;  // (launch_build_tables)
 
 constexpr int table_smem(int P) { return P * kTablePitch * (int)(sizeof(double) + sizeof(float)); }
 
-__global__ void __launch_bounds__(kTableThreads) k_build_tables(TableBuildArgs a) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_build_tables(TableBuildArgs a) {
   extern __shared__ double s_val[];  // [P][kTablePitch] sigma*n, then the FP32 cumulative sums
   const int P = a.P, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float* s_cum = reinterpret_cast<float*>(s_val + P * kTablePitch);
   const int i0 = blockIdx.x * kTableRows, rows = min(kTableRows, a.M - i0), i = i0 + lane;
   const double energy = __dmul_rn((double)i, a.step);
-  for (int p = w; p < P; p += kTableThreads / 32)
+  for (int p = w; p < P; p += THREADS / 32)
     s_val[p * kTablePitch + lane] = lane < rows ? table_value(a, p, energy) : 0.0;
   __syncthreads();
   if (w == 0) {
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(kTableThreads) k_build_tables(TableBuildArgs a
   }
   __syncthreads();
   // pair (row, next row); the next block's first row completes this one's last
-  for (int k = threadIdx.x; k < rows * a.stride; k += kTableThreads) {
+  for (int k = threadIdx.x; k < rows * a.stride; k += THREADS) {
     const int r = k / a.stride, p = k - r * a.stride;
     const size_t o = (size_t)(i0 + r) * a.stride + p;
     if (p >= P) {
@@ -1107,8 +1108,17 @@ void launch_init(const InitArgs& a, cudaStream_t s) {
   k_init<<<blocks_for(a.n, 256), 256, 0, s>>>(a);
 }
 
-void launch_build_tables(const TableBuildArgs& a, cudaStream_t s) {
-  k_build_tables<<<blocks_for(a.M, kTableRows), kTableThreads, table_smem(a.P), s>>>(a);
+// A block that has its SM to itself, because there are no more blocks than SMs or because
+// two blocks' values do not fit one, takes 32 warps instead of 8: its processes'
+// interpolations are chains of dependent loads and divisions. Whole calls with 8 and 32:
+// 100 rows of 196 processes 121 and 84 us, of 410 215 and 150; 1000 rows 174 and 138, 327 and
+// 268; 4864 rows of 40 and 410 105 and 103, 835 and 769, 10,000 of 410 1765 and 1619. With
+// several blocks to an SM the small ones leave it sooner: 10,000 rows of 40 processes 182
+// and 193, of 65 285 and 300.
+void launch_build_tables(const TableBuildArgs& a, int sm_count, cudaStream_t s) {
+  const int blocks = blocks_for(a.M, kTableRows), smem = table_smem(a.P);
+  if (blocks <= sm_count || 2 * smem > 227 * 1024) k_build_tables<kTableThreadsAlone><<<blocks, kTableThreadsAlone, smem, s>>>(a);
+  else k_build_tables<kTableThreads><<<blocks, kTableThreads, smem, s>>>(a);
   const int bounds = a.nu_coarse ? blocks_for(a.n_coarse, kPrefixThreads / 32) : 0;
   k_table_bounds<<<1 + bounds, kPrefixThreads, 0, s>>>(a.nu_tot, a.nu_max, a.M, a.nu_pair, a.coarse_shift, a.nu_coarse,
                                                        a.n_coarse);
@@ -1163,7 +1173,9 @@ void launch_pop_control(const AdvanceArgs& adv, const PopArgs& a, cudaStream_t s
 
 cudaError_t prepare_kernels() {
   static_assert(table_smem(kMaxProcesses) <= 227 * 1024, "the tables of the most processes fit a block");
-  cudaError_t e = cudaFuncSetAttribute(k_build_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, table_smem(kMaxProcesses));
+  cudaError_t e = cudaFuncSetAttribute(k_build_tables<kTableThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, table_smem(kMaxProcesses));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_build_tables<kTableThreadsAlone>, cudaFuncAttributeMaxDynamicSharedMemorySize, table_smem(kMaxProcesses));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_a, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistASmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_b, cudaFuncAttributeMaxDynamicSharedMemorySize, kHistBSmem);
   if (e == cudaSuccess)

@@ -133,7 +133,7 @@ struct TableBuildArgs {
   float* nu_coarse;   // block bounds for the coarse null test [n_coarse], may be null
   int coarse_shift, n_coarse;
 };
-void launch_build_tables(const TableBuildArgs& a, cudaStream_t s);
+void launch_build_tables(const TableBuildArgs& a, int sm_count, cudaStream_t s);
 
 // Distribution tallies of one sample (BoltzmannMC.C:1550-1571).
 struct HistArgs {
