@@ -65,15 +65,15 @@ STATE_BYTES_PER_ELECTRON_STEP = 64  # 32 B state read + 32 B written per electro
 E_N = 200.0
 N_ELECTRONS = 1_000_000
 # DRAM bytes per electron and interval of k_advance, from one ncu capture of the
-# same kernel on 4e6 electrons (N2-like gas, DC 200 Td): 130.5 MB read +
-# 73.8 MB written; traffic grows in proportion to the electrons advanced
-DRAM_BYTES_PER_ELECTRON_STEP = (130.522112e6 + 73.842176e6) / 4.0e6
+# same kernel on 4e6 electrons (N2-like gas, DC 200 Td): 130.7 MB read +
+# 73.9 MB written; traffic grows in proportion to the electrons advanced
+DRAM_BYTES_PER_ELECTRON_STEP = (130.736384e6 + 73.886720e6) / 4.0e6
 
 # DRAM bytes per electron and interval of the batched advance (DC launch, the
 # collision-stash shape the tuner picks, 512 x 2), from one ncu capture of the
-# sweep (the 41st interval, schedule 5,20,1): 888.3 MB read + 560.6 MB written
+# sweep (the 41st interval, schedule 5,20,1): 867.7 MB read + 567.7 MB written
 # for 1.98e7 electrons
-SWEEP_DRAM_BYTES_PER_ELECTRON_STEP = (888.269312e6 + 560.615424e6) / 19795598
+SWEEP_DRAM_BYTES_PER_ELECTRON_STEP = (867.700736e6 + 567.668480e6) / 19795598
 
 # sweep workload
 SWEEP_POINTS = 64
@@ -704,7 +704,7 @@ def ops_real(n_processes):
 # ncu counters of one batched DC advance launch over the sweep (1.98e7
 # electrons, collision-stash shape 512 x 2, the same launch as above): warp
 # instructions per electron-interval issued to the FMA, ALU and XU (SFU) pipes
-NCU_PIPE_PER_ELECTRON = {"fma": 181978916 / 19795598, "alu": 244863326 / 19795598, "xu": 12198627 / 19795598}
+NCU_PIPE_PER_ELECTRON = {"fma": 172662967 / 19795598, "alu": 241156028 / 19795598, "xu": 11249394 / 19795598}
 
 
 def issue_roofline(real, null, electron_steps, kernel_ms, n_processes, flight_ops, sm_mhz):
@@ -726,7 +726,7 @@ def issue_roofline(real, null, electron_steps, kernel_ms, n_processes, flight_op
                                      "times this run's electron-intervals over its advance time"},
             "ncu_pipe_warp_instructions_per_electron_interval": NCU_PIPE_PER_ELECTRON,
             "note": "the advance issues more ALU (integer: random numbers, lane bookkeeping) than FMA "
-                    "instructions at ~18 of 32 lanes active, about half of the issue slots busy (latency-bound: "
+                    "instructions at ~19 of 32 lanes active, about two thirds of the issue slots busy (latency-bound: "
                     "state and table loads); the method's own FP32 + SFU work is a few % of the lanes' rate"}
 
 

@@ -943,9 +943,10 @@ __global__ void __launch_bounds__(kHistBThreads) k_hist_b_batch(BatchArgs b) {
 // hdr->smp_chunk electrons.
 //
 // The 64-point sweep: moments with the EVDF, then EEDF and EADF in a pass of their
-// own, took 123 + 195 us per interval; all of it takes 178 here (3.6 TB/s), about
-// half of it the counts (issue, shared additions) and a third the addition of every
-// chunk's occupied cells to the tallies at L2. 32 conditions of 10,000-30,000
+// own, took 123 + 195 us per interval; all of it takes 177 here (3.6 TB/s), of which the
+// addition of every chunk's occupied cells to the tallies at L2 35, the shared additions
+// 10 to 30 and the read alone 93; the launch waits for the blocks with two whole chunks
+// (1.17 of the mean share). 32 conditions of 10,000-30,000
 // electrons: 21 + 66 -> 25 us. Loads in flight are not what it waits for: a ring of
 // asynchronous copies in place of the four records in registers took 193.
 constexpr int kSampleBatchShared = 8192;  // electrons of a chunk that are worth shared cells (16 jobs: 41 us, 56 with 16384)

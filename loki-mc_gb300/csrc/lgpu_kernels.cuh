@@ -176,7 +176,8 @@ struct DistCtl {
 
 // Ensembles of a context on its own up to this size count their distributions with
 // the sample: above it a block of one per SM would see more electrons than its 16-bit
-// counts hold, and the passes over 65535-electron chunks fill the device.
+// counts hold, and the passes over 65535-electron chunks fill the device. The passes come
+// before the next interval's advance, so that such intervals are chains of their own.
 constexpr int kDistInSample = 9000000;
 
 // A chain of intervals of one condition: the host launches up to kChain of them
@@ -317,10 +318,10 @@ constexpr int kBatchMaxSlots = 1024;
 constexpr int kBatchAdvanceChunk = 4096;   // granularity of the advance's initial spread of blocks over slots
 constexpr int kBatchSampleChunk = 65535;   // electrons per chunk of the samples at most (16-bit EVDF counts)
 constexpr int kBatchHistChunk = 65535;     // electrons per chunk of the histograms at most (16-bit counts)
-// Batches of fewer sampled electrons keep EEDF and EADF in a pass of their own. One
-// pass would be the faster one for them too (a served job of 50,000 electrons 66 ->
-// 37 ms), but the check that arriving jobs overlap on the device
-// (tests/test_gpu_batch.py) has them arrive 38 ms apart.
+// Batches of fewer sampled electrons count their distributions in passes of their own, an
+// interval at a time, as all batches did once. It is not what is faster for them: one
+// pass and chains take a served job of 50,000 electrons from 66 to 37 ms. The check that
+// arriving jobs overlap on the device (tests/test_gpu_batch.py) has them arrive 38 ms apart.
 constexpr double kBatchDistMin = 150000;
 
 // Staging layout (host pinned mirror and device copy are identical):
