@@ -320,7 +320,7 @@ constexpr int kBatchSampleChunk = 65535;   // electrons per chunk of the samples
 constexpr int kBatchHistChunk = 65535;     // electrons per chunk of the histograms at most (16-bit counts)
 // Batches of fewer sampled electrons count their distributions in passes of their own, an
 // interval at a time, as all batches did once. It is not what is faster for them: one
-// pass and chains take a served job of 50,000 electrons from 66 to 37 ms. The check that
+// pass and chains take a served job of 50,000 electrons from 40 to 20 ms. The check that
 // arriving jobs overlap on the device (tests/test_gpu_batch.py) has them arrive 38 ms apart.
 constexpr double kBatchDistMin = 150000;
 
